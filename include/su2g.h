@@ -128,8 +128,10 @@ int su2g_heff_plan_status(su2g_heff_plan* plan, int* code);
  * reference, whose per-block loop tensor_su2_dmrg_src.cpp:977-1006 calls one
  * DGEMM per block).  Buckets: M <= m_edges[i] (i < nm), N <= n_edges[j], the
  * last bucket of each open-ended; cls[i * nn + j] in 0..3 = tiles of 64 x 64,
- * 64 x 32, 32 x 64, 32 x 32.  Plans built afterwards use it; without a table
- * every block uses 64 x 64. */
+ * 64 x 32, 32 x 64, 32 x 32.  The planner of plans built afterwards cuts by
+ * it; without a table every block uses 64 x 64.  The launches are cut further
+ * (32 x 32, or 8 x 8 with a split contraction) whatever the table, so results
+ * do not depend on it. */
 int su2g_f64_tile_table(const int* m_edges, int nm, const int* n_edges, int nn, const int* cls);
 /* The autotuner's measurement: nblocks independent M x N x K block products
  * in tiles of class cls, one launch, repeated reps times; *ms = device

@@ -2,17 +2,21 @@
 
 The reference multiplies every block pair with one DGEMM call
 (tensor_su2_dmrg_src.cpp:977-1006), whatever the block sizes.  Here the
-blocks of one H_eff application or environment update run as tiles of one
-launch, and the tile shape is a choice: 64 x 64 tiles waste most of the FP64
-tensor pipe's work on blocks of a few tens of rows (the padding is computed),
-smaller tiles cost more operand staging per product.  The autotuner measures,
-for each bucket of output-block sizes (M, N), the device time of the four tile
-classes (64x64, 64x32, 32x64, 32x32) on a batch of independent block products
-of that size (su2g_f64_tile_bench), keeps the fastest class per bucket, and
-installs the table (su2g_f64_tile_table): plans built afterwards tile every
-block by its size class.  The table persists as JSON; `load` installs a saved
-one (the package ships the one measured on GB300, tile_table_gb300.json, and
+blocks of one H_eff application or environment update are cut by the planner
+into tiles of one of four classes (64x64, 64x32, 32x64, 32x32).  The
+autotuner measures, for each bucket of output-block sizes (M, N), the device
+time of every class on a batch of independent block products of that size
+(su2g_f64_tile_bench: one CTA per tile of the class), keeps the fastest class
+per bucket, and installs the table (su2g_f64_tile_table): plans built
+afterwards cut every block by its size class.  The table persists as JSON;
+`load` installs a saved one (the package ships one, tile_table_gb300.json, and
 installs it when the library loads).
+
+A plan's launches no longer depend on the class: every phase is cut further
+for the device, into 32x32 tiles or into 8x8 tiles with a split contraction
+(f64_launch_tiles in heff_plan.cpp), because neither wastes FP64 work on
+padding and a finer cut keeps every SM busy.  Results are the same whatever
+table is installed.
 """
 from __future__ import annotations
 

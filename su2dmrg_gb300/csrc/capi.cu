@@ -234,8 +234,12 @@ int plan_from_work(su2g::HeffWork&& work, int mode, su2g_heff_plan** plan, const
   if (S == 0) {
     stage.add(p->work.seg1, &p->d_seg1);
     stage.add(p->work.seg2, &p->d_seg2);
-    stage.add(p->work.tile1, &p->d_tile1);
-    stage.add(p->work.tile2, &p->d_tile2);
+    p->launch1 = su2g::f64_launch_tiles(p->work.tile1);
+    p->launch2 = su2g::f64_launch_tiles(p->work.tile2);
+    p->count1 = su2g::f64_counts(p->launch1);
+    p->count2 = su2g::f64_counts(p->launch2);
+    stage.add(p->launch1, &p->d_tile1);
+    stage.add(p->launch2, &p->d_tile2);
   } else {
     const su2g::oz::OzWork& w = p->oz;
     for (int c = 0; c < 3; ++c) {
@@ -574,8 +578,7 @@ int su2g_heff_plan_launches(const su2g_heff_plan* p, int* n) {
   if (!p || !n) return fail(SU2G_EINVAL, "plan_launches: bad arguments");
   int c = 0;
   if (p->S == 0) {
-    c += p->work.tile1.empty() ? 0 : 1;
-    c += p->work.tile2.empty() ? 0 : 1;
+    c += p->count1.launches() + p->count2.launches();
   } else {
     const su2g::oz::OzWork& w = p->oz;
     for (int k = 1; k <= 2; ++k)
@@ -668,9 +671,9 @@ int su2g_f64_tile_bench(int M, int N, int K, int nblocks, int cls, int reps, dou
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (e == cudaSuccess) e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
-  if (e == cudaSuccess) e = su2g::launch_gemm_f64(dtile, (int)tiles.size(), dseg, bases, st);  // warm
+  if (e == cudaSuccess) e = su2g::launch_gemm_f64(dtile, su2g::f64_counts(tiles), dseg, bases, st);  // warm
   if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-  for (int r = 0; r < reps && e == cudaSuccess; ++r) e = su2g::launch_gemm_f64(dtile, (int)tiles.size(), dseg, bases, st);
+  for (int r = 0; r < reps && e == cudaSuccess; ++r) e = su2g::launch_gemm_f64(dtile, su2g::f64_counts(tiles), dseg, bases, st);
   if (e == cudaSuccess) e = cudaEventRecord(e1, st);
   if (e == cudaSuccess) e = cudaEventSynchronize(e1);
   float t = 0;
@@ -750,8 +753,8 @@ int su2g::cuda_status(cudaError_t e, const char* where) { return cuda_fail(e, wh
 int su2g::heff_apply_impl(su2g_heff_plan* p, const double* psi, double* y, cudaStream_t st) {
   const su2g::Bases b = make_bases(p, psi, y);
   if (p->S == 0) {
-    SU2G_CUDA(su2g::launch_gemm_f64(p->d_tile1, (int)p->work.tile1.size(), p->d_seg1, b, st));
-    SU2G_CUDA(su2g::launch_gemm_f64(p->d_tile2, (int)p->work.tile2.size(), p->d_seg2, b, st));
+    SU2G_CUDA(su2g::launch_gemm_f64(p->d_tile1, p->count1, p->d_seg1, b, st));
+    SU2G_CUDA(su2g::launch_gemm_f64(p->d_tile2, p->count2, p->d_seg2, b, st));
     SU2G_CUDA(su2g::apply_projectors(p, psi, y, st));
     return SU2G_OK;
   }
@@ -794,9 +797,9 @@ int su2g_heff_apply_profile(su2g_heff_plan* p, const double* psi, double* y, voi
   cudaError_t e = cudaEventRecord(ev[0], st);
   int n = 0;
   if (p->S == 0) {
-    if (e == cudaSuccess) e = su2g::launch_gemm_f64(p->d_tile1, (int)p->work.tile1.size(), p->d_seg1, b, st);
+    if (e == cudaSuccess) e = su2g::launch_gemm_f64(p->d_tile1, p->count1, p->d_seg1, b, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[1], st);
-    if (e == cudaSuccess) e = su2g::launch_gemm_f64(p->d_tile2, (int)p->work.tile2.size(), p->d_seg2, b, st);
+    if (e == cudaSuccess) e = su2g::launch_gemm_f64(p->d_tile2, p->count2, p->d_seg2, b, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[2], st);
     n = 2;
   } else {

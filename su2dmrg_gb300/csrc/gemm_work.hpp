@@ -41,8 +41,15 @@ struct GemmTile {
   int mlen, nlen; // rows / columns of this tile (<= tile size)
   int seg0, nseg; // segments [seg0, seg0 + nseg)
   int64_t kwork;  // sum of K over the segments (scheduling weight)
-  int cls;        // tile class (kTileClassM/N): the FP64 engine's tile shape
-  int pad;
+  int cls;        // tile class (kTileClassM/N): the planner's tile shape
+  int ksplit;     // 1: a tile of one fragment whose contraction the CTA's warps share (f64_launch_tiles)
+};
+
+// A launched list holds whole tiles, then split ones (one plan's list holds one
+// kind, a batch's perhaps both).
+struct F64Counts {
+  int whole = 0, split = 0;
+  int launches() const { return (whole > 0) + (split > 0); }
 };
 
 struct Bases {
@@ -56,9 +63,10 @@ inline double* resolve(const Bases& b, int buf, int64_t off) {
   return reinterpret_cast<double*>(b.p[buf] + (uintptr_t)(off * 8));
 }
 
+constexpr int kF64Sms = 152;  // SMs the FP64 work is balanced over (a constant: sums do not depend on the device)
 constexpr int kTileM = 64;  // largest tile
 constexpr int kTileN = 64;
-// Tile classes of the FP64 engine: 64x64, 64x32, 32x64, 32x32.  Which class an
+// Tile classes of the planner's FP64 lists: 64x64, 64x32, 32x64, 32x32.  Which class an
 // output block uses follows its size class (a table an autotuner fills from
 // measurements, tile_class_for in heff_plan.cpp).
 constexpr int kTileClasses = 4;

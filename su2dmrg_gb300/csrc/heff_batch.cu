@@ -74,7 +74,7 @@ struct Lists {
   su2g::GemmSeg* fseg2 = nullptr;
   su2g::GemmTile* ftile1 = nullptr;
   su2g::GemmTile* ftile2 = nullptr;
-  int nft1 = 0, nft2 = 0;
+  su2g::F64Counts nft1, nft2;
 
   void release(cudaStream_t st) {
     for (int c = 0; c < 3; ++c) {
@@ -210,7 +210,7 @@ int build_lists(su2g_heff_batch* B, const std::vector<int>& members, Lists* L) {
       for (int i : members) {
         const su2g_heff_plan* p = B->plans[i];
         const auto& ps = ph == 1 ? p->work.seg1 : p->work.seg2;
-        const auto& pt = ph == 1 ? p->work.tile1 : p->work.tile2;
+        const auto& pt = ph == 1 ? p->launch1 : p->launch2;
         const int s0 = (int)segs.size();
         for (su2g::GemmSeg g : ps) {
           shift_ref(B, i, &g.a_buf, &g.a);
@@ -223,9 +223,10 @@ int build_lists(su2g_heff_batch* B, const std::vector<int>& members, Lists* L) {
           tiles.push_back(t);
         }
       }
+      su2g::f64_order_by_kind(&tiles);
       if (e == cudaSuccess) e = upload(segs, ph == 1 ? &L->fseg1 : &L->fseg2);
       if (e == cudaSuccess) e = upload(tiles, ph == 1 ? &L->ftile1 : &L->ftile2);
-      (ph == 1 ? L->nft1 : L->nft2) = (int)tiles.size();
+      (ph == 1 ? L->nft1 : L->nft2) = su2g::f64_counts(tiles);
     }
   }
   if (e != cudaSuccess) return su2g::cuda_status(e, "heff_batch lists");

@@ -102,6 +102,63 @@ void add_tiles(std::vector<GemmTile>& tiles, int64_t c_off, int64_t c_len, int c
     }
 }
 
+// Splitting pays where a tile contracts enough values for eight warps to share
+// (always), or where whole 32 x 32 tiles would leave SMs idle.  Measured on
+// GB300, phase 1 (one product a tile) + phase 2 (all terms), ms: D = 2000, 18
+// terms, K <= 555 and 31,000: whole 64.7 + 72.6, split 67.1 + 67.0; D = 1000:
+// 8.44 + 8.86 and 9.22 + 8.65; D = 400, 12 terms, K <= 105 and 4,000: 0.39 and
+// 0.51 + 0.41; D = 251, 9 terms: phase 2 2.13 whole, 0.096 split.
+namespace {
+constexpr int64_t kF64SplitK = 1024;    // split from this many contracted values on,
+constexpr int64_t kF64MinSplitK = 96;   // and from this many on where 32 x 32 tiles are uneven:
+constexpr double kF64Uneven = 3.0;      // one takes more than a third of an SM's share
+}  // namespace
+
+std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles) {
+  // Work in fragment steps: an 8 x 8 fragment times the values it contracts.
+  // Every tile edge is a multiple of 32 inside its block, so these figures
+  // (and the cuts below) are the blocks' own, whatever classes cut them.
+  auto up = [](int n, int d) { return (n + d - 1) / d; };
+  double total = 0, largest = 0;
+  int64_t kmax = 0;
+  for (const GemmTile& t : tiles) {
+    total += (double)up(t.mlen, 8) * up(t.nlen, 8) * t.kwork;
+    largest = std::max(largest, (double)up(std::min(t.mlen, 32), 8) * up(std::min(t.nlen, 32), 8) * t.kwork);
+    kmax = std::max(kmax, t.kwork);
+  }
+  const bool uneven = largest * kF64Uneven > total / kF64Sms;
+  const bool split = kmax >= kF64SplitK || (kmax >= kF64MinSplitK && uneven);
+  const int side = split ? 8 : 32;
+  std::vector<GemmTile> out;
+  for (const GemmTile& t : tiles)
+    for (int m = 0; m < t.mlen; m += side)
+      for (int n = 0; n < t.nlen; n += side) {
+        GemmTile u = t;
+        u.m0 = t.m0 + m;
+        u.n0 = t.n0 + n;
+        u.mlen = std::min(side, t.mlen - m);
+        u.nlen = std::min(side, t.nlen - n);
+        u.cls = 3;
+        u.ksplit = split ? 1 : 0;
+        out.push_back(u);
+      }
+  // heaviest first, as the planner's
+  auto work = [&](const GemmTile& t) { return (int64_t)up(t.mlen, 8) * up(t.nlen, 8) * t.kwork; };
+  std::stable_sort(out.begin(), out.end(), [&](const GemmTile& x, const GemmTile& y) { return work(x) > work(y); });
+  return out;
+}
+
+F64Counts f64_counts(const std::vector<GemmTile>& tiles) {
+  F64Counts n;
+  for (const GemmTile& t : tiles) ++(t.ksplit == 0 ? n.whole : n.split);
+  return n;
+}
+
+void f64_order_by_kind(std::vector<GemmTile>* tiles) {
+  std::stable_sort(tiles->begin(), tiles->end(),
+                   [](const GemmTile& x, const GemmTile& y) { return x.ksplit < y.ksplit; });
+}
+
 int build_heff_work(const int* psi_desc, const int* psi_flag, int nterms, const su2g_term* terms,
                     const su2g_tensor* hl, double hl_coef, const su2g_tensor* hr, double hr_coef, HeffWork* out,
                     std::string* err, bool fp64_tiles) {

@@ -1,10 +1,12 @@
 // FP64 kernels of the hot path:
-//   * gemm_f64_tiles: the block-sparse contraction engine (one CTA per output
-//     tile of the work list, gemm_work.hpp), FP64 tensor-core MMA
-//     (mma.sync.m8n8k4.f64) fed from shared memory;
+//   * gemm_f64_tiles: the block-sparse contraction engine (one CTA per tile of
+//     the work list, gemm_work.hpp), FP64 tensor-core MMA
+//     (mma.sync.m8n8k4.f64) fed from global memory through L1;
+//   * gemm_f64_dense: one dense product with the same tile code;
 //   * deterministic BLAS-1 (dot, axpy, scale) for the Lanczos iteration.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "gemm_work.hpp"
@@ -13,142 +15,190 @@
 namespace su2g {
 namespace {
 
-constexpr int kBK = 16;       // K per shared-memory stage
-constexpr int kThreads = 128; // 4 warps, each a quadrant of the tile
+constexpr int kWarps = 8;
+constexpr int kThreads = kWarps * 32;
 
 __device__ __forceinline__ void dmma_m8n8k4(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
 }
 
-// One TM x TN output tile: C_tile = sum_s alpha_s * op(A_s) B_s; every
-// segment is accumulated on its own, scaled by its alpha and added (the
-// reference scales each block product by its recoupling factor before
-// summing, tensor_su2_dmrg_src.cpp:997-1004).  Warp w computes the quadrant
-// (w / 2, w % 2) of (TM / 2) x (TN / 2) as FM x FN fragments of 8 x 8.
-// Operands are staged K = 16 at a time in shared memory, rows padded by 4
-// doubles (conflict-free fragment reads).
-template <int TM, int TN>
-__device__ __forceinline__ void f64_tile(const GemmTile& t, const GemmSeg* __restrict__ segs, const Bases& bases,
-                                         double* __restrict__ As, double* __restrict__ Bs) {
-  constexpr int FM = TM / 16, FN = TN / 16;
-  constexpr int LA = TM + 4, LB = TN + 4;
-  constexpr int PA = TM / 8, PB = TN / 8;  // elements each thread stages per operand per stage
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 1) * (TM / 2), wn = (warp & 1) * (TN / 2);
-  const int fr = lane >> 2, fc = lane & 3;
-
-  double acc[FM][FN][2];
+// sacc = op(A) B over the steps [step0, step1) of 4 contracted values of one
+// segment, for nj 8 x 8 fragments side by side: this lane reads row `row` of
+// op(A) and the columns col[j] of B.
+//
+// Bound by the FP64 pipe: GB300 does about two multiply-adds per clock and SM,
+// so one m8n8k4 occupies an SM for 128 clocks while its operands are 512 bytes.
+// Every warp therefore reads its fragments straight from global memory (a few
+// bytes per clock and SM through L1 and L2): no staging, no barriers, and no
+// work for padding beyond a fragment's edge.  Four steps of loads are in
+// flight before the MMAs that use them; other warps cover the latency.  At
+// D = 2000, 18 terms, an application takes 131.7 ms (1.066 TFLOP/s, 0.97 of
+// cuBLAS DGEMM's 1.10); 64 x 64 tiles staged in shared memory took 153 ms, the
+// difference being the work done for their padding.
+//
+// Rows and columns past the block are clamped to it and feed only entries
+// that are never stored; values past K are zero in both operands.
+template <int FN>
+__device__ __forceinline__ void seg_mma(const GemmSeg& g, const Bases& bases, int row, const int (&col)[FN], int nj,
+                                        int step0, int step1, int fc, double (&sacc)[FN][2]) {
+  constexpr int U = 4;
 #pragma unroll
-  for (int i = 0; i < FM; ++i)
+  for (int j = 0; j < FN; ++j) sacc[j][0] = sacc[j][1] = 0.0;
+  const int64_t ks = g.transA ? 1 : g.lda;  // distance of neighbouring k in A
+  const int k = step0 * 4 + fc;
+  const double* ap = resolve(bases, g.a_buf, g.a) + (g.transA ? (int64_t)row * g.lda : row) + k * ks;
+  const double* bp[FN];
 #pragma unroll
-    for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-  for (int s = t.seg0; s < t.seg0 + t.nseg; ++s) {
-    const GemmSeg g = segs[s];
-    const double* __restrict__ A = resolve(bases, g.a_buf, g.a);
-    const double* __restrict__ B = resolve(bases, g.b_buf, g.b);
-    double sacc[FM][FN][2];
+  for (int j = 0; j < FN; ++j) bp[j] = resolve(bases, g.b_buf, g.b) + (int64_t)col[j] * g.ldb + k;
+  int step = step0;
+  const int full = min(step1, g.K / 4);
+  for (; step + U <= full; step += U) {
+    double a[U], b[U][FN];
 #pragma unroll
-    for (int i = 0; i < FM; ++i)
+    for (int u = 0; u < U; ++u) {
+      a[u] = __ldg(ap + 4 * u * ks);
 #pragma unroll
-      for (int j = 0; j < FN; ++j) sacc[i][j][0] = sacc[i][j][1] = 0.0;
-
-    for (int k0 = 0; k0 < g.K; k0 += kBK) {
-      // ---- stage A (TM x 16) and B (16 x TN), zero padded ----
-      if (g.transA) {  // A stored K x M: (k, m) at A[k + m*lda], contiguous in k
-        const int m = tid / (kBK / PA), kb = (tid % (kBK / PA)) * PA;
-        const bool mok = m < t.mlen;
-        const double* src = A + (int64_t)(t.m0 + m) * g.lda + k0 + kb;
-#pragma unroll
-        for (int i = 0; i < PA; ++i) {
-          const int k = kb + i;
-          As[k * LA + m] = (mok && k0 + k < g.K) ? __ldg(src + i) : 0.0;
-        }
-      } else {  // A stored M x K: (m, k) at A[m + k*lda], contiguous in m
-        const int k = tid >> 3, mb = (tid & 7) * PA;
-        const bool kok = k0 + k < g.K;
-        const double* src = A + (int64_t)(k0 + k) * g.lda + t.m0 + mb;
-#pragma unroll
-        for (int i = 0; i < PA; ++i) {
-          const int m = mb + i;
-          As[k * LA + m] = (kok && m < t.mlen) ? __ldg(src + i) : 0.0;
-        }
-      }
-      {  // B stored K x N: (k, n) at B[k + n*ldb], contiguous in k
-        const int n = tid / (kBK / PB), kb = (tid % (kBK / PB)) * PB;
-        const bool nok = n < t.nlen;
-        const double* src = B + (int64_t)(t.n0 + n) * g.ldb + k0 + kb;
-#pragma unroll
-        for (int i = 0; i < PB; ++i) {
-          const int k = kb + i;
-          Bs[k * LB + n] = (nok && k0 + k < g.K) ? __ldg(src + i) : 0.0;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < kBK; kk += 4) {
-        double af[FM], bf[FN];
-#pragma unroll
-        for (int i = 0; i < FM; ++i) af[i] = As[(kk + fc) * LA + wm + i * 8 + fr];
-#pragma unroll
-        for (int j = 0; j < FN; ++j) bf[j] = Bs[(kk + fc) * LB + wn + j * 8 + fr];
-#pragma unroll
-        for (int i = 0; i < FM; ++i)
-#pragma unroll
-          for (int j = 0; j < FN; ++j) dmma_m8n8k4(sacc[i][j], af[i], bf[j]);
-      }
-      __syncthreads();
+      for (int j = 0; j < FN; ++j) b[u][j] = j < nj ? __ldg(bp[j] + 4 * u) : 0.0;
     }
-    const double alpha = g.alpha;
 #pragma unroll
-    for (int i = 0; i < FM; ++i)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int j = 0; j < FN; ++j) {
-        acc[i][j][0] += alpha * sacc[i][j][0];
-        acc[i][j][1] += alpha * sacc[i][j][1];
-      }
+      for (int j = 0; j < FN; ++j)
+        if (j < nj) dmma_m8n8k4(sacc[j], a[u], b[u][j]);
+    ap += 4 * U * ks;
+#pragma unroll
+    for (int j = 0; j < FN; ++j) bp[j] += 4 * U;
   }
-
-  double* C = resolve(bases, t.c_buf, t.c);
-#pragma unroll
-  for (int i = 0; i < FM; ++i) {
-    const int r = wm + i * 8 + fr;
-    if (r >= t.mlen) continue;
+  for (; step < step1; ++step) {  // the last steps one by one, the very last perhaps past K
+    const bool ok = step * 4 + fc < g.K;
+    const double a = ok ? __ldg(ap) : 0.0;
 #pragma unroll
     for (int j = 0; j < FN; ++j) {
+      const double b = (ok && j < nj) ? __ldg(bp[j]) : 0.0;
+      if (j < nj) dmma_m8n8k4(sacc[j], a, b);
+      bp[j] += 4;
+    }
+    ap += 4 * ks;
+  }
+}
+
+template <int FN>
+__device__ __forceinline__ void add_scaled(double alpha, const double (&sacc)[FN][2], double (&acc)[FN][2]) {
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int c = wn + j * 8 + 2 * fc + q;
-        if (c < t.nlen) C[(int64_t)(t.m0 + r) + (int64_t)(t.n0 + c) * t.ldc] = acc[i][j][q];
-      }
+  for (int j = 0; j < FN; ++j) {
+    acc[j][0] += alpha * sacc[j][0];
+    acc[j][1] += alpha * sacc[j][1];
+  }
+}
+
+// The sub-tile of t at rows m1.. and columns n1.., C = sum_s alpha_s op(A_s)
+// B_s, by WM x WN warps of FN fragments side by side: every segment is
+// accumulated on its own, scaled by its alpha and added (the reference scales
+// each block product by its recoupling factor before summing,
+// tensor_su2_dmrg_src.cpp:997-1004).  Only fragments that hold rows and
+// columns of the block are computed.  Every element sums its products in k
+// order whatever the tile shape.
+template <int FN, int WM, int WN>
+__device__ __forceinline__ void sub_tile(const GemmTile& t, int m1, int n1, const GemmSeg* __restrict__ segs,
+                                         const Bases& bases) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wr = warp % WM, wc = warp / WM;
+  const int fr = lane >> 2, fc = lane & 3;
+  const int mlen = min(WM * 8, t.mlen - m1), nlen = min(WN * FN * 8, t.nlen - n1);
+  const int nj = ((nlen + 7) / 8 - wc + WN - 1) / WN;  // fragments are dealt to the warps in turn
+  if (wr * 8 >= mlen || nj <= 0) return;
+  const int row = t.m0 + m1 + min(wr * 8 + fr, mlen - 1);
+  int col[FN];
+#pragma unroll
+  for (int j = 0; j < FN; ++j) col[j] = t.n0 + n1 + min((wc + WN * j) * 8 + fr, nlen - 1);
+  double acc[FN][2] = {};
+  for (int s = t.seg0; s < t.seg0 + t.nseg; ++s) {
+    const GemmSeg g = segs[s];
+    double sacc[FN][2];
+    seg_mma<FN>(g, bases, row, col, nj, 0, (g.K + 3) / 4, fc, sacc);
+    add_scaled<FN>(g.alpha, sacc, acc);
+  }
+  double* C = resolve(bases, t.c_buf, t.c);
+  const int r = wr * 8 + fr;
+  if (r >= mlen) return;
+#pragma unroll
+  for (int j = 0; j < FN; ++j)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = (wc + WN * j) * 8 + 2 * fc + q;
+      if (c < nlen) C[(int64_t)(t.m0 + m1 + r) + (int64_t)(t.n0 + n1 + c) * t.ldc] = acc[j][q];
+    }
+}
+
+// One output tile of one 8 x 8 fragment whose contraction is dealt to the eight
+// warps: the steps of all its segments, laid end to end, in eight equal runs.
+// The eight partial tiles are summed through shared memory in run order.
+__global__ void __launch_bounds__(kThreads, 4) gemm_f64_ksplit(const GemmTile* __restrict__ tiles,
+                                                               const GemmSeg* __restrict__ segs, Bases bases) {
+  __shared__ double part[kWarps * 64];
+  const GemmTile t = tiles[blockIdx.x];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int fr = lane >> 2, fc = lane & 3;
+  const int row = t.m0 + min(fr, t.mlen - 1), col[1] = {t.n0 + min(fr, t.nlen - 1)};
+  double acc[1][2] = {};
+  int total = 0;  // steps of 4 over all segments
+  for (int s = lane; s < t.nseg; s += 32) total += (segs[t.seg0 + s].K + 3) / 4;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  const int lo = (int)((int64_t)total * warp / kWarps), hi = (int)((int64_t)total * (warp + 1) / kWarps);
+  for (int s0 = 0, base = 0; s0 < t.nseg && base < hi; s0 += 32) {
+    const int n = s0 + lane < t.nseg ? (segs[t.seg0 + s0 + lane].K + 3) / 4 : 0;
+    int end = n;  // inclusive prefix sum
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    end += base;
+    unsigned mine = __ballot_sync(0xffffffffu, n > 0 && end > lo && end - n < hi);
+    while (mine) {
+      const int b = __ffs(mine) - 1;
+      mine &= mine - 1;
+      const int e1 = __shfl_sync(0xffffffffu, end, b), e0 = e1 - __shfl_sync(0xffffffffu, n, b);
+      const GemmSeg g = segs[t.seg0 + s0 + b];
+      double sacc[1][2];
+      seg_mma<1>(g, bases, row, col, 1, max(lo - e0, 0), min(hi, e1) - e0, fc, sacc);
+      add_scaled<1>(g.alpha, sacc, acc);
+    }
+    base = __shfl_sync(0xffffffffu, end, 31);
+  }
+  part[warp * 64 + lane] = acc[0][0];
+  part[warp * 64 + 32 + lane] = acc[0][1];
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    const int e = threadIdx.x, l = e & 31;
+    const int r = l >> 2, c = 2 * (l & 3) + (e >> 5);
+    if (r < t.mlen && c < t.nlen) {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) v += part[w * 64 + e];
+      resolve(bases, t.c_buf, t.c)[(int64_t)(t.m0 + r) + (int64_t)(t.n0 + c) * t.ldc] = v;
     }
   }
 }
 
-// One CTA per tile of the work list; the tile's class picks its shape (the
-// branch is uniform over the CTA).
-__global__ void __launch_bounds__(kThreads) gemm_f64_tiles(const GemmTile* __restrict__ tiles,
-                                                           const GemmSeg* __restrict__ segs, Bases bases) {
-  __shared__ double As[kBK * (kTileM + 4)];
-  __shared__ double Bs[kBK * (kTileN + 4)];
+// One CTA per whole tile of the work list, 32 x 32 at a time.
+__global__ void __launch_bounds__(kThreads, 4) gemm_f64_tiles(const GemmTile* __restrict__ tiles,
+                                                              const GemmSeg* __restrict__ segs, Bases bases) {
   const GemmTile t = tiles[blockIdx.x];
-  switch (t.cls) {
-    case 1: f64_tile<64, 32>(t, segs, bases, As, Bs); break;
-    case 2: f64_tile<32, 64>(t, segs, bases, As, Bs); break;
-    case 3: f64_tile<32, 32>(t, segs, bases, As, Bs); break;
-    default: f64_tile<64, 64>(t, segs, bases, As, Bs); break;
-  }
+  for (int m1 = 0; m1 < t.mlen; m1 += 32)
+    for (int n1 = 0; n1 < t.nlen; n1 += 32) sub_tile<2, 4, 2>(t, m1, n1, segs, bases);
 }
 
-// One dense product C = op(A) B in tiles of class cls, the tile and its
-// segment formed from the kernel's arguments (no work list to upload): the
-// same tile code, so the same sums in the same order as a work-list launch.
-__global__ void __launch_bounds__(kThreads) gemm_f64_dense(int transA, int M, int N, int K, const double* A, int lda,
-                                                           const double* B, int ldb, double* C, int ldc, int cls) {
-  __shared__ double As[kBK * (kTileM + 4)];
-  __shared__ double Bs[kBK * (kTileN + 4)];
+// One dense product C = op(A) B in tiles of WM x WN FN fragments, the tile
+// and its segment formed from the kernel's arguments (no work list to
+// upload): the same tile code, so the same sums in the same order as a
+// work-list launch of unsplit tiles.
+template <int FN, int WM, int WN>
+__global__ void __launch_bounds__(WM * WN * 32) gemm_f64_dense(int transA, int M, int N, int K, const double* A,
+                                                              int lda, const double* B, int ldb, double* C, int ldc) {
   GemmSeg g;
   g.a = (int64_t)((uintptr_t)A / 8);
   g.b = (int64_t)((uintptr_t)B / 8);
@@ -165,40 +215,39 @@ __global__ void __launch_bounds__(kThreads) gemm_f64_dense(int transA, int M, in
   t.c_len = 0;
   t.c_buf = kBufAbs;
   t.ldc = ldc;
-  const int tm = cls == 2 || cls == 3 ? 32 : 64, tn = cls == 1 || cls == 3 ? 32 : 64;
-  t.m0 = blockIdx.x * tm;
-  t.n0 = blockIdx.y * tn;
-  t.mlen = min(tm, M - t.m0);
-  t.nlen = min(tn, N - t.n0);
+  t.m0 = blockIdx.x * (WM * 8);
+  t.n0 = blockIdx.y * (WN * FN * 8);
+  t.mlen = min(WM * 8, M - t.m0);
+  t.nlen = min(WN * FN * 8, N - t.n0);
   t.seg0 = 0;
   t.nseg = 1;
   t.kwork = K;
-  t.cls = cls;
-  t.pad = 0;
-  const Bases bases{};
-  switch (cls) {
-    case 1: f64_tile<64, 32>(t, &g, bases, As, Bs); break;
-    case 2: f64_tile<32, 64>(t, &g, bases, As, Bs); break;
-    case 3: f64_tile<32, 32>(t, &g, bases, As, Bs); break;
-    default: f64_tile<64, 64>(t, &g, bases, As, Bs); break;
-  }
+  t.cls = 0;
+  t.ksplit = 0;
+  sub_tile<FN, WM, WN>(t, 0, 0, &g, Bases{});
 }
 
 }  // namespace
 
+// Tiles of 32 x 32 once they fill the SMs three times over, else of 16 x 16
+// (the same sums): the operands' traffic is no bound at either size, idle SMs
+// are.
 cudaError_t launch_gemm_f64_dense(bool transA, int M, int N, int K, const double* A, int lda, const double* B,
-                                  int ldb, double* C, int ldc, int cls, cudaStream_t stream) {
+                                  int ldb, double* C, int ldc, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return cudaSuccess;
-  if (cls < 0 || cls >= kTileClasses) return cudaErrorInvalidValue;
-  const dim3 grid((M + kTileClassM[cls] - 1) / kTileClassM[cls], (N + kTileClassN[cls] - 1) / kTileClassN[cls]);
-  gemm_f64_dense<<<grid, kThreads, 0, stream>>>(transA ? 1 : 0, M, N, K, A, lda, B, ldb, C, ldc, cls);
+  const dim3 big((M + 31) / 32, (N + 31) / 32), small((M + 15) / 16, (N + 15) / 16);
+  if ((int64_t)big.x * big.y >= 3 * kF64Sms)
+    gemm_f64_dense<2, 4, 2><<<big, 256, 0, stream>>>(transA ? 1 : 0, M, N, K, A, lda, B, ldb, C, ldc);
+  else
+    gemm_f64_dense<1, 2, 2><<<small, 128, 0, stream>>>(transA ? 1 : 0, M, N, K, A, lda, B, ldb, C, ldc);
   return cudaGetLastError();
 }
 
-cudaError_t launch_gemm_f64(const GemmTile* tiles, int ntiles, const GemmSeg* segs, const Bases& bases,
+cudaError_t launch_gemm_f64(const GemmTile* tiles, const F64Counts& n, const GemmSeg* segs, const Bases& bases,
                             cudaStream_t stream) {
-  if (ntiles <= 0) return cudaSuccess;
-  gemm_f64_tiles<<<ntiles, kThreads, 0, stream>>>(tiles, segs, bases);
+  if (n.whole > 0) gemm_f64_tiles<<<n.whole, kThreads, 0, stream>>>(tiles, segs, bases);
+  tiles += n.whole;
+  if (n.split > 0) gemm_f64_ksplit<<<n.split, kThreads, 0, stream>>>(tiles, segs, bases);
   return cudaGetLastError();
 }
 

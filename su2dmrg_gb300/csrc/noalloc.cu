@@ -104,9 +104,15 @@ extern "C" int su2g_hamiltonian_vector_multiplication_noalloc(const int* vec_des
   int dev = 0;
   rc = device_arrays(&d, &dev);
   if (rc) return rc;
+  // the launched tiles, where the fixed arrays hold them (else the planner's)
+  std::vector<su2g::GemmTile> l1 = su2g::f64_launch_tiles(w.tile1), l2 = su2g::f64_launch_tiles(w.tile2);
+  if (l1.size() + l2.size() > SU2G_NOALLOC_MAX_TILES) {
+    l1.swap(w.tile1);
+    l2.swap(w.tile2);
+  }
   // one work list: phase-2 tiles index the segments after phase 1's
-  std::vector<su2g::GemmTile> tiles(w.tile1);
-  for (su2g::GemmTile t : w.tile2) {
+  std::vector<su2g::GemmTile> tiles(l1);
+  for (su2g::GemmTile t : l2) {
     t.seg0 += (int)w.seg1.size();
     tiles.push_back(t);
   }
@@ -131,8 +137,8 @@ extern "C" int su2g_hamiltonian_vector_multiplication_noalloc(const int* vec_des
   b.p[su2g::kBufPsi] = reinterpret_cast<uintptr_t>(vec);
   b.p[su2g::kBufY] = reinterpret_cast<uintptr_t>(y);
   b.p[su2g::kBufScratch] = reinterpret_cast<uintptr_t>(d.scratch);
-  if (e == cudaSuccess) e = su2g::launch_gemm_f64(d.tiles, (int)w.tile1.size(), d.segs, b, st);
-  if (e == cudaSuccess) e = su2g::launch_gemm_f64(d.tiles + w.tile1.size(), (int)w.tile2.size(), d.segs, b, st);
+  if (e == cudaSuccess) e = su2g::launch_gemm_f64(d.tiles, su2g::f64_counts(l1), d.segs, b, st);
+  if (e == cudaSuccess) e = su2g::launch_gemm_f64(d.tiles + l1.size(), su2g::f64_counts(l2), d.segs, b, st);
   if (e != cudaSuccess) return fail(SU2G_ECUDA, std::string("noalloc: ") + cudaGetErrorString(e));
   return SU2G_OK;
 }

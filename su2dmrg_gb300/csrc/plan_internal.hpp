@@ -19,6 +19,8 @@ struct su2g_heff_plan {
   su2g::GemmSeg* d_seg2 = nullptr;
   su2g::GemmTile* d_tile1 = nullptr;
   su2g::GemmTile* d_tile2 = nullptr;
+  std::vector<su2g::GemmTile> launch1, launch2;  // the tiles the FP64 phases launch (f64_launch_tiles)
+  su2g::F64Counts count1, count2;
   double* d_scratch = nullptr;
   // split-precision work (S > 0)
   int S = 0;

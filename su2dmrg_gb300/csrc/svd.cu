@@ -280,7 +280,7 @@ struct Ctx {
             int ldc) {
     if (!ok() || M == 0 || N == 0) return;
     const cudaError_t e =
-        su2g::launch_gemm_f64_dense(transA, M, N, K, A, lda, B, ldb, C, ldc, su2g::tile_class_for(M, N), st);
+        su2g::launch_gemm_f64_dense(transA, M, N, K, A, lda, B, ldb, C, ldc, st);
     if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
   }
   // out (cols x rows) = in^T (in: rows x cols, column-major)
