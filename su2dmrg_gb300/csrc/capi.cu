@@ -901,57 +901,28 @@ struct LanczosCtx {
   double* ff(int i) { return p->d_krylov + (int64_t)i * n; }
   double* tmp() { return p->d_krylov + (int64_t)(p->krylov_vectors - 1) * n; }
 
-  int dot(const double* x, const double* y, double* out) {
-    const int ns = su2g::reduction_scratch_doubles();
-    cudaError_t e = su2g::launch_dot(x, y, n, p->d_red, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, p->d_red + ns - 1, sizeof(double), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_fail(e, "lanczos dot");
-    return SU2G_OK;
-  }
   int matvec(const double* x, double* y) {
     ++nmatvec;
     return su2g::heff_apply_impl(p, x, y, st);
-  }
-  int axpy(double a, const double* x, double* y) {
-    cudaError_t e = su2g::launch_axpy(a, x, y, n, st);
-    return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos axpy");
-  }
-  int scale(double a, double* x) {
-    cudaError_t e = su2g::launch_scale(a, x, n, st);
-    return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos scale");
   }
   int copy(const double* x, double* y) {
     cudaError_t e = cudaMemcpyAsync(y, x, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
     return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos copy");
   }
 
-  // ---- device-side coefficients: alpha[j], beta[j], q[j] (reorthogonalisation), nn ----
+  // ---- device-side coefficients: alpha[j], beta[j], q[j] (reorthogonalisation) ----
   int M() const { return p->lcoef_m; }
   double* alpha(int j) { return p->d_lcoef + j; }
   double* beta(int j) { return p->d_lcoef + M() + 1 + j; }
   double* q(int j) { return p->d_lcoef + 2 * (M() + 1) + j; }
-  double* nnd() { return p->d_lcoef + 3 * (M() + 1); }
 
   // Enqueues the Lanczos step that produces ff[m] on stream s (lanczos_su2.cpp:136-142
   // for m = 1, :156-173 for m >= 2): matvec, alpha[m-1], the two three-term
   // updates, full reorthogonalisation against ff[0..m-1], beta[m] and the
-  // normalisation -- the same kernels in the same order as the host-driven
-  // sequence, with every scalar kept on the device.
+  // normalisation, with every scalar kept on the device.
   cudaError_t enqueue_step(int m, cudaStream_t s) {
     if (su2g::heff_apply_impl(p, ff(m - 1), ff(m), s) != SU2G_OK) return cudaErrorUnknown;
-    cudaError_t e = su2g::launch_dot_to(ff(m - 1), ff(m), n, p->d_red, alpha(m - 1), s);
-    if (e == cudaSuccess) e = su2g::launch_axpy_neg_dev(alpha(m - 1), ff(m - 1), ff(m), n, s);
-    if (m >= 2) {
-      if (e == cudaSuccess) e = su2g::launch_axpy_neg_dev(beta(m - 1), ff(m - 2), ff(m), n, s);
-      for (int j = 0; j < m && e == cudaSuccess; ++j) {
-        e = su2g::launch_dot_to(ff(m), ff(j), n, p->d_red, q(j), s);
-        if (e == cudaSuccess) e = su2g::launch_axpy_neg_dev(q(j), ff(j), ff(m), n, s);
-      }
-    }
-    if (e == cudaSuccess) e = su2g::launch_dot_to(ff(m), ff(m), n, p->d_red, nnd(), s);
-    if (e == cudaSuccess) e = su2g::launch_normalize_dev(nnd(), ff(m), n, beta(m), s);
-    return e;
+    return su2g::launch_lanczos_tail(m, ff(0), n, n, alpha(0), beta(0), q(0), p->d_red, s);
   }
   // the final matvec and its alpha (lanczos_su2.cpp:189-194)
   cudaError_t enqueue_last(int m, cudaStream_t s) {
@@ -988,27 +959,27 @@ struct LanczosCtx {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos fetch");
   }
-  // vout = sum_j z[j] ff[j]  (lanczos_su2::compute_eigenvector, lanczos_su2.cpp:262-279)
+  // vout = sum_j z[j] ff[j]  (lanczos_su2::compute_eigenvector, lanczos_su2.cpp:262-279);
+  // leaves the partial sums of its norm in half 0 of the scratch
   int combine(const std::vector<double>& z, int m, double* vout) {
-    int rc = copy(ff(0), vout);
-    if (!rc) rc = scale(z[0], vout);
-    for (int j = 1; j < m && !rc; ++j) rc = axpy(z[j], ff(j), vout);
-    return rc;
+    cudaError_t e = su2g::launch_combine_vectors(z.data(), m, ff(0), n, vout, n, p->d_red, 0, st);
+    return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos combine");
   }
-  // lanczos_su2::check_eigenvector (lanczos_su2.cpp:320-332): normalises v,
-  // returns |Hv| and |<Hv,v>|/|Hv|
+  // lanczos_su2::check_eigenvector (lanczos_su2.cpp:320-332) of the vector
+  // combine() just left in v: normalises it, returns |Hv| and |<Hv,v>|/|Hv|
   int check(double* v, double* eig, double* olap) {
-    double nn;
-    int rc = dot(v, v, &nn);
-    if (!rc) rc = scale(1.0 / std::sqrt(nn), v);
-    if (!rc) rc = matvec(v, tmp());
-    double pp = 0, ov = 0;
-    if (!rc) rc = dot(tmp(), tmp(), &pp);
-    if (!rc) rc = dot(tmp(), v, &ov);
+    cudaError_t e = su2g::launch_normalize_part(p->d_red, 0, v, n, nullptr, st);
+    if (e != cudaSuccess) return cuda_fail(e, "lanczos check");
+    int rc = matvec(v, tmp());
     if (rc) return rc;
-    const double prod = std::sqrt(pp);
+    e = su2g::launch_dot2(tmp(), v, n, p->d_red, st);
+    if (e != cudaSuccess) return cuda_fail(e, "lanczos check");
+    double r[2];  // |Hv|^2, <Hv,v>
+    rc = fetch(p->d_red + su2g::lanczos_scratch_doubles() - 2, r, 2);
+    if (rc) return rc;
+    const double prod = std::sqrt(r[0]);
     *eig = prod;
-    *olap = std::fabs(ov / prod);
+    *olap = std::fabs(r[1] / prod);
     return SU2G_OK;
   }
 };
@@ -1029,13 +1000,13 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
     SU2G_CUDA(dalloc(&p->d_krylov, (size_t)need * n * sizeof(double)));
     p->krylov_vectors = need;
   }
-  if (!p->d_red) SU2G_CUDA(dalloc(&p->d_red, su2g::reduction_scratch_doubles() * sizeof(double)));
+  if (!p->d_red) SU2G_CUDA(dalloc(&p->d_red, su2g::lanczos_scratch_doubles() * sizeof(double)));
   if (p->lcoef_m < mlanc) {
     p->drop_graphs();
     su2g::dev_free(p->d_lcoef, p->last_st);
     p->d_lcoef = nullptr;
     p->lcoef_m = 0;
-    SU2G_CUDA(dalloc(&p->d_lcoef, (size_t)(3 * (mlanc + 1) + 1) * sizeof(double)));
+    SU2G_CUDA(dalloc(&p->d_lcoef, (size_t)(3 * (mlanc + 1)) * sizeof(double)));
     p->lcoef_m = mlanc;
   }
   p->last_st = (cudaStream_t)stream;
@@ -1043,11 +1014,14 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
   const double tol = 1.e-6;  // lanczos_su2.cpp:128
   std::vector<double> aal(mlanc, 0.0), nnl(mlanc + 1, 0.0), eig, z;
   int rc;
-  // alpha[0..m-1] and beta[1..m] to the host (one copy each)
+  // alpha[0..m-1] and beta[1..m] to the host (they lie in one block: one copy)
+  std::vector<double> coefs(2 * (L.M() + 1));
   auto fetch_coefs = [&](int m) -> int {
-    int r = L.fetch(L.alpha(0), aal.data(), m);
-    if (!r && m >= 1) r = L.fetch(L.beta(1), nnl.data() + 1, m);
-    return r;
+    const int r = L.fetch(L.alpha(0), coefs.data(), L.M() + 1 + m + 1);
+    if (r) return r;
+    std::copy(coefs.begin(), coefs.begin() + m, aal.begin());
+    std::copy(coefs.begin() + L.M() + 2, coefs.begin() + L.M() + 2 + m, nnl.begin() + 1);
+    return SU2G_OK;
   };
   auto tridiag = [&](int m) {  // lanczos_su2::diatridiag (lanczos_su2.cpp:237-259)
     std::vector<double> d(aal.begin(), aal.begin() + m), e(m > 1 ? m - 1 : 0);
@@ -1075,8 +1049,8 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
 
   // ff[0] = normalised start vector (lanczos_su2.cpp:45-46)
   if ((rc = L.copy(psi, L.ff(0)))) return rc;
-  SU2G_CUDA(su2g::launch_dot_to(L.ff(0), L.ff(0), n, p->d_red, L.nnd(), L.st));
-  SU2G_CUDA(su2g::launch_normalize_dev(L.nnd(), L.ff(0), n, L.beta(0), L.st));
+  SU2G_CUDA(su2g::launch_dot_partial(L.ff(0), L.ff(0), n, p->d_red, 0, L.st));
+  SU2G_CUDA(su2g::launch_normalize_part(p->d_red, 0, L.ff(0), n, L.beta(0), L.st));
   // first step (lanczos_su2.cpp:136-142)
   if ((rc = L.run_graph(false, 1))) return rc;
   if (mlanc == 2) {  // lanczos_su2.cpp:143-154

@@ -105,7 +105,7 @@ struct su2g_heff_batch {
   double* d_red = nullptr;
   cudaStream_t last_st = nullptr;
 
-  int coef_len() const { return 3 * (kry_m + 1) + 1; }
+  int coef_len() const { return 3 * (kry_m + 1); }
   double* ff(int m) { return d_kry + (int64_t)m * total; }
   double* tmpv() { return d_kry + (int64_t)(kry_m + 1) * total; }
   double* stage() { return d_kry + (int64_t)(kry_m + 2) * total; }
@@ -308,11 +308,10 @@ struct Solve {
   int nmv = 0;
   double energy = 0.0;
   enum { kNone, kFinal, kEarly } pending = kNone;
-  double nn = 0, pp = 0, ov = 0;  // check() scalars
+  double pp = 0, ov = 0;  // check() scalars
   double* alpha(int j) { return coef + j; }
   double* beta(int j) { return coef + M + 1 + j; }
   double* q(int j) { return coef + 2 * (M + 1) + j; }
-  double* nnd() { return coef + 3 * (M + 1); }
 };
 
 }  // namespace
@@ -401,7 +400,7 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
     s.mlanc = mlanc > s.n ? (int)s.n + 1 : mlanc;  // dmrg_su2.cpp:532
     M = std::max(M, s.mlanc);
   }
-  const int ns = su2g::reduction_scratch_doubles();
+  const int ns = su2g::lanczos_scratch_doubles();
   if (B->kry_m < M) {
     su2g::dev_free(B->d_kry, st);
     su2g::dev_free(B->d_coef, st);
@@ -425,8 +424,8 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
   for (Solve& s : sv) {
     double* f0 = slice(B->ff(0), s);
     BATCH_CUDA(cudaMemcpyAsync(f0, s.psi, s.n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    BATCH_CUDA(su2g::launch_dot_to(f0, f0, s.n, s.red, s.nnd(), st));
-    BATCH_CUDA(su2g::launch_normalize_dev(s.nnd(), f0, s.n, s.beta(0), st));
+    BATCH_CUDA(su2g::launch_dot_partial(f0, f0, s.n, s.red, 0, st));
+    BATCH_CUDA(su2g::launch_normalize_part(s.red, 0, f0, s.n, s.beta(0), st));
   }
   // host copies of the device scalars of several solves, one synchronisation
   std::vector<double> hbuf;
@@ -437,26 +436,18 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
   };
   // psi = sum_j z[j] ff[j]  (lanczos_su2::compute_eigenvector, lanczos_su2.cpp:262-279)
   auto combine = [&](Solve& s, int m) -> int {
-    BATCH_CUDA(cudaMemcpyAsync(s.psi, slice(B->ff(0), s), s.n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    BATCH_CUDA(su2g::launch_scale(s.z[0], s.psi, s.n, st));
-    for (int j = 1; j < m; ++j) BATCH_CUDA(su2g::launch_axpy(s.z[j], slice(B->ff(j), s), s.psi, s.n, st));
+    BATCH_CUDA(su2g::launch_combine_vectors(s.z.data(), m, slice(B->ff(0), s), B->total, s.psi, s.n, s.red, 0, st));
     return SU2G_OK;
   };
   // lanczos_su2::check_eigenvector (lanczos_su2.cpp:320-332) for every solve
-  // in `who`: normalise psi, one shared matvec, |Hv| and |<Hv,v>|/|Hv|
+  // in `who`, whose vector combine() just formed: normalise psi, one shared
+  // matvec, |Hv| and |<Hv,v>|/|Hv|
   auto checks = [&](const std::vector<int>& who) -> int {
     if (who.empty()) return SU2G_OK;
     hbuf.assign(2 * who.size(), 0.0);
     for (size_t k = 0; k < who.size(); ++k) {
       Solve& s = sv[who[k]];
-      BATCH_CUDA(su2g::launch_dot(s.psi, s.psi, s.n, s.red, st));
-      BATCH_CUDA(cudaMemcpyAsync(&hbuf[k], s.red + ns - 1, sizeof(double), cudaMemcpyDeviceToHost, st));
-    }
-    BATCH_CUDA(cudaStreamSynchronize(st));
-    for (size_t k = 0; k < who.size(); ++k) {
-      Solve& s = sv[who[k]];
-      s.nn = hbuf[k];
-      BATCH_CUDA(su2g::launch_scale(1.0 / std::sqrt(s.nn), s.psi, s.n, st));
+      BATCH_CUDA(su2g::launch_normalize_part(s.red, 0, s.psi, s.n, nullptr, st));
       BATCH_CUDA(cudaMemcpyAsync(slice(B->stage(), s), s.psi, s.n * sizeof(double), cudaMemcpyDeviceToDevice, st));
       ++s.nmv;
     }
@@ -465,10 +456,8 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
     for (size_t k = 0; k < who.size(); ++k) {
       Solve& s = sv[who[k]];
       double* t = slice(B->tmpv(), s);
-      BATCH_CUDA(su2g::launch_dot(t, t, s.n, s.red, st));
-      BATCH_CUDA(cudaMemcpyAsync(&hbuf[2 * k], s.red + ns - 1, sizeof(double), cudaMemcpyDeviceToHost, st));
-      BATCH_CUDA(su2g::launch_dot(t, s.psi, s.n, s.red, st));
-      BATCH_CUDA(cudaMemcpyAsync(&hbuf[2 * k + 1], s.red + ns - 1, sizeof(double), cudaMemcpyDeviceToHost, st));
+      BATCH_CUDA(su2g::launch_dot2(t, s.psi, s.n, s.red, st));
+      BATCH_CUDA(cudaMemcpyAsync(&hbuf[2 * k], s.red + ns - 2, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     BATCH_CUDA(cudaStreamSynchronize(st));
     for (size_t k = 0; k < who.size(); ++k) {
@@ -490,20 +479,11 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
     if (rc) return rc;
     for (int i : act) {
       Solve& s = sv[i];
-      double* fm = slice(B->ff(m), s);
-      double* fm1 = slice(B->ff(m - 1), s);
-      BATCH_CUDA(su2g::launch_dot_to(fm1, fm, s.n, s.red, s.alpha(m - 1), st));
-      if (m == s.mlanc) continue;  // the final matvec: alpha only (lanczos_su2.cpp:189-194)
-      BATCH_CUDA(su2g::launch_axpy_neg_dev(s.alpha(m - 1), fm1, fm, s.n, st));
-      if (m >= 2) {  // lanczos_su2.cpp:156-173
-        BATCH_CUDA(su2g::launch_axpy_neg_dev(s.beta(m - 1), slice(B->ff(m - 2), s), fm, s.n, st));
-        for (int j = 0; j < m; ++j) {
-          BATCH_CUDA(su2g::launch_dot_to(fm, slice(B->ff(j), s), s.n, s.red, s.q(j), st));
-          BATCH_CUDA(su2g::launch_axpy_neg_dev(s.q(j), slice(B->ff(j), s), fm, s.n, st));
-        }
-      }
-      BATCH_CUDA(su2g::launch_dot_to(fm, fm, s.n, s.red, s.nnd(), st));
-      BATCH_CUDA(su2g::launch_normalize_dev(s.nnd(), fm, s.n, s.beta(m), st));
+      if (m == s.mlanc)  // the final matvec: alpha only (lanczos_su2.cpp:189-194)
+        BATCH_CUDA(su2g::launch_dot_to(slice(B->ff(m - 1), s), slice(B->ff(m), s), s.n, s.red, s.alpha(m - 1), st));
+      else
+        BATCH_CUDA(su2g::launch_lanczos_tail(m, slice(B->ff(0), s), B->total, s.n, s.alpha(0), s.beta(0), s.q(0),
+                                             s.red, st));
     }
     // alpha[0..m-1], beta[1..m] of every active solve to the host
     for (int i : act) {

@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "gemm_work.hpp"
 #include "kernels.hpp"
@@ -257,34 +258,174 @@ namespace {
 constexpr int kRedBlocks = 512;  // fixed: the summation order never depends on the device
 constexpr int kRedThreads = 256;
 
+// the sum of a block's values, valid in thread 0: sh[t] += sh[t + s] for
+// s = 128 .. 1, the last five steps inside warp 0
 __device__ __forceinline__ double block_sum(double v, double* sh) {
   const int tid = threadIdx.x;
+  __syncthreads();  // sh may still be read from an earlier sum
   sh[tid] = v;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (tid < s) sh[tid] += sh[tid + s];
+#pragma unroll
+  for (int s = kRedThreads / 2; s >= 32; s >>= 1) {
+    if (tid < s) sh[tid] = v = v + sh[tid + s];
     __syncthreads();
   }
-  return sh[0];
+  if (tid < 32) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
+  }
+  return v;
+}
+
+// a dot product's value from its kRedBlocks partial sums, in every thread
+__device__ __forceinline__ double sum_partials(const double* __restrict__ part, double* sh) {
+  double v = 0;
+#pragma unroll
+  for (int i = 0; i < kRedBlocks; i += kRedThreads) v += part[i + threadIdx.x];
+  v = block_sum(v, sh);
+  if (threadIdx.x == 0) sh[0] = v;
+  __syncthreads();
+  v = sh[0];
+  return v;
+}
+
+// Elements of a block's share in order, four in flight: f(i, count) handles
+// the elements i, i + stride, ..., count of them (four, or the last one by one).
+template <class F>
+__device__ __forceinline__ void grid_stride4(int64_t n, F f) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < n; i += 4 * stride) f(i, stride, std::integral_constant<int, 4>());
+  for (; i < n; i += stride) f(i, stride, std::integral_constant<int, 1>());
 }
 
 __global__ void __launch_bounds__(kRedThreads) dot_partial(const double* __restrict__ x, const double* __restrict__ y,
                                                           int64_t n, double* __restrict__ part) {
   __shared__ double sh[kRedThreads];
   double v = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v += x[i] * y[i];
+  grid_stride4(n, [&](int64_t i, int64_t stride, auto U) {
+    double a[U.value], b[U.value];
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) a[u] = x[i + u * stride], b[u] = y[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) v += a[u] * b[u];
+  });
   const double s = block_sum(v, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-__global__ void __launch_bounds__(kRedThreads) dot_final(const double* __restrict__ part, int nparts,
-                                                        double* __restrict__ out) {
+// x . x and x . y in one pass
+__global__ void __launch_bounds__(kRedThreads) dot2_partial(const double* __restrict__ x, const double* __restrict__ y,
+                                                           int64_t n, double* __restrict__ part) {
   __shared__ double sh[kRedThreads];
+  double v = 0, w = 0;
+  grid_stride4(n, [&](int64_t i, int64_t stride, auto U) {
+    double a[U.value], b[U.value];
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) a[u] = x[i + u * stride], b[u] = y[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) v += a[u] * a[u], w += a[u] * b[u];
+  });
+  const double s = block_sum(v, sh), t = block_sum(w, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s, part[kRedBlocks + blockIdx.x] = t;
+}
+
+// out[b] = the value of the dot product whose partial sums are part[b kRedBlocks ..]
+__global__ void __launch_bounds__(kRedThreads) dot_final(const double* __restrict__ part, double* __restrict__ out) {
+  __shared__ double sh[kRedThreads];
+  const double s = sum_partials(part + blockIdx.x * kRedBlocks, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
+// One update of the Lanczos recurrence and the reduction the next one needs:
+//     c = the dot product whose partial sums are part_in;  *c_out = c
+//     y -= c x0;  y -= (*c1) x1 (c1 null: not);  part_out = partial sums of y . z
+// (z null: y . y).  Every block sums the 512 partials itself (4 KB from L2, in
+// the order of dot_final), so a coefficient costs no launch and no round trip
+// of its own.  Bound by launch and L2 latency up to D = 600 or so, then by the
+// passes over y, x0 and z.  A step that orthogonalises against m vectors is
+// m + 3 launches where a dot product, its final sum and an update apiece were
+// 3 m + 7; with the eigenvector's combination below in one launch, a solve on
+// a kept plan (five vectors, seven matvecs) takes 547 us instead of 797 at
+// D = 123 in FP64 and 2459 instead of 2704 at D = 600 with 7 slices.  The
+// same operations on the same values in the same order.
+__global__ void __launch_bounds__(kRedThreads) update_dot_kernel(const double* __restrict__ part_in, double* c_out,
+                                                                const double* __restrict__ x0,
+                                                                const double* __restrict__ c1,
+                                                                const double* __restrict__ x1, double* y,
+                                                                const double* z, int64_t n,
+                                                                double* __restrict__ part_out) {
+  __shared__ double sh[kRedThreads];
+  if ((int64_t)blockIdx.x * kRedThreads >= n) {  // no element here
+    if (threadIdx.x == 0) part_out[blockIdx.x] = 0.0;
+    return;
+  }
+  const double c = sum_partials(part_in, sh);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *c_out = c;
+  const double a0 = -c, a1 = c1 ? -*c1 : 0.0;
   double v = 0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) v += part[i];
+  grid_stride4(n, [&](int64_t i, int64_t stride, auto U) {
+    double f[U.value], g[U.value], h[U.value], w[U.value];
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) {
+      const int64_t k = i + u * stride;
+      f[u] = y[k];
+      g[u] = x0[k];
+      h[u] = c1 ? x1[k] : 0.0;
+      w[u] = z ? z[k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) {
+      double t = fma(a0, g[u], f[u]);
+      if (c1) t = fma(a1, h[u], t);
+      y[i + u * stride] = t;
+      v += t * (z ? w[u] : t);
+    }
+  });
   const double s = block_sum(v, sh);
-  if (threadIdx.x == 0) *out = s;
+  if (threadIdx.x == 0) part_out[blockIdx.x] = s;
+}
+
+// b = sqrt of the dot product whose partial sums are part_in, x *= 1 / b
+// (b_out null: not stored)
+__global__ void __launch_bounds__(kRedThreads) normalize_part_kernel(const double* __restrict__ part_in,
+                                                                    double* __restrict__ x, int64_t n,
+                                                                    double* b_out) {
+  __shared__ double sh[kRedThreads];
+  if ((int64_t)blockIdx.x * kRedThreads >= n) return;
+  const double b = sqrt(sum_partials(part_in, sh));
+  const double f = 1.0 / b;
+  if (b_out && blockIdx.x == 0 && threadIdx.x == 0) *b_out = b;
+  grid_stride4(n, [&](int64_t i, int64_t stride, auto U) {
+    double t[U.value];
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) t[u] = x[i + u * stride];
+#pragma unroll
+    for (int u = 0; u < U.value; ++u) x[i + u * stride] = t[u] * f;
+  });
+}
+
+// v = z_0 f_0 + z_1 f_1 + ... (f_j = f + j stride), added in that order
+// (first: v starts from z_0 f_0, else from v); part: partial sums of v . v
+constexpr int kCombineMax = 16;
+struct CombineCoefs {
+  double z[kCombineMax];
+};
+__global__ void __launch_bounds__(kRedThreads) combine_vectors_kernel(CombineCoefs c, int m, bool first,
+                                                                     const double* __restrict__ f, int64_t stride_f,
+                                                                     double* __restrict__ v, int64_t n,
+                                                                     double* __restrict__ part) {
+  __shared__ double sh[kRedThreads];
+  double s = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double t = first ? __dmul_rn(c.z[0], f[i]) : fma(c.z[0], f[i], v[i]);
+#pragma unroll 4
+    for (int j = 1; j < m; ++j) t = fma(c.z[j], f[j * stride_f + i], t);
+    v[i] = t;
+    s += t * t;
+  }
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
 __global__ void axpy_kernel(double alpha, const double* __restrict__ x, double* __restrict__ y, int64_t n) {
@@ -300,56 +441,75 @@ __global__ void scale_kernel(double alpha, double* __restrict__ x, int64_t n) {
 }  // namespace
 
 int reduction_scratch_doubles() { return kRedBlocks + 1; }
+int lanczos_scratch_doubles() { return 2 * kRedBlocks + 2; }
 
 cudaError_t launch_dot(const double* x, const double* y, int64_t n, double* scratch, cudaStream_t stream) {
-  dot_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  dot_final<<<1, kRedThreads, 0, stream>>>(scratch, kRedBlocks, scratch + kRedBlocks);
-  return cudaGetLastError();
+  return launch_dot_to(x, y, n, scratch, scratch + kRedBlocks, stream);
 }
 
 cudaError_t launch_dot_to(const double* x, const double* y, int64_t n, double* scratch, double* out,
                           cudaStream_t stream) {
-  dot_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_dot_partial(x, y, n, scratch, 0, stream);
   if (e != cudaSuccess) return e;
-  dot_final<<<1, kRedThreads, 0, stream>>>(scratch, kRedBlocks, out);
+  dot_final<<<1, kRedThreads, 0, stream>>>(scratch, out);
   return cudaGetLastError();
 }
 
-// y -= (*c) x, the coefficient read on the device
-__global__ void axpy_neg_dev_kernel(const double* __restrict__ c, const double* __restrict__ x, double* __restrict__ y,
-                                    int64_t n) {
-  const double a = -*c;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] += a * x[i];
-}
-
-// b = sqrt(*nn), *b_out = b, x *= 1 / b
-__global__ void normalize_dev_kernel(const double* __restrict__ nn, double* __restrict__ x, int64_t n,
-                                     double* __restrict__ b_out) {
-  const double b = sqrt(*nn);
-  const double f = 1.0 / b;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *b_out = b;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    x[i] *= f;
-}
-
-cudaError_t launch_axpy_neg_dev(const double* c, const double* x, double* y, int64_t n, cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 4 * 152 * 4) blocks = 4 * 152 * 4;
-  axpy_neg_dev_kernel<<<blocks, 256, 0, stream>>>(c, x, y, n);
+cudaError_t launch_dot_partial(const double* x, const double* y, int64_t n, double* scratch, int half,
+                               cudaStream_t stream) {
+  dot_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch + half * kRedBlocks);
   return cudaGetLastError();
 }
 
-cudaError_t launch_normalize_dev(const double* nn, double* x, int64_t n, double* b_out, cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 4 * 152 * 4) blocks = 4 * 152 * 4;
-  normalize_dev_kernel<<<blocks, 256, 0, stream>>>(nn, x, n, b_out);
+cudaError_t launch_update_dot(double* scratch, int half, double* c_out, const double* x0, const double* c1,
+                              const double* x1, double* y, const double* z, int64_t n, cudaStream_t stream) {
+  update_dot_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(scratch + half * kRedBlocks, c_out, x0, c1, x1, y, z, n,
+                                                            scratch + (1 - half) * kRedBlocks);
   return cudaGetLastError();
+}
+
+cudaError_t launch_normalize_part(const double* scratch, int half, double* x, int64_t n, double* b_out,
+                                  cudaStream_t stream) {
+  normalize_part_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(scratch + half * kRedBlocks, x, n, b_out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_combine_vectors(const double* z, int m, const double* f, int64_t stride_f, double* v, int64_t n,
+                                   double* scratch, int half, cudaStream_t stream) {
+  for (int j0 = 0; j0 < m; j0 += kCombineMax) {
+    CombineCoefs c{};
+    const int k = std::min(kCombineMax, m - j0);
+    std::copy(z + j0, z + j0 + k, c.z);
+    combine_vectors_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(c, k, j0 == 0, f + j0 * stride_f, stride_f, v, n,
+                                                                  scratch + half * kRedBlocks);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_dot2(const double* x, const double* y, int64_t n, double* scratch, cudaStream_t stream) {
+  dot2_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch);
+  dot_final<<<2, kRedThreads, 0, stream>>>(scratch, scratch + 2 * kRedBlocks);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_lanczos_tail(int m, double* f, int64_t stride_f, int64_t n, double* alpha, double* beta, double* q,
+                                double* scratch, cudaStream_t stream) {
+  auto ff = [&](int j) { return f + j * stride_f; };
+  double* y = ff(m);
+  cudaError_t e = launch_dot_partial(ff(m - 1), y, n, scratch, 0, stream);
+  int half = 0;
+  if (m < 2) {
+    if (e == cudaSuccess) e = launch_update_dot(scratch, half, alpha + m - 1, ff(0), nullptr, nullptr, y, nullptr, n, stream);
+    half ^= 1;
+  } else {
+    if (e == cudaSuccess)
+      e = launch_update_dot(scratch, half, alpha + m - 1, ff(m - 1), beta + m - 1, ff(m - 2), y, ff(0), n, stream);
+    half ^= 1;
+    for (int j = 0; j < m && e == cudaSuccess; ++j, half ^= 1)
+      e = launch_update_dot(scratch, half, q + j, ff(j), nullptr, nullptr, y, j + 1 < m ? ff(j + 1) : nullptr, n, stream);
+  }
+  if (e == cudaSuccess) e = launch_normalize_part(scratch, half, y, n, beta + m, stream);
+  return e;
 }
 
 cudaError_t launch_axpy(double alpha, const double* x, double* y, int64_t n, cudaStream_t stream) {
