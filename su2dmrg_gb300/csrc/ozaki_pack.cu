@@ -1,10 +1,10 @@
 // Splitting of FP64 operands into BF16 digit slices (layout in ozaki.hpp), in
 // two launches: the row exponents (one warp per row), then the digits (one CTA
-// per row tile and 64 k).  The scaling and rounding to integers use integer
-// operations only (FP64 throughput is scarce on GB300).
+// per row tile and 32 k).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "kernels.hpp"
@@ -55,7 +55,7 @@ template <>
 constexpr long long kDigitBias<0> = 0;
 
 constexpr int kRowsPerUnit = kTM;  // row slots per unit in the row kernel (RT <= 128)
-constexpr int kDigitKt = 4;        // k tiles (16 k each) per CTA of the digit kernel
+constexpr int kDigitKt = 2;        // k tiles (16 k each) per CTA of the digit kernel
 
 // Row exponents: one warp per row of every unit, lanes along k (coalesced):
 // |alpha X| 2^-e < 1/2 with e = ilogb(max |alpha X|) + 2, kExpZero for a zero row.
@@ -71,19 +71,22 @@ __global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob* 
   if (row >= job.rt || job.rowmax >= 0) return;  // row maxima left by the producing GEMM
   const int r = u.y * job.rt + row;
   unsigned long long m = 0;  // max |x| as a bit pattern (order-preserving for |x|)
+  // the sign comes off the high word alone: masking the 64 bits compiles to an
+  // FP64 |x|, sixteen clocks a warp
+  auto bits = [](double x) {
+    unsigned hi;
+    asm("and.b32 %0, %1, 0x7FFFFFFF;" : "=r"(hi) : "r"(__double2hiint(x)));
+    return ((unsigned long long)hi << 32) | (unsigned)__double2loint(x);
+  };
   if (r < job.R) {
     const double* p = resolve(bases, job.src_buf, job.src) + (int64_t)r * job.ld_r;
     int k = lane;
     for (; k + 96 < job.K; k += 128) {  // four loads in flight
-      const unsigned long long a = __double_as_longlong(p[(int64_t)k * job.ld_k]);
-      const unsigned long long b = __double_as_longlong(p[(int64_t)(k + 32) * job.ld_k]);
-      const unsigned long long c = __double_as_longlong(p[(int64_t)(k + 64) * job.ld_k]);
-      const unsigned long long d = __double_as_longlong(p[(int64_t)(k + 96) * job.ld_k]);
-      m = max(m, max(max(a & 0x7FFFFFFFFFFFFFFFull, b & 0x7FFFFFFFFFFFFFFFull),
-                     max(c & 0x7FFFFFFFFFFFFFFFull, d & 0x7FFFFFFFFFFFFFFFull)));
+      const double a = p[(int64_t)k * job.ld_k], b = p[(int64_t)(k + 32) * job.ld_k];
+      const double c = p[(int64_t)(k + 64) * job.ld_k], d = p[(int64_t)(k + 96) * job.ld_k];
+      m = max(m, max(max(bits(a), bits(b)), max(bits(c), bits(d))));
     }
-    for (; k < job.K; k += 32)
-      m = max(m, (unsigned long long)__double_as_longlong(p[(int64_t)k * job.ld_k]) & 0x7FFFFFFFFFFFFFFFull);
+    for (; k < job.K; k += 32) m = max(m, bits(p[(int64_t)k * job.ld_k]));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -101,24 +104,101 @@ __global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob* 
   }
 }
 
-// Digits: one CTA per (unit, kDigitKt k tiles); a warp converts 8 rows x 32 k,
-// a thread one row x 8 k into S 16-byte core rows, so that a warp's stores
-// fill whole 256-byte core-row groups.  The k-chunk-0 CTA also records the
-// row tile's largest exponent.
+// Digits: one CTA per (unit, `span` times kDigitKt k tiles); a warp converts 8
+// rows x 32 k at a time, a thread one row x 8 k into S 16-byte core rows, so
+// that a warp's stores fill whole 256-byte core-row groups.  The k-chunk-0 CTA
+// also records the row tile's largest exponent.
+//
+// Bound by instruction issue and, at size, nearly by HBM (8 bytes in, 2 S out an
+// element).  Rows lie at 8-byte alignment: a warp loads 256 contiguous bytes of
+// a row at a time, the next tile while it converts this one, and turns the tile
+// through padded shared memory, so that each thread reads its 64 bytes by
+// conflict-free 16-byte loads.  One FP64 multiply-add scales, rounds and biases
+// an element, and a digit is one mask and one FFMA, where shifts, compares and
+// masks of 64-bit integers took some 50 instructions an element.  The
+// intermediates at D = 2000 (78 M elements, 7 slices): 321 us of 434, 5.3 TB/s
+// or 0.79 of the copy rate; at D = 777 (7.9 M, 6 slices) 41 us of 65; the
+// vector's own pack 43 of 60 and 22 of 30 us.  8-byte asynchronous copies
+// instead of loads took 381 us, converting half the elements with integer
+// instructions the same 321.
+constexpr int kPitch = 34;                             // doubles a staged row takes (16-byte aligned, conflict-free)
+
+// The S digits of eight elements given as mantissas 2^51 + N + bias (the low 52
+// bits of lo, hi): a thread's 16-byte core row of every slice.  Balanced
+// base-128 digits d_q in [-64, 63] (the leading one takes the rest): N + sum_q
+// 64 * 128^q has the plain base-128 digits d_q + 64.  A digit's bits under the
+// exponent of 2^23 are 2^23 + u 2^b for its place b in the word, and one FFMA
+// makes that u - 64, exact, whose BF16 bits are the FP32 value's upper half.
 template <int S>
-__global__ void __launch_bounds__(kPackThreads) pack_digits_kernel(const PackJob* __restrict__ jobs,
+__device__ __forceinline__ void store_digits(const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint8_t* base,
+                                             int64_t slice_bytes) {
+#pragma unroll
+  for (int q = 0; q < S; ++q) {
+    constexpr int kTop = kBits * (S - 1);  // place of the leading digit
+    const int place = kBits * (S - 1 - q);
+    uint32_t fb[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float f;
+      if (q == 0) {  // with the 2^51 above it: 2^(51 - kTop) + (N' >> kTop)
+        const uint32_t u = (hi[i] >> (kTop - 32)) & ((1u << (52 - kTop)) - 1u);
+        f = __uint_as_float(0x4B000000u | u) - (8388608.0f + (float)(1 << (51 - kTop)) + 64.0f);
+      } else {
+        const int word = place / 21;  // words start at bits 0 and 21
+        const int b = place - 21 * word;
+        const uint32_t w = word == 0 ? lo[i] : __funnelshift_r(lo[i], hi[i], 21);
+        f = __fmaf_rn(__uint_as_float((w & (127u << b)) | 0x4B000000u), 1.0f / (float)(1 << b),
+                      -(8388608.0f / (float)(1 << b) + 64.0f));
+      }
+      fb[i] = __float_as_uint(f);
+    }
+    uint4 v;
+    v.x = __byte_perm(fb[0], fb[1], 0x7632);
+    v.y = __byte_perm(fb[2], fb[3], 0x7632);
+    v.z = __byte_perm(fb[4], fb[5], 0x7632);
+    v.w = __byte_perm(fb[6], fb[7], 0x7632);
+    *reinterpret_cast<uint4*>(base + q * slice_bytes) = v;
+  }
+}
+
+template <int S>
+__global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const PackJob* __restrict__ jobs,
                                                                    const int2* __restrict__ units, Bases bases,
                                                                    uint8_t* __restrict__ packed,
-                                                                   int* __restrict__ exps) {
+                                                                   int* __restrict__ exps, int span) {
   __shared__ int rexp[kTM];
   __shared__ int tmax;
+  __shared__ __align__(16) double stage[kPackThreads / 32][8 * kPitch];  // a tile a warp
   const int2 u = units[blockIdx.x];
   const PackJob job = jobs[u.x];
-  const int kt0 = blockIdx.y * kDigitKt;
+  const int kt0 = blockIdx.y * kDigitKt * span;
   if (kt0 >= job.nkt) return;
   const int rt = u.y, RT = job.rt, r0 = rt * RT;
   const double* src = resolve(bases, job.src_buf, job.src);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // a warp's tiles: the 8-row groups warp (and, for 128 rows, warp + 8) of every 32 k
+  const int two = RT == kTM ? 1 : 0;
+  const int ntiles = min(span, (job.nkt - kt0 + kDigitKt - 1) / kDigitKt) << two;
+  double* const mine = stage[warp];
+  const bool rows = job.ld_k == 1;  // contiguous rows: a row of 32 k an instruction; else 8 rows x 4 k
+  const int tr = rows ? 0 : lane & 7, tk = rows ? lane : lane >> 3;  // this lane's element of a tile's first load,
+  const int dr = rows ? 1 : 0, dk = rows ? 0 : 4;                    // and the step to the next
+  const int64_t step = rows ? job.ld_r : 4 * job.ld_k;
+  double next[8];
+  auto group_of = [&](int i) { return warp + ((i & two) << 3); };
+  auto fetch = [&](int i) {
+    const int r = r0 + group_of(i) * 8, k = (kt0 + (i >> two) * kDigitKt) * kKS;
+    const double* p = src + (int64_t)(r + tr) * job.ld_r + (int64_t)(k + tk) * job.ld_k;
+    if (r + 8 <= job.R && k + kDigitKt * kKS <= job.K) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j, p += step) next[j] = __ldg(p);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j, p += step)
+        next[j] = (r + tr + j * dr < job.R && k + tk + j * dk < job.K) ? __ldg(p) : 0.0;
+    }
+  };
+  if (ntiles > 0) fetch(0);
   if (tid == 0) tmax = kExpZero;
   __syncthreads();
   if (tid < RT) {
@@ -137,66 +217,72 @@ __global__ void __launch_bounds__(kPackThreads) pack_digits_kernel(const PackJob
   if (blockIdx.y == 0 && tid == 0) exps[job.texp + rt] = tmax;
 
   const bool unit_alpha = job.alpha == 1.0 || job.alpha == -1.0;
-  const int ncore_k = min(job.nkt - kt0, kDigitKt) * (kKS / 8);
-  const int nkq = (ncore_k + 3) / 4;  // groups of 4 core columns (32 k)
   const int64_t unit_bytes = (int64_t)S * RT * kKS * 2;
   const int64_t slice_bytes = (int64_t)RT * kKS * 2;
   uint8_t* dst = packed + job.dst + ((int64_t)rt * job.nkt + kt0) * unit_bytes;
-  const int r8 = lane & 7, kq = lane >> 3;
-  for (int item = warp; item < (RT / 8) * nkq; item += kPackThreads / 32) {
-    const int rg = item % (RT / 8), kc = (item / (RT / 8)) * 4 + kq;
-    if (kc >= ncore_k) continue;
+  const int r8 = lane & 7, kc = lane >> 3;  // this thread's row of the group and core column
+  const int kin = kc % (kKS / 8);
+  constexpr double kMagic = 6755399441055744.0 + (double)kDigitBias<S>;  // 1.5 2^52 + bias
+  double* const put = mine + tr * kPitch + tk;
+  const int put_step = rows ? kPitch : 4;
+  for (int i = 0; i < ntiles; ++i) {
+    __syncwarp();  // the tile before has been read
+#pragma unroll
+    for (int j = 0; j < 8; ++j) put[j * put_step] = next[j];
+    __syncwarp();
+    if (i + 1 < ntiles) fetch(i + 1);
+    const int rg = group_of(i);
+    const int kt = (i >> two) * kDigitKt + kc / (kKS / 8);
+    if (kt0 + kt >= job.nkt) continue;
     const int r = rg * 8 + r8;
+    uint8_t* const out = dst + (int64_t)kt * unit_bytes + (r / 8) * kSBO + kin * 128 + (r % 8) * 16;
+    if (r0 + rg * 8 >= job.R) {  // rows past the operand: zeros
+#pragma unroll
+      for (int q = 0; q < S; ++q) *reinterpret_cast<uint4*>(out + q * slice_bytes) = make_uint4(0, 0, 0, 0);
+      continue;
+    }
     const int e = rexp[r];
-    const bool live = (r0 + r < job.R) && e != kExpZero;
-    const int s = kBits * S - e;
-    long long N[8];
-    const double* p = src + (int64_t)(r0 + r) * job.ld_r;
-    const int k0 = (kt0 * (kKS / 8) + kc) * 8;
-    double xv[8];
-    if (live && k0 + 8 <= job.K && job.ld_k == 1) {  // whole group along a contiguous row
-      const double* q = p + k0;
+    const int sh = kBits * S - e;
+    const double2* x2 = reinterpret_cast<const double2*>(mine + r8 * kPitch + kc * 8);
+    double x[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) xv[i] = q[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) xv[i] = (live && k0 + i < job.K) ? p[(int64_t)(k0 + i) * job.ld_k] : 0.0;
+    for (int j = 0; j < 4; ++j) {
+      const double2 t = x2[j];
+      x[2 * j] = t.x;
+      x[2 * j + 1] = t.y;
     }
+    if (!unit_alpha) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const double x = xv[i];
-      N[i] = scale_round(unit_alpha ? (job.alpha < 0 ? -x : x) : x * job.alpha, s);
+      for (int j = 0; j < 8; ++j) x[j] *= job.alpha;
     }
-    // Balanced base-128 digits d_q in [-64, 63] (the leading one takes the
-    // rest): N + sum_q 64 * 128^q has the plain base-128 digits d_q + 64, so
-    // each digit is one shift and mask.  A digit's BF16 bits are the upper
-    // half of the exact FP32 value (2^23 + u) - (2^23 + 64).
+    uint32_t lo[8], hi[8];
+    // 2^sh is a normal number, and e <= 1025 for finite rows; a zero row (e =
+    // kExpZero) holds zeros
+    if (e == kExpZero || (e <= 1025 && sh <= 1000)) {
+      const int field = e == kExpZero ? 0 : sh + 1023;
+      const double scale = __hiloint2double((field << 20) | (job.alpha == -1.0 ? (int)0x80000000u : 0), 0);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) N[i] += kDigitBias<S>;
-    const int kt = kc / (kKS / 8), kin = kc % (kKS / 8);
-    uint8_t* base = dst + (int64_t)kt * unit_bytes + (r / 8) * kSBO + kin * 128 + (r % 8) * 16;
-#pragma unroll
-    for (int q = 0; q < S; ++q) {
-      uint32_t fb[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float f;
-        if (q == 0) {  // leading digit: (N' >> 7(S-1)) - 64 in [-65, 65]
-          const int u0 = (int)(N[i] >> (kBits * (S - 1))) + 1;
-          f = __int_as_float(0x4B000000 + u0) - 8388673.0f;
-        } else {
-          const uint32_t uq = (uint32_t)(N[i] >> (kBits * (S - 1 - q))) & 127u;
-          f = __int_as_float(0x4B000000 | uq) - 8388672.0f;
-        }
-        fb[i] = __float_as_uint(f);
+      for (int j = 0; j < 8; ++j) {
+        const double t = __fma_rn(x[j], scale, kMagic);
+        lo[j] = (uint32_t)__double2loint(t);
+        hi[j] = (uint32_t)__double2hiint(t);
       }
-      uint4 v;
-      v.x = __byte_perm(fb[0], fb[1], 0x7632);
-      v.y = __byte_perm(fb[2], fb[3], 0x7632);
-      v.z = __byte_perm(fb[4], fb[5], 0x7632);
-      v.w = __byte_perm(fb[6], fb[7], 0x7632);
-      *reinterpret_cast<uint4*>(base + q * slice_bytes) = v;
+    } else {
+#pragma unroll 1
+      for (int o = 0; o < 8; ++o) {
+        // the loop is not unrolled: this is rare, and its code would be eight times as long
+        double xi = 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) xi = j == o ? x[j] : xi;
+        const long long n = scale_round(job.alpha == -1.0 ? -xi : xi, sh) + kDigitBias<S> + (1ll << 51);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          lo[j] = j == o ? (uint32_t)n : lo[j];
+          hi[j] = j == o ? (uint32_t)((unsigned long long)n >> 32) : hi[j];
+        }
+      }
     }
+    store_digits<S>(lo, hi, out, slice_bytes);
   }
 }
 
@@ -244,11 +330,15 @@ cudaError_t launch_pack(int S, const PackJob* jobs, const int2* units, int nunit
     const int rows_blocks = (int)((warps + kPackThreads / 32 - 1) / (kPackThreads / 32));
     pack_rows_kernel<<<rows_blocks, kPackThreads, 0, stream>>>(jobs, units, nunits, bases, exps);
   }
-  const dim3 grid(nunits, (max_nkt + kDigitKt - 1) / kDigitKt);
+  // CTAs of several chunks (exponents read once, tiles fetched ahead) once
+  // there are enough to fill the SMs' slots twice over: 321 us at D = 2000
+  // where CTAs of one chunk take 432, 41 at D = 777 where longer ones take 49
+  const int chunks = (max_nkt + kDigitKt - 1) / kDigitKt;
+  const int span = (int)std::min<int64_t>(std::max<int64_t>((int64_t)nunits * chunks / (8 * kF64Sms), 1), 8);
+  const dim3 grid(nunits, (chunks + span - 1) / span);
   switch (S) {
-    case 6: pack_digits_kernel<6><<<grid, kPackThreads, 0, stream>>>(jobs, units, bases, packed, exps); break;
-    case 7: pack_digits_kernel<7><<<grid, kPackThreads, 0, stream>>>(jobs, units, bases, packed, exps); break;
-    case 8: pack_digits_kernel<8><<<grid, kPackThreads, 0, stream>>>(jobs, units, bases, packed, exps); break;
+    case 6: pack_digits_kernel<6><<<grid, kPackThreads, 0, stream>>>(jobs, units, bases, packed, exps, span); break;
+    case 7: pack_digits_kernel<7><<<grid, kPackThreads, 0, stream>>>(jobs, units, bases, packed, exps, span); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
