@@ -5,7 +5,9 @@
 //     eigenvalues ascending like dsyev), then the reference's refinement:
 //     while more than one eigenvalue
 //     lies below 0.1 of the largest of the current subspace, re-diagonalise
-//     the original Gram matrix projected on that subspace;
+//     the original Gram matrix projected on that subspace (from the basis at
+//     hand by a few products where that converges, else by another
+//     eigendecomposition);
 //   * the other factor by one more product, singular values = sqrt of the
 //     eigenvalues above 1e-100 of the largest, columns scaled by s^(p1-1) and
 //     s^p2 (or the mirror for wide blocks);
@@ -102,6 +104,77 @@ __global__ void __launch_bounds__(256) canonical_signs_kernel(double* z, int row
   for (int w = 1; w < 8; ++w) first = min(first, sfirst[w]);
   if (first < rows && col[first] < 0)
     for (int i = threadIdx.x; i < rows; i += blockDim.x) col[i] = -col[i];
+}
+
+// ---- refinement levels without an eigendecomposition ----
+// A level's matrix M (n x n, the Gram matrix projected on the level's subspace)
+// is nearly diagonal already: the basis came from an eigendecomposition, whose
+// rounding is all that is left off the diagonal.  What the level must resolve
+// are the eigenvectors of its top decade T (the rest is projected again and
+// resolved on later levels), and those follow from M by the quadratically
+// convergent iteration of Ogita & Aishima ("Iterative refinement for symmetric
+// eigenvalue decomposition", Japan J. Indust. Appl. Math. 35 (2018)): with
+// S = X^T M X and R = I - X^T X,
+//     lambda_i = S_ii / (1 - R_ii),
+//     X <- X + X E,  E_ij = (S_ij + lambda_j R_ij) / (lambda_j - lambda_i),
+//     E_ii = R_ii / 2,
+// here with E_ij = R_ij / 2 (orthonormality only) where neither i nor j lies in
+// T, or where the coupling is rounding noise of the level and as large as the
+// gap (a degenerate pair: any basis of it is as good).  Mostly one step from X =
+// I does, which is one launch and no product.  A level of 101 rows takes 0.3 ms
+// where cuSOLVER's eigendecomposition takes 4.6 (it is a chain of some hundred
+// dependent launches); a truncation at D = 400 (14 sectors of up to 108 rows, 10
+// levels) 48.3 -> 13.7 ms, those of a sweep of the 8x4 cylinder at D = 400 2.49
+// -> 0.52 s, with the same or smaller residuals and orthonormality errors.
+constexpr double kDecade = 0.1;         // T: diagonal entries from a tenth of the largest on
+constexpr double kStepDone = 1e-8;      // steps up to this leave an error below rounding
+constexpr double kStepMax = 1e-3;       // larger ones: an eigendecomposition
+constexpr int kRefineMax = 6000;        // the kernel's shared memory (48 KB of eigenvalues)
+constexpr double kLevelNoise = 8 * 2.220446049250313e-16;  // of the level's largest entry
+
+// x = I + E from S (the upper triangle counts; ld n) and P = X^T X (null: X =
+// I).  info[0]: the largest |E_ij| (as bits), lam[i] the eigenvalue estimates.
+// One CTA per column; every CTA finds the decade's first index itself.
+__global__ void __launch_bounds__(256) refine_step_kernel(const double* __restrict__ S, const double* __restrict__ P,
+                                                          int n, double* __restrict__ x, double* __restrict__ lam,
+                                                          unsigned long long* info) {
+  extern __shared__ double d[];  // n eigenvalue estimates
+  __shared__ double red[8];
+  __shared__ int redi[8];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, j = blockIdx.x;
+  double top = 0;
+  for (int i = tid; i < n; i += 256) {
+    const double v = S[(int64_t)i * n + i] / (P ? P[(int64_t)i * n + i] : 1.0);  // 1 - R_ii = P_ii
+    d[i] = v;
+    if (j == 0) lam[i] = v;
+    top = fmax(top, v);
+  }
+  for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if (lane == 0) red[wid] = top;
+  __syncthreads();
+  for (int w = 0; w < 8; ++w) top = fmax(top, red[w]);
+  int t0 = 0;  // T = [t0, n): after the last entry below a tenth of the largest
+  for (int i = tid; i < n; i += 256)
+    if (!(d[i] >= kDecade * top)) t0 = i + 1;
+  for (int o = 16; o > 0; o >>= 1) t0 = max(t0, __shfl_xor_sync(0xffffffffu, t0, o));
+  if (lane == 0) redi[wid] = t0;
+  __syncthreads();
+  for (int w = 0; w < 8; ++w) t0 = max(t0, redi[w]);
+  const double noise = kLevelNoise * top;
+  double big = 0;
+  for (int i = tid; i < n; i += 256) {
+    const int64_t at = i < j ? (int64_t)j * n + i : (int64_t)i * n + j;  // the upper triangle's copy
+    const double r = P ? (i == j ? 1.0 : 0.0) - P[at] : 0.0;
+    double e = 0.5 * r;
+    if (i != j && (i >= t0 || j >= t0)) {
+      const double m = S[at] + d[j] * r, gap = d[j] - d[i];
+      if (!(fabs(m) <= noise && fabs(m) > kStepMax * fabs(gap))) e = m / gap;
+    }
+    x[(int64_t)j * n + i] = (i == j ? 1.0 : 0.0) + e;
+    big = fmax(big, isfinite(e) ? fabs(e) : 1e300);
+  }
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0 && big > 0) atomicMax(info, (unsigned long long)__double_as_longlong(big));
 }
 
 // Per-device resources kept across calls: lanes (one stream and one cuSOLVER
@@ -237,6 +310,13 @@ class SectorThreads {
   size_t idle_ = 0;
 };
 
+// index after the last eigenvalue below tol1 of the largest (tensor.cpp:1492-1497)
+int small_count(const std::vector<double>& w, int n) {
+  for (int i = n - 1; i >= 0; --i)
+    if (w[i] / w[n - 1] < 1.e-1) return i + 1;
+  return 0;
+}
+
 // The work of one sector: its lane, its allocations (from the pool, on the
 // lane's stream; released on `free_st` once the caller's stream has used
 // them) and its error state.
@@ -296,6 +376,65 @@ struct Ctx {
     cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
   }
+  // The eigenvectors of a level's top decade from its nearly diagonal matrix m
+  // (n x n), the rest of the basis orthonormal beside them: x (n x n), lam the
+  // eigenvalues (top decade) and diagonal entries (rest).  False, x undefined,
+  // where the level needs an eigendecomposition: the couplings are too large
+  // for the gaps, the order of the values is not settled, or the subspace left
+  // is the last to be looked at (its values are reported as they are).
+  // y, p, q: n x n scratch.
+  bool refine(const double* m, int n, double lam_cut, double* x, double* y, double* p, double* q,
+              std::vector<double>* lam) {
+    if (n > kRefineMax) return false;
+    double* dlam = dalloc(n + 1);
+    if (!ok()) return false;
+    unsigned long long* info = (unsigned long long*)(dlam + n);
+    std::vector<double> h(n + 1);
+    for (int it = 0; it < 4 && ok(); ++it) {
+      if (it > 0) {
+        gemm(false, n, n, n, m, n, x, n, y, n);
+        gemm(true, n, n, n, x, n, y, n, q, n);  // S
+        gemm(true, n, n, n, x, n, x, n, p, n);  // P
+      }
+      double* step = it > 0 ? y : x;
+      cudaError_t e = cudaMemsetAsync(info, 0, sizeof(*info), st);
+      if (e == cudaSuccess) {
+        refine_step_kernel<<<n, 256, n * sizeof(double), st>>>(it > 0 ? q : m, it > 0 ? p : nullptr, n, step, dlam, info);
+        e = cudaGetLastError();
+      }
+      if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), dlam, (n + 1) * sizeof(double), cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      if (e != cudaSuccess) {
+        set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
+        return false;
+      }
+      const double big = h[n];
+      const int t0 = small_count(h, n);
+      // the kernel's T: from t0 on, in ascending order, everything below it
+      // smaller than a tenth of the last entry
+      bool good = big <= (it > 0 ? 10 * kStepMax : kStepMax) && h[n - 1] > 0;
+      for (int i = 0; i < n && good; ++i) {
+        const bool in_top = h[i] >= kDecade * h[n - 1];
+        good = in_top == (i >= t0) && (i <= t0 || h[i] >= h[i - 1]);
+      }
+      if (good && it == 0 && t0 > 1) good = !(lam_cut > 0 && h[t0 - 1] < kDecade * lam_cut);
+      if (!good) return false;
+      if (it > 0) {
+        gemm(false, n, n, n, x, n, y, n, q, n);
+        copy(x, q, (int64_t)n * n);
+      }
+      if (big <= kStepDone) {
+        if (!ok()) return false;
+        canonical_signs_kernel<<<n, 256, 0, st>>>(x, n);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
+        h.resize(n);
+        lam->swap(h);
+        return ok();
+      }
+    }
+    return false;
+  }
   // symmetric eigendecomposition in place (a: n x n, ld n), eigenvector signs
   // by the canonical rule; w: host eigenvalues
   void eigh(double* a, int n, std::vector<double>* w) {
@@ -329,13 +468,6 @@ struct Ctx {
     else if (info != 0) set(SU2G_ECUDA, "svd: syevd did not converge (info " + std::to_string(info) + ")");
   }
 };
-
-// index after the last eigenvalue below tol1 of the largest (tensor.cpp:1492-1497)
-int small_count(const std::vector<double>& w, int n) {
-  for (int i = n - 1; i >= 0; --i)
-    if (w[i] / w[n - 1] < 1.e-1) return i + 1;
-  return 0;
-}
 
 struct Sector {
   int i = -1;      // leg-0 sector index
@@ -399,6 +531,7 @@ void sector_finish(Ctx& c, const double* blk, int m, int n, double p1, double p2
     double* app = c.dalloc((int64_t)k * k);
     double* vpp = c.dalloc((int64_t)k * k);
     double* tmp = c.dalloc((int64_t)k * k);
+    double* scr = c.dalloc((int64_t)k * k);
     c.copy(ap, e.A0, (int64_t)k * k);
     c.copy(vp, G, (int64_t)k * k);
     int npp = np;
@@ -409,7 +542,12 @@ void sector_finish(Ctx& c, const double* blk, int m, int n, double p1, double p2
       c.gemm(true, npp, np, np, vp, np, ap, np, app, npp);
       c.gemm(false, npp, npp, np, app, npp, vp, np, vpp, npp);
       c.copy(ap, vpp, (int64_t)npp * npp);
-      c.eigh(vpp, npp, &ws);
+      // the level's eigenvectors: by refinement of the basis at hand, else (ap
+      // still holds the matrix) by an eigendecomposition
+      if (!c.refine(ap, npp, lam_cut, vpp, app, tmp, scr, &ws)) {
+        c.copy(vpp, ap, (int64_t)npp * npp);
+        c.eigh(vpp, npp, &ws);
+      }
       if (!c.ok()) return;
       for (int q = 0; q < npp; ++q) w[q] = ws[q];
       c.gemm(false, k, npp, npp, G, k, vpp, npp, tmp, k);
