@@ -299,6 +299,10 @@ typedef struct {
 } su2g_env_job;
 int su2g_env_layout(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2g_env_job* jobs, int slot,
                     int* out_desc, int out_desc_cap, int* out_flag, int out_flag_cap, int64_t* out_len);
+/* The layouts of all slots in one call: the desc of slot s at out_desc + s *
+ * desc_stride, the flags of the slots one after another, out_len[s]. */
+int su2g_env_layouts(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2g_env_job* jobs, int nslots,
+                     int* out_desc, int desc_stride, int* out_flag, int out_flag_cap, int64_t* out_len);
 int su2g_env_run(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2g_env_job* jobs, int nslots,
                  double* const* outs, int mode, void* stream);
 /* Host-only dry run of su2g_env_run: builds and bounds-checks the work list

@@ -99,6 +99,7 @@ _PROTOS = {
     "su2g_overlap_transformation_layout": (_i, [Tensor, Tensor, _i, Tensor, _vp, _i, _vp, _i, _vp]),
     "su2g_overlap_transformation": (_i, [Tensor, Tensor, _i, _i, _vp, _vp, _i, _vp]),
     "su2g_env_layout": (_i, [Tensor, Tensor, _i, _i, _vp, _i, _vp, _i, _vp, _i, _vp]),
+    "su2g_env_layouts": (_i, [Tensor, Tensor, _i, _i, _vp, _i, _vp, _i, _vp, _i, _vp]),
     "su2g_env_run": (_i, [Tensor, Tensor, _i, _i, _vp, _i, _vp, _i, _vp]),
     "su2g_env_validate": (_i, [Tensor, Tensor, _i, _i, _vp, _i, _i, _vp, _vp]),
     "su2g_env_digest": (_i, [Tensor, Tensor, _i, _i, _vp, _i, _vp, _i, _vp]),

@@ -304,6 +304,23 @@ int env_batch_run(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2
   return su2g::run_work_once(std::move(w), mode, stream);
 }
 
+int write_struct(const su2g::Struct& y, int* out_desc, int out_desc_cap, int* out_flag, int out_flag_cap,
+                 int64_t* out_len) {
+  std::vector<int> d = {y.nbond, y.locspin};
+  for (int l = 0; l < y.nbond; ++l) {
+    d.push_back(y.legs[l].dir);
+    d.push_back(y.legs[l].n());
+    for (int a : y.legs[l].angm) d.push_back(a);
+    for (int x : y.legs[l].dim) d.push_back(x);
+  }
+  if (!out_desc || !out_flag || (int)d.size() > out_desc_cap || y.nten > out_flag_cap)
+    return fail(SU2G_EINVAL, "env layout: output arrays too small");
+  std::copy(d.begin(), d.end(), out_desc);
+  std::copy(y.flag.begin(), y.flag.end(), out_flag);
+  if (out_len) *out_len = y.total;
+  return SU2G_OK;
+}
+
 int env_batch_layout(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2g_env_job* jobs, int slot,
                      int* out_desc, int out_desc_cap, int* out_flag, int out_flag_cap, int64_t* out_len) {
   su2g::HeffWork w;
@@ -319,20 +336,7 @@ int env_batch_layout(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const 
   if (mine.empty()) return fail(SU2G_EINVAL, "env layout: no job writes slot " + std::to_string(slot));
   int rc = su2g::build_env_batch(uu, vv, flag, (int)mine.size(), mine.data(), 1, nullptr, &w, &ys, &err);
   if (rc) return fail(rc, err);
-  const su2g::Struct& y = ys[0];
-  std::vector<int> d = {y.nbond, y.locspin};
-  for (int l = 0; l < y.nbond; ++l) {
-    d.push_back(y.legs[l].dir);
-    d.push_back(y.legs[l].n());
-    for (int a : y.legs[l].angm) d.push_back(a);
-    for (int x : y.legs[l].dim) d.push_back(x);
-  }
-  if (!out_desc || !out_flag || (int)d.size() > out_desc_cap || y.nten > out_flag_cap)
-    return fail(SU2G_EINVAL, "env layout: output arrays too small");
-  std::copy(d.begin(), d.end(), out_desc);
-  std::copy(y.flag.begin(), y.flag.end(), out_flag);
-  if (out_len) *out_len = y.total;
-  return SU2G_OK;
+  return write_struct(ys[0], out_desc, out_desc_cap, out_flag, out_flag_cap, out_len);
 }
 
 // overlap_transformation / operator_transformation batches: one job per operator
@@ -401,6 +405,23 @@ int su2g_overlap_transformation(su2g_tensor uu, su2g_tensor vv, int flag, int no
 int su2g_env_layout(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2g_env_job* jobs, int slot,
                     int* out_desc, int out_desc_cap, int* out_flag, int out_flag_cap, int64_t* out_len) {
   return env_batch_layout(uu, vv, flag, njobs, jobs, slot, out_desc, out_desc_cap, out_flag, out_flag_cap, out_len);
+}
+
+int su2g_env_layouts(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2g_env_job* jobs, int nslots,
+                     int* out_desc, int desc_stride, int* out_flag, int out_flag_cap, int64_t* out_len) {
+  su2g::HeffWork w;
+  std::vector<su2g::Struct> ys;
+  std::string err;
+  const int rc = su2g::build_env_batch(uu, vv, flag, njobs, jobs, nslots, nullptr, &w, &ys, &err);
+  if (rc) return fail(rc, err);
+  int at = 0;
+  for (int s = 0; s < nslots; ++s) {
+    const int r = write_struct(ys[s], out_desc ? out_desc + (int64_t)s * desc_stride : nullptr, desc_stride,
+                               out_flag ? out_flag + at : nullptr, out_flag_cap - at, out_len ? out_len + s : nullptr);
+    if (r) return r;
+    at += ys[s].nten;
+  }
+  return SU2G_OK;
 }
 
 int su2g_env_run(su2g_tensor uu, su2g_tensor vv, int flag, int njobs, const su2g_env_job* jobs, int nslots,

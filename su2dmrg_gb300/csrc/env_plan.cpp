@@ -21,8 +21,8 @@
 
 #include <algorithm>
 #include <cmath>
-#include <tuple>
-#include <unordered_map>
+#include <map>
+#include <utility>
 
 namespace su2g {
 namespace {
@@ -71,8 +71,9 @@ struct Contrib {
   int xj;  // X block, -1: none (U^T V)
   int xs;  // X slice
   int k, l;
-  int m, os;  // output block and slice
-  double w;
+  int m, os;   // output block and slice
+  double w;    // recoupling factor and site elements (the job's coefficient comes last)
+  int64_t t0;  // the slice-0 offset of T in the scratch
 };
 
 // one parsed job
@@ -85,44 +86,22 @@ struct Job {
   const double* s1 = nullptr;
   const double* s2 = nullptr;
   Struct Y;  // output structure (flags filled later)
+  size_t c0 = 0, c1 = 0;  // its contributions
 };
+
+// Two overlap or transformation jobs whose operators have one structure visit
+// the same blocks with the same factors: a batch computes them once.
+bool same_walk(const Job& a, const Job& b) {
+  if (a.kind != b.kind || (a.kind != SU2G_ENV_OVERLAP && a.kind != SU2G_ENV_TRANSFORM)) return false;
+  for (int l = 0; l < a.X.nbond; ++l)
+    if (!same_sectors(a.X.legs[l], b.X.legs[l])) return false;
+  return a.X.flag == b.X.flag;
+}
 
 int64_t block_size(const Struct& s, int b) {
   int64_t n = 1;
   for (int l = 0; l < s.nbond; ++l) n *= s.block_dim(b, l);
   return n;
-}
-
-// The stored blocks of a tensor grouped by the 2j of one leg (or of two legs),
-// each group in ascending block order: the contribution loops visit exactly
-// the blocks a full scan with the same tests would, in the same order,
-// without scanning every block of uu and vv for every operator block.
-struct Buckets {
-  int w2 = 1;
-  std::vector<std::vector<int>> b;
-  const std::vector<int>& at(int a1, int a2 = 0) const {
-    static const std::vector<int> none;
-    if (a1 < 0 || a2 < 0 || a2 >= w2) return none;
-    const size_t key = (size_t)a1 * w2 + a2;
-    return key < b.size() ? b[key] : none;
-  }
-};
-
-Buckets bucket(const Struct& s, int l1, int l2 = -1) {
-  auto width = [&](int l) {
-    int m = 0;
-    for (int a : s.legs[l].angm) m = std::max(m, a);
-    return m + 1;
-  };
-  Buckets r;
-  r.w2 = l2 >= 0 ? width(l2) : 1;
-  r.b.resize((size_t)width(l1) * r.w2);
-  for (int k = 0; k < s.nten; ++k) {
-    if (!s.flag[k]) continue;
-    const int a1 = s.block_angm(k, l1), a2 = l2 >= 0 ? s.block_angm(k, l2) : 0;
-    if (a1 >= 0 && a2 >= 0) r.b[(size_t)a1 * r.w2 + a2].push_back(k);
-  }
-  return r;
 }
 
 }  // namespace
@@ -167,6 +146,7 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
   std::vector<Contrib> cs;
   std::vector<std::vector<int>> present(nslots);
   std::vector<int> slot_owner(nslots, -1);
+  std::vector<int> walks;  // jobs whose contributions were computed, not copied
   for (int t = 0; t < njobs; ++t) {
     const su2g_env_job& in = jobs[t];
     Job& jb = J[t];
@@ -248,9 +228,20 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
       return true;
     };
     auto angm_ok = [&](int a) { return a >= 0 && a < kMaxAngm; };
-    const size_t c0 = cs.size();
+    jb.c0 = cs.size();
+    const Job* like = nullptr;
+    for (int o : walks)
+      if (same_walk(J[o], jb)) like = &J[o];
 
-    if (kind == SU2G_ENV_OVERLAP || kind == SU2G_ENV_TRANSFORM) {
+    if (like) {
+      cs.reserve(cs.size() + (like->c1 - like->c0));
+      for (size_t q = like->c0; q < like->c1; ++q) {
+        cs.push_back(cs[q]);
+        cs.back().job = t;
+        pres[cs[q].m] = 1;
+      }
+    } else if (kind == SU2G_ENV_OVERLAP || kind == SU2G_ENV_TRANSFORM) {
+      walks.push_back(t);
       // reference loop order: X block, U block, V block
       const int xr = xlegs - 1;
       for (int j = 0; j < jb.X.nten; ++j) {
@@ -272,7 +263,7 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
               if (std::fabs(fac) < 1.e-8) continue;
             }
             pres[m] = 1;
-            for (int sg = 0; sg < ms; ++sg) cs.push_back(Contrib{t, j, sg, k, l, m, sg, fac});
+            for (int sg = 0; sg < ms; ++sg) cs.push_back(Contrib{t, j, sg, k, l, m, sg, fac, 0});
           }
         }
       }
@@ -305,7 +296,7 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
               const double fac = fac_operator_onsite(flag, c, s, cp, ap, sig + sigp * 3);
               if (std::fabs(fac) < 1.e-8) continue;
               pres[m] = 1;
-              cs.push_back(Contrib{t, jb.has_x ? e : -1, 0, k, l, m, 0, fac * op});
+              cs.push_back(Contrib{t, jb.has_x ? e : -1, 0, k, l, m, 0, fac * op, 0});
             }
           }
         }
@@ -335,7 +326,7 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
               if (block_size(S, n) != ms)
                 return fail(SU2G_EINVAL, t, "site operator block does not match the operator spin multiplicity");
               pres[m] = 1;
-              for (int sg = 0; sg < ms; ++sg) cs.push_back(Contrib{t, j, sg, k, l, m, 0, fac * jb.s1[S.offset[n] + sg]});
+              for (int sg = 0; sg < ms; ++sg) cs.push_back(Contrib{t, j, sg, k, l, m, 0, fac * jb.s1[S.offset[n] + sg], 0});
             }
           }
         }
@@ -385,15 +376,16 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
                 double fac1 = 0;
                 for (int64_t e = 0; e < n1; ++e) fac1 += jb.s1[O1.offset[mm] + e] * jb.s2[O2.offset[nn] + e];
                 pres[m] = 1;
-                cs.push_back(Contrib{t, k, 0, j, l, m, 0, fac * fac1});
+                cs.push_back(Contrib{t, k, 0, j, l, m, 0, fac * fac1, 0});
               }
             }
           }
         }
       }
     }
-    for (size_t q = c0; q < cs.size(); ++q) cs[q].w *= jb.coef;
+    jb.c1 = cs.size();
   }
+  for (Contrib& c : cs) c.w *= J[c.job].coef;
   // slot structures
   for (int sl = 0; sl < nslots; ++sl) {
     if (slot_owner[sl] < 0) {
@@ -418,22 +410,36 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
     }
   }
   // ---- phase 1: T = X_s^T U per (job, X block, U block, slice) ----
-  struct TKeyHash {
-    size_t operator()(const std::tuple<int, int, int>& k) const {
-      const uint64_t a = (uint32_t)std::get<0>(k), b = (uint32_t)std::get<1>(k), c = (uint32_t)std::get<2>(k);
-      return (size_t)((a * 0x9e3779b97f4a7c15ull) ^ (b * 0xc2b2ae3d27d4eb4full) ^ (c * 0x165667b19e3779f9ull));
-    }
-  };
-  // (job, X block, U block) -> slice-0 T offset; lookups only (offsets follow contribution order)
-  std::unordered_map<std::tuple<int, int, int>, int64_t, TKeyHash> tpos;
-  for (const Contrib& c : cs) {
-    if (c.xj < 0 || tpos.count({c.job, c.xj, c.k})) continue;
+  // Contributions of one job and one (X block, U block) follow one another,
+  // except where an endt meets several site blocks: those look theirs up
+  // (slice-0 T offset of the job at hand).
+  const Contrib* last = nullptr;
+  std::map<std::pair<int, int>, int64_t> endt_pos;
+  w.seg1.reserve(cs.size());
+  w.blk1.reserve(cs.size());
+  for (Contrib& c : cs) {
+    if (c.xj < 0) continue;
     const Job& jb = J[c.job];
+    const bool same_job = last && last->job == c.job;
+    if (same_job && last->xj == c.xj && last->k == c.k) {
+      c.t0 = last->t0;
+      continue;
+    }
+    if (!same_job) endt_pos.clear();
+    last = &c;
+    if (jb.kind == SU2G_ENV_INITIAL) {
+      const auto known = endt_pos.find({c.xj, c.k});
+      if (known != endt_pos.end()) {
+        c.t0 = known->second;
+        continue;
+      }
+      endt_pos[{c.xj, c.k}] = w.scratch_len;
+    }
     const int xr = jb.X.nbond - 1;
     const int A = jb.X.block_dim(c.xj, 0), Ap = jb.X.block_dim(c.xj, xr);
     const int ms = jb.X.nbond == 3 ? jb.X.block_dim(c.xj, 1) : 1;
     const int C = U.block_dim(c.k, 2);
-    tpos[{c.job, c.xj, c.k}] = w.scratch_len;
+    c.t0 = w.scratch_len;
     for (int sg = 0; sg < ms; ++sg) {
       GemmSeg g;
       g.a = abs_off(jb.xb, jb.X.offset[c.xj] + (int64_t)A * sg);
@@ -459,28 +465,32 @@ int build_env_batch(const su2g_tensor& uu, const su2g_tensor& vv, int flag, int 
   // ---- phase 2: out(c, s, c') = sum w T_s^T V (or w U^T V), per block and slice ----
   // contributions grouped by (slot, block, slice) in ascending order, each
   // group in contribution order
-  using OutKey = std::tuple<int, int, int>;
-  std::vector<std::pair<OutKey, int>> by_out(cs.size());
-  for (int q = 0; q < (int)cs.size(); ++q) by_out[q] = {OutKey{J[cs[q].job].slot, cs[q].m, cs[q].os}, q};
-  std::stable_sort(by_out.begin(), by_out.end(),
-                   [](const std::pair<OutKey, int>& x, const std::pair<OutKey, int>& y) { return x.first < y.first; });
+  struct ByOut {
+    uint64_t blk;  // slot, block
+    uint64_t seq;  // slice, contribution
+    bool operator<(const ByOut& o) const { return blk != o.blk ? blk < o.blk : seq < o.seq; }
+  };
+  std::vector<ByOut> by_out(cs.size());
+  for (size_t q = 0; q < cs.size(); ++q)
+    by_out[q] = {(uint64_t)J[cs[q].job].slot << 32 | (uint32_t)cs[q].m, (uint64_t)cs[q].os << 32 | (uint32_t)q};
+  std::sort(by_out.begin(), by_out.end());
+  w.seg2.reserve(cs.size());
   for (size_t g0 = 0; g0 < by_out.size();) {
     size_t g1 = g0;
-    while (g1 < by_out.size() && by_out[g1].first == by_out[g0].first) ++g1;
-    const int sl = std::get<0>(by_out[g0].first), m = std::get<1>(by_out[g0].first), os = std::get<2>(by_out[g0].first);
+    while (g1 < by_out.size() && by_out[g1].blk == by_out[g0].blk && by_out[g1].seq >> 32 == by_out[g0].seq >> 32) ++g1;
+    const int sl = (int)(by_out[g0].blk >> 32), m = (int)(uint32_t)by_out[g0].blk, os = (int)(by_out[g0].seq >> 32);
     const Struct& Y = (*slot_structs)[sl];
     const int C = Y.block_dim(m, 0), Cp = Y.block_dim(m, Y.nbond - 1), ms = Y.nbond == 3 ? Y.block_dim(m, 1) : 1;
     const int seg0 = (int)w.seg2.size();
     int64_t kwork = 0;
     for (size_t gi = g0; gi < g1; ++gi) {
-      const int q = by_out[gi].second;
-      const Contrib& c = cs[q];
+      const Contrib& c = cs[(uint32_t)by_out[gi].seq];
       const Job& jb = J[c.job];
       GemmSeg g;
       int K;
       if (c.xj >= 0) {
         K = jb.X.block_dim(c.xj, jb.X.nbond - 1);
-        g.a = tpos[{c.job, c.xj, c.k}] + (int64_t)c.xs * K * C;
+        g.a = c.t0 + (int64_t)c.xs * K * C;
         g.a_buf = kBufScratch;
         g.a_len = (int64_t)K * C;
       } else {

@@ -251,20 +251,22 @@ int build_heff_work(const int* psi_desc, const int* psi_flag, int nterms, const 
     double fac;
   };
   std::vector<TBlock> tb;
+  const Buckets p_left = bucket(P, 0);
+  std::vector<Buckets> right(nterms);  // op2's blocks by the legs T meets
   for (int t = 0; t < nterms; ++t) {
     const Struct &s1 = op1[t].s, &s2 = op2[t].s;
+    right[t] = bucket(s2, 0, 1);
     for (int j = 0; j < s1.nten; ++j) {
       if (!s1.flag[j]) continue;
       const int ja = s1.block_angm(j, 0), s = s1.block_angm(j, 1), jc = s1.block_angm(j, 2);
       const int a = s1.block_dim(j, 0), ms = s1.block_dim(j, 1), c = s1.block_dim(j, 2);
-      for (int k = 0; k < P.nten; ++k) {
-        if (!P.flag[k] || P.block_angm(k, 0) != ja) continue;
+      for (int k : p_left.at(ja)) {
         const int jb = P.block_angm(k, 1), b = P.block_dim(k, 1);
         // does this step1 block reach a stored output block through op2?
         bool used = false;
         double f = 0;
-        for (int l = 0; l < s2.nten && !used; ++l) {
-          if (!s2.flag[l] || s2.block_angm(l, 0) != jb || s2.block_angm(l, 1) != s) continue;
+        for (int l : right[t].at(jb, s)) {
+          if (used) break;
           const int jd = s2.block_angm(l, 2);
           const int oa[2] = {jc, jd};
           if (!legal_angm(oa, 2, 0)) continue;
@@ -371,9 +373,8 @@ int build_heff_work(const int* psi_desc, const int* psi_flag, int nterms, const 
     for (const TBlock& T : tb) {
       if (T.jc != jc) continue;
       const Struct& s2 = op2[T.t].s;
-      for (int l = 0; l < s2.nten; ++l) {
-        if (!s2.flag[l] || s2.block_angm(l, 0) != T.jb || s2.block_angm(l, 1) != T.s || s2.block_angm(l, 2) != jd)
-          continue;
+      for (int l : right[T.t].at(T.jb, T.s)) {
+        if (s2.block_angm(l, 2) != jd) continue;
         GemmSeg g;
         g.a = T.off;
         g.a_buf = kBufScratch;

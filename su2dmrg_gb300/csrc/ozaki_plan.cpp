@@ -7,46 +7,62 @@
 
 #include <algorithm>
 #include <cstring>
-#include <tuple>
-#include <unordered_map>
+#include <utility>
 
 namespace su2g {
 namespace oz {
 namespace {
 
-using Key = std::tuple<int, int64_t, int64_t, int64_t, int, int, int, uint64_t>;
-
-struct KeyHash {
-  size_t operator()(const Key& k) const {
-    uint64_t h = 0x9e3779b97f4a7c15ull;
-    auto mix = [&](uint64_t x) { h ^= x + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2); };
-    mix((uint64_t)std::get<0>(k));
-    mix((uint64_t)std::get<1>(k));
-    mix((uint64_t)std::get<2>(k));
-    mix((uint64_t)std::get<3>(k));
-    mix((uint64_t)std::get<4>(k));
-    mix((uint64_t)std::get<5>(k));
-    mix((uint64_t)std::get<6>(k));
-    mix(std::get<7>(k));
-    return (size_t)h;
+// Open-addressed table of indices into lists that hold their own keys; sized
+// for the most entries up front, so it is one allocation.
+struct IndexTable {
+  std::vector<int> slot;  // -1: empty
+  size_t mask = 0;
+  explicit IndexTable(size_t most) {
+    size_t n = 16;
+    while (n < 2 * most) n *= 2;
+    slot.assign(n, -1);
+    mask = n - 1;
+  }
+  // the entry for which `is` holds, or the empty place for it
+  template <class Is>
+  int& find(uint64_t hash, Is is) {
+    size_t i = (hash ^ hash >> 29) & mask;
+    while (slot[i] >= 0 && !is(slot[i])) i = (i + 1) & mask;
+    return slot[i];
   }
 };
+inline uint64_t mixed(uint64_t h, uint64_t x) { return (h ^ x) * 0x9e3779b97f4a7c15ull; }
 
 struct Builder {
   int S;
   OzWork* w;
-  // key -> (class, job index); lookups only: jobs are numbered in order of first use
-  std::unordered_map<Key, std::pair<int, int>, KeyHash> index;
+  IndexTable index;  // jobs by operand view, 3 * index + class; jobs are numbered in order of first use
   std::vector<PackJob>* lists[3];
+
+  Builder(int s, OzWork* work, size_t products) : S(s), w(work), index(2 * products) {
+    for (int c = 0; c < 3; ++c) lists[c] = &w->jobs[c];
+  }
+  static int class_of(int src_buf) { return src_buf == kBufAbs ? 0 : (src_buf == kBufPsi ? 1 : 2); }
 
   // class 0 = operator (packed once), 1 = from psi, 2 = from the phase-1 intermediates
   int job(int src_buf, int64_t src, int64_t ld_r, int64_t ld_k, int R, int K, int rt, double alpha) {
     uint64_t abits;
     std::memcpy(&abits, &alpha, 8);
-    const Key key{src_buf, src, ld_r, ld_k, R, K, rt, abits};
-    auto it = index.find(key);
-    const int cls = src_buf == kBufAbs ? 0 : (src_buf == kBufPsi ? 1 : 2);
-    if (it != index.end()) return it->second.second;
+    const int cls = class_of(src_buf);
+    std::vector<PackJob>& list = *lists[cls];
+    uint64_t h = mixed(mixed(mixed((uint64_t)src, (uint64_t)ld_r << 32 ^ (uint64_t)ld_k), (uint64_t)R << 32 ^ (uint64_t)K),
+                       (uint64_t)src_buf << 32 ^ (uint64_t)rt);
+    h = mixed(h ^ h >> 31, abits);
+    int& at = index.find(h ^ h >> 31, [&](int e) {
+      if (e % 3 != cls) return false;
+      const PackJob& j = list[e / 3];
+      uint64_t jbits;
+      std::memcpy(&jbits, &j.alpha, 8);
+      return j.src_buf == src_buf && j.src == src && j.ld_r == ld_r && j.ld_k == ld_k && j.R == R && j.K == K &&
+             j.rt == rt && jbits == abits;
+    });
+    if (at >= 0) return at / 3;
     PackJob j;
     j.src = src;
     j.src_buf = src_buf;
@@ -64,15 +80,12 @@ struct Builder {
     j.rowmax = -1;
     w->packed_bytes += (int64_t)j.nrt * j.nkt * S * rt * kKS * 2;
     w->exp_len += (int64_t)j.nrt * rt + j.nrt;
-    lists[cls]->push_back(j);
-    const int id = (int)lists[cls]->size() - 1;
-    index[key] = {cls, id};
+    list.push_back(j);
+    const int id = (int)list.size() - 1;
+    at = 3 * id + cls;
     return id;
   }
-  const PackJob& get(int src_buf, int id) {
-    const int cls = src_buf == kBufAbs ? 0 : (src_buf == kBufPsi ? 1 : 2);
-    return (*lists[cls])[id];
-  }
+  const PackJob& get(int src_buf, int id) { return (*lists[class_of(src_buf)])[id]; }
 };
 
 // The exact combination of a tile's group sums holds at most 2^17 contracted
@@ -85,10 +98,29 @@ constexpr int64_t kMaxKPerTile = (int64_t)1 << 17;
 int build_phase(Builder& B, const std::vector<GemmSeg>& segs, const std::vector<OutBlock>& blks,
                 std::vector<OzSeg>* oseg, std::vector<OzTile>* otile, std::string* err, bool may_split) {
   const int S = B.S;
+  {  // the lists' lengths (phase 2: but for blocks in several runs)
+    size_t nt = 0, ns = 0;
+    for (const OutBlock& ob : blks) {
+      const size_t t = (size_t)((std::max(ob.M, 0) + kTM - 1) / kTM) * ((std::max(ob.N, 0) + kTN - 1) / kTN);
+      nt += t;
+      ns += t * ob.nseg;
+    }
+    otile->reserve(nt);
+    oseg->reserve(ns);
+  }
+  // what the tiles of one block take from each of its products
+  struct Prod {
+    int64_t a_dst, a_row, b_dst, b_row, a_exp, a_texp, b_exp;
+    int nks;
+  };
+  std::vector<std::pair<int, int>> ids;  // (A job, B job) indices
+  std::vector<Prod> prods;
+  std::vector<std::pair<int, int>> runs;  // (first product, count) relative to ob.seg0
   for (const OutBlock& ob : blks) {
     // pack jobs of every product of this block
-    std::vector<std::pair<int, int>> ids;  // (A job, B job) indices
-    std::vector<std::pair<int, int>> bufs;
+    ids.clear();
+    prods.clear();
+    runs.clear();
     for (int s = ob.seg0; s < ob.seg0 + ob.nseg; ++s) {
       const GemmSeg& g = segs[s];
       double aa = 1.0, ab = 1.0;
@@ -104,11 +136,16 @@ int build_phase(Builder& B, const std::vector<GemmSeg>& segs, const std::vector<
       const int ja = B.job(g.a_buf, g.a, a_ldr, a_ldk, ob.M, g.K, kTM, aa);
       const int jb = B.job(g.b_buf, g.b, g.ldb, 1, ob.N, g.K, kTN, ab);
       ids.push_back({ja, jb});
-      bufs.push_back({g.a_buf, g.b_buf});
+    }
+    for (int s = 0; s < ob.nseg; ++s) {
+      const GemmSeg& g = segs[ob.seg0 + s];
+      const PackJob& a = B.get(g.a_buf, ids[s].first);
+      const PackJob& b = B.get(g.b_buf, ids[s].second);
+      prods.push_back(Prod{a.dst, (int64_t)a.nkt * a_unit_bytes(S), b.dst, (int64_t)b.nkt * b_unit_bytes(S), a.exp,
+                           a.texp, b.exp, a.nkt});
     }
     // runs of products within the bounds of one tile (one run: the whole
     // block, also when no product reaches it)
-    std::vector<std::pair<int, int>> runs;  // (first product, count) relative to ob.seg0
     {
       int r0 = 0;
       int64_t k = 0;
@@ -170,15 +207,14 @@ int build_phase(Builder& B, const std::vector<GemmSeg>& segs, const std::vector<
           t.rms = 1;
           t.pad2 = 0;
           for (int s = run.first; s < run.first + run.second; ++s) {
-            const PackJob& a = B.get(bufs[s].first, ids[s].first);
-            const PackJob& b = B.get(bufs[s].second, ids[s].second);
+            const Prod& p = prods[s];
             OzSeg z;
-            z.a_unit = a.dst + (int64_t)(m0 / kTM) * a.nkt * a_unit_bytes(S);
-            z.b_unit = b.dst + (int64_t)(n0 / kTN) * b.nkt * b_unit_bytes(S);
-            z.a_exp = a.exp + m0;
-            z.b_exp = b.exp + n0;
-            z.a_tmax = a.texp + m0 / kTM;
-            z.nks = a.nkt;
+            z.a_unit = p.a_dst + (m0 / kTM) * p.a_row;
+            z.b_unit = p.b_dst + (n0 / kTN) * p.b_row;
+            z.a_exp = p.a_exp + m0;
+            z.b_exp = p.b_exp + n0;
+            z.a_tmax = p.a_texp + m0 / kTM;
+            z.nks = p.nks;
             z.pad = 0;
             t.work += z.nks;
             oseg->push_back(z);
@@ -272,9 +308,9 @@ void schedule_tiles(std::vector<OzTile>* tiles, const std::vector<OzSeg>& segs, 
       c += segs[s].nks + 5 * ((segs[s].nks + kChunkStages - 1) / kChunkStages);
     cost[i] = c;
   }
-  std::vector<int> order(n);
-  for (int i = 0; i < n; ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+  std::vector<std::pair<int64_t, int>> order(n);  // heaviest first, equal ones by index
+  for (int i = 0; i < n; ++i) order[i] = {-cost[i], i};
+  std::sort(order.begin(), order.end());
   // Longest first to the least-loaded CTA (the lower CTA on equal loads): a
   // binary min-heap on (load, cta), whose top takes each tile's cost and
   // sinks; every (load, cta) key is distinct, so the choices are those of any
@@ -283,8 +319,8 @@ void schedule_tiles(std::vector<OzTile>* tiles, const std::vector<OzSeg>& segs, 
   for (int b = 0; b < grid; ++b) heap[b] = {0, b};
   std::vector<int> count(grid, 0);
   std::vector<int64_t> slot(n);  // position of tile i in the schedule: cta + k * grid
-  for (int i : order) {
-    const int b = heap[0].second;
+  for (const auto& o : order) {
+    const int i = o.second, b = heap[0].second;
     slot[i] = b + (int64_t)count[b]++ * grid;
     heap[0].first += cost[i];
     for (int p = 0;;) {  // sink the top
@@ -314,12 +350,7 @@ int build_ozaki_work(const HeffWork& hw, int S, OzWork* out, std::string* err) {
   w = OzWork();
   w.S = S;
   w.scratch_base = hw.scratch_len;
-  Builder B;
-  B.S = S;
-  B.w = &w;
-  B.lists[0] = &w.jobs[0];
-  B.lists[1] = &w.jobs[1];
-  B.lists[2] = &w.jobs[2];
+  Builder B(S, &w, hw.seg1.size() + hw.seg2.size());
   int rc = build_phase(B, hw.seg1, hw.blk1, &w.seg1, &w.tile1, err, false);
   if (rc) return rc;
   rc = build_phase(B, hw.seg2, hw.blk2, &w.seg2, &w.tile2, err, true);
@@ -329,29 +360,39 @@ int build_ozaki_work(const HeffWork& hw, int S, OzWork* out, std::string* err) {
   // (i+1)*rms - 1, all block rows), the phase-1 tiles leave the row maxima
   // and the pack skips its own pass over the block.
   {
-    std::unordered_map<int64_t, std::vector<int>> by_src;
-    for (int j = 0; j < (int)w.jobs[2].size(); ++j)
-      if (w.jobs[2][j].src_buf == kBufScratch) by_src[w.jobs[2][j].src].push_back(j);
+    const std::vector<PackJob>& feeds = w.jobs[2];
+    IndexTable by_src(feeds.size());  // intermediate origin -> first job that reads it
+    std::vector<char> again(feeds.size(), 0);  // (first jobs) another one reads it too
+    auto origin = [&](int64_t src) -> int& {
+      const uint64_t h = mixed(0, (uint64_t)src);
+      return by_src.find(h ^ h >> 31, [&](int j) { return feeds[j].src == src; });
+    };
+    for (int j = 0; j < (int)feeds.size(); ++j) {
+      if (feeds[j].src_buf != kBufScratch) continue;
+      int& at = origin(feeds[j].src);
+      if (at >= 0) again[at] = 1;
+      else at = j;
+    }
     w.rowmax_base = w.exp_len;
-    std::unordered_map<int64_t, std::pair<int64_t, int>> slots;  // block origin -> (slots, rms)
+    size_t t0 = 0;  // the block's tiles: phase 1 lists them block by block
     for (const OutBlock& ob : hw.blk1) {
-      auto it = by_src.find(ob.c);
-      if (ob.c_buf != kBufScratch || it == by_src.end() || it->second.size() != 1) continue;
-      PackJob& j = w.jobs[2][it->second[0]];
+      const size_t t1 = t0 + (size_t)((std::max(ob.M, 0) + kTM - 1) / kTM) * ((std::max(ob.N, 0) + kTN - 1) / kTN);
+      const size_t first = t0;
+      t0 = t1;
+      const int q = ob.c_buf == kBufScratch ? origin(ob.c) : -1;
+      if (q < 0 || again[q]) continue;
+      PackJob& j = w.jobs[2][q];
       if (j.alpha != 1.0 || j.ld_k != 1 || j.R <= 0 || ob.N % j.R != 0) continue;
       const int rms = ob.N / j.R;
       if (j.ld_r != (int64_t)ob.ldc * rms || j.K != ob.M * rms || ob.ldc != ob.M) continue;
       j.rowmax = w.exp_len;
       w.exp_len += j.R;
-      slots[ob.c] = {j.rowmax, rms};
+      for (size_t t = first; t < t1; ++t) {
+        w.tile1[t].rowmax = j.rowmax;
+        w.tile1[t].rms = rms;
+      }
     }
     w.rowmax_len = w.exp_len - w.rowmax_base;
-    for (OzTile& t : w.tile1) {
-      auto it = slots.find(t.c);
-      if (it == slots.end()) continue;
-      t.rowmax = it->second.first;
-      t.rms = it->second.second;
-    }
   }
   split_phase2(w);
   const int grid = ozaki_persistent_grid();

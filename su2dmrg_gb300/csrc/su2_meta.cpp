@@ -4,11 +4,12 @@
 // host architecture.
 #include "su2_meta.hpp"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
-#include <map>
 #include <mutex>
 #include <tuple>
+#include <unordered_map>
 #include <utility>
 
 namespace su2g {
@@ -95,6 +96,23 @@ void Struct::set_layout(const int* flags) {
     offset[i] = total;
     total += sz;
   }
+}
+
+Buckets bucket(const Struct& s, int l1, int l2) {
+  auto width = [&](int l) {
+    int m = 0;
+    for (int a : s.legs[l].angm) m = std::max(m, a);
+    return m + 1;
+  };
+  Buckets r;
+  r.w2 = l2 >= 0 ? width(l2) : 1;
+  r.b.resize((size_t)width(l1) * r.w2);
+  for (int k = 0; k < s.nten; ++k) {
+    if (!s.flag[k]) continue;
+    const int a1 = s.block_angm(k, l1), a2 = l2 >= 0 ? s.block_angm(k, l2) : 0;
+    if (a1 >= 0 && a2 >= 0) r.b[(size_t)a1 * r.w2 + a2].push_back(k);
+  }
+  return r;
 }
 
 Bond fuse(const Bond& b1, const Bond& b2) {
@@ -292,11 +310,22 @@ double compute_optrans(int side, int j, int m, int l, int i, int k, int p) {
 
 }  // namespace
 
+// A table's entries by their seven indices.
+using FacKey = std::tuple<int, int, int, int, int, int, int>;
+struct FacHash {
+  size_t operator()(const FacKey& k) const {
+    uint64_t h = 0;
+    std::apply([&](auto... x) { ((h = (h ^ (uint32_t)x) * 0x9e3779b97f4a7c15ull, h ^= h >> 29), ...); }, k);
+    return (size_t)h;
+  }
+};
+using FacCache = std::unordered_map<FacKey, double, FacHash>;
+
 double fac_operator_transformation(int side, int j, int m, int l, int i, int k, int p) {
   if (!optrans_defined(j, m, l, i, k, p) || j >= kMaxAngm || l >= kMaxAngm || i >= kMaxAngm || k >= kMaxAngm)
     return 0.0;
   static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int, int, int, int>, double> cache;
+  static FacCache cache;
   const auto key = std::make_tuple(side, j, m, l, i, k, p);
   {
     std::lock_guard<std::mutex> lock(mu);
@@ -332,7 +361,7 @@ bool tri(int a, int b, int c) { return c >= std::abs(a - b) && c <= a + b; }
 template <class F>
 double cached(int table, int side, int a, int b, int c, int d, int e, F compute) {
   static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int, int, int, int>, double> cache;
+  static FacCache cache;
   const auto key = std::make_tuple(table, side, a, b, c, d, e);
   {
     std::lock_guard<std::mutex> lock(mu);

@@ -69,6 +69,22 @@ struct Struct {
   int block_angm(int idx, int leg) const { return legs[leg].angm[block_sector(idx, leg)]; }
 };
 
+// The stored blocks of a tensor grouped by the 2j of one leg (or of two legs),
+// each group in ascending block order: the planners' loops visit exactly
+// the blocks a full scan with the same tests would, in the same order,
+// without scanning every block of one tensor for every block of another.
+struct Buckets {
+  int w2 = 1;
+  std::vector<std::vector<int>> b;
+  const std::vector<int>& at(int a1, int a2 = 0) const {
+    static const std::vector<int> none;
+    if (a1 < 0 || a2 < 0 || a2 >= w2) return none;
+    const size_t key = (size_t)a1 * w2 + a2;
+    return key < b.size() ? b[key] : none;
+  }
+};
+Buckets bucket(const Struct& s, int l1, int l2 = -1);
+
 // true when `locspin` is reachable by fusing angm[0..n) left to right
 bool legal_angm(const int* angm, int n, int locspin);
 

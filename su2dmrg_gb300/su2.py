@@ -125,14 +125,21 @@ class _Pinned:
     def __init__(self, struct):
         self.desc = np.ascontiguousarray(struct.desc(), np.int32)
         self.flag = np.ascontiguousarray(struct.flag, np.int32)
+        self.pdesc, self.pflag = ptr(self.desc), ptr(self.flag)
 
 
-def _tensor(struct: Su2Struct, data, keep: list) -> capi.Tensor:
+def _tensor(struct: Su2Struct, data, keep: list, pinned: dict = None) -> capi.Tensor:
+    """pinned: the structures this call has packed already, by id (operands of
+    one call often share theirs; `keep` holds each of them meanwhile)."""
     if getattr(data, "is_cuda", True) is False:  # a torch tensor in host memory
         raise ValueError("tensor data must be in device memory (numpy arrays for one-site operators)")
-    p = _Pinned(struct)
-    keep.append(p)
-    return capi.Tensor(ptr(p.desc), ptr(p.flag), ptr(data))
+    p = pinned.get(id(struct)) if pinned is not None else None
+    if p is None:
+        p = _Pinned(struct)
+        keep += (p, struct)
+        if pinned is not None:
+            pinned[id(struct)] = p
+    return capi.Tensor(p.pdesc, p.pflag, ptr(data))
 
 
 class _PlanArgs:
@@ -140,10 +147,10 @@ class _PlanArgs:
     the host arrays stay referenced while the call runs."""
 
     def __init__(self, psi, terms, hl, hr):
-        self.keep = []
+        self.keep, seen = [], {}
         self.tarr = (capi.Term * max(1, len(terms)))()
         for i, (s1, x1, s2, x2, c) in enumerate(terms):
-            self.tarr[i] = capi.Term(_tensor(s1, x1, self.keep), _tensor(s2, x2, self.keep), float(c))
+            self.tarr[i] = capi.Term(_tensor(s1, x1, self.keep, seen), _tensor(s2, x2, self.keep, seen), float(c))
         self.h = []
         for h in (hl, hr):
             if h is None:
@@ -431,7 +438,7 @@ class _EnvJobs:
     """ctypes job array; keeps every desc/flag/data array alive for the call."""
 
     def __init__(self, jobs):
-        self.keep = []
+        self.keep, seen = [], {}
         self.arr = (capi.EnvJob * max(1, len(jobs)))()
         for i, jb in enumerate(jobs):
             kind, slot, coef = jb["kind"], jb.get("slot", 0), jb.get("coef", 1.0)
@@ -440,13 +447,13 @@ class _EnvJobs:
             e.slot = int(slot)
             e.coef = float(coef)
             if jb.get("x") is not None:
-                e.x = _tensor(jb["x"][0], jb["x"][1], self.keep)
+                e.x = _tensor(jb["x"][0], jb["x"][1], self.keep, seen)
             for name in ("site1", "site2"):
                 if jb.get(name) is not None:
                     s, d = jb[name]
                     d = np.ascontiguousarray(d, np.float64)  # site operators travel as host data
                     self.keep.append(d)
-                    setattr(e, name, _tensor(s, d, self.keep))
+                    setattr(e, name, _tensor(s, d, self.keep, seen))
         self.n = len(jobs)
 
     @property
@@ -515,14 +522,30 @@ def env_digest(uu, xu, vv, xv, flag: int, jobs, outs, mode: int = capi.MODE_F64)
 
 
 def env_batch(uu, xu, vv, xv, flag: int, jobs, mode: int = capi.MODE_F64, stream=None):
-    """env_layout + allocation + env_run: returns [(Su2Struct, device tensor)] per slot."""
+    """Layouts + allocation + run: returns [(Su2Struct, device tensor)] per slot."""
     import torch
 
     nslots = 1 + max(int(j.get("slot", 0)) for j in jobs)
     dev = xu.device if hasattr(xu, "device") else torch.device("cuda")
-    res = [(st, torch.empty(max(1, st.size()), dtype=torch.float64, device=dev))
-           for st in env_layouts(uu, xu, vv, xv, flag, jobs, range(nslots))]
-    env_run(uu, xu, vv, xv, flag, jobs, [r[1] for r in res], mode, stream)
+    # the operands are packed once, and one call lays out every slot
+    keep = []
+    J = _EnvJobs(jobs)
+    tu, tv = _tensor(uu, xu, keep), _tensor(vv, xv, keep)
+    stride = 4 + 3 * (2 + 2 * 64)
+    desc = np.empty((nslots, stride), np.int32)
+    flags = np.empty(nslots * 64 * len(uu.bonds[-1].angm) * len(vv.bonds[-1].angm), np.int32)
+    size = np.empty(nslots, np.int64)
+    check(lib().su2g_env_layouts(tu, tv, int(flag), J.n, J.ptr, nslots, ptr(desc), stride, ptr(flags), len(flags),
+                                 ptr(size)))
+    res, at = [], 0
+    for d, n in zip(desc, size.tolist()):
+        st = _parse_desc(d)
+        st.flag = flags[at: at + st.nten].copy()
+        at += st.nten
+        res.append((st, torch.empty(max(1, n), dtype=torch.float64, device=dev)))
+    optr = (ctypes.c_void_p * nslots)(*[y.data_ptr() for _, y in res])
+    check(lib().su2g_env_run(tu, tv, int(flag), J.n, J.ptr, nslots, ctypes.addressof(optr), int(mode),
+                             stream_handle(stream)))
     return res
 
 
@@ -550,10 +573,10 @@ def operator_combine(ops, coefs, stream=None):
     structure: returns (Su2Struct with the union of blocks, device tensor)."""
     import torch
 
-    keep = []
+    keep, seen = [], {}
     arr = (capi.Tensor * len(ops))()
     for i, (s, x) in enumerate(ops):
-        arr[i] = _tensor(s, x, keep)
+        arr[i] = _tensor(s, x, keep, seen)
     first = ops[0][0]
     flags = np.zeros(first.nten, np.int32)
     n = ctypes.c_int64()
