@@ -23,14 +23,16 @@
 //
 // What bounds it.  The MMAs of a stage take 910 clocks, and what is left
 // between chunks is the drain of the low groups, about 1,200.  At D = 2000, 18
-// terms, S = 7, the two launches of an application take 1288 + 1297 us (28 BF16
-// products per FP64 product: 1520 TFLOP/s, 0.78 of the measured burst rate)
+// terms, S = 7, the two launches of an application take 1247 + 1297 us (28 BF16
+// products per FP64 product: 1540 TFLOP/s, 0.79 of the measured burst rate)
 // and the GPU runs into its power limit (1350 W, clocks from 2070 to 2040 MHz).
 // They took 1591 + 1691 us while the MMA thread waited and looked at the abort
 // flag between stages, one drain of all groups stood between two chunks, and
 // every tile's exponents, maxima and conversions were chains of global loads,
 // named barriers and FP64 instructions.  At D = 777, 11 terms, the drain warps'
-// work on short tiles still shows: 102 + 100 us (S = 7; 129 + 129 before).
+// work on short tiles still shows: 96 + 96 us (S = 7; 129 + 129 before).  Short
+// tiles are not bound by the conversions' rate: FADDs instead of F2I wherever
+// a short chunk's sums allow them changed nothing, and the added code lost 3%.
 //
 // Every mbarrier wait is bounded; on time-out the CTA records an error code
 // in *err, drains its outstanding tensor-core work and bulk copies (bounded)
@@ -195,8 +197,10 @@ __device__ __noinline__ int subnormal_ilogb(int hi, int lo) {
 // whenever the result is a normal number below 2^1023.  *odd: it is not (or
 // may not be), and scaled_slow gives it.  Two ways to the same bits: integer
 // instructions only, or the FP64 pipe's conversion (2 a clock and SM) and an
-// addition to its exponent field.  A thread takes them by turns, so that the
-// integer pipe and the otherwise idle FP64 pipe share the work.
+// addition to its exponent field.  A thread takes the second for fourteen of its
+// sixteen columns: the integer chains of twenty-odd instructions cost more, in
+// issue slots and in code, than the conversion's rate (by turns, the two
+// launches at D = 2000 take 1272 + 1308 us, so 1247 + 1297; all sixteen 1245 + 1305).
 __device__ __forceinline__ double scaled_by_int(long long v, int e, bool* odd) {
   const unsigned sign = (unsigned)(v >> 32) & 0x80000000u;
   const unsigned long long u = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
@@ -587,6 +591,21 @@ __global__ void __launch_bounds__(kThreads, 1) ozaki_gemm(const OzTile* __restri
       const int emax = bk.emax[row];
       const int nseg = bk.t.nseg;
       const OzSeg* sg = segs + bk.t.seg0;
+      if (lq * 32 >= bk.t.mlen || col0 >= bk.t.nlen) {
+        // Every row or column of this warp lies beyond the block's edge: it
+        // only keeps the barriers' count (D = 200, where a tile is half full:
+        // 18 + 18 -> 16 + 16 us).
+        for (int s = 0; s < nseg && ok; ++s) {
+          const int nchunks = (sg[s].nks + kChunkStages - 1) / kChunkStages;
+          for (int c = 0; c < 2 * nchunks && ok; ++c) {
+            ok = mbar_wait(smem_u32(&bar_accf[c & 1]), chunk & 1, abort_v);
+            if (lane == 0 && ok) mbar_arrive(smem_u32(&bar_acce[c & 1]));
+            chunk += c & 1;
+          }
+        }
+        if (lane == 0 && ok) mbar_arrive(smem_u32(&bar_booke[n & 1]));
+        continue;
+      }
       long long acc[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) acc[j] = 0;
@@ -672,7 +691,7 @@ __global__ void __launch_bounds__(kThreads, 1) ozaki_gemm(const OzTile* __restri
       for (int jj = 0; jj < kCols; ++jj) {
         bool o;
         const int e = ebase + bk.fmax[col0 + jj];
-        out[jj] = jj & 1 ? scaled_by_fp64(acc[jj], e, &o) : scaled_by_int(acc[jj], e, &o);
+        out[jj] = jj % 8 != 1 ? scaled_by_fp64(acc[jj], e, &o) : scaled_by_int(acc[jj], e, &o);
         odd |= o ? 1u << jj : 0u;
       }
       if (odd) {
