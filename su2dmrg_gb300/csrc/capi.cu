@@ -950,10 +950,21 @@ struct LanczosCtx {
     if (su2g::heff_apply_impl(p, ff(m - 1), ff(m), s) != SU2G_OK) return cudaErrorUnknown;
     return su2g::launch_dot_to(ff(m - 1), ff(m), n, p->d_red, alpha(m - 1), s);
   }
-  // runs a step as a CUDA graph, captured on first use
+  // Runs a step: launched directly the first time (a plan of a sweep is solved
+  // once, and capturing and instantiating a graph costs the host more than the
+  // launches: 120 us a solve at D = 123), as a CUDA graph from the second on.
   int run_graph(bool last, int m) {
     std::vector<cudaGraphExec_t>& v = last ? p->lanc_last : p->lanc_step;
+    std::vector<char>& ran = last ? p->lanc_last_ran : p->lanc_step_ran;
     if ((int)v.size() <= m) v.resize(m + 1, nullptr);
+    if ((int)ran.size() <= m) ran.resize(m + 1, 0);
+    if (!ran[m]) {
+      const cudaError_t e = last ? enqueue_last(m, st) : enqueue_step(m, st);
+      if (e != cudaSuccess) return cuda_fail(e, "lanczos step");
+      ran[m] = 1;
+      ++nmatvec;
+      return SU2G_OK;
+    }
     if (!v[m]) {
       if (!p->cap_stream) SU2G_CUDA(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
       SU2G_CUDA(cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal));
@@ -1085,11 +1096,23 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
     tridiag(2);
     return finish(2, false);
   }
+  // The coefficients are read where a check needs them (every fourth step and
+  // the last), so that the device does not wait for the host in between.  A
+  // norm below tol found then ends the solve at its own step, as if it had
+  // been looked at there: what came after is dropped.
+  int seen = 1;
   for (int m = 2; m < mlanc; ++m) {  // lanczos_su2.cpp:155-188
     if ((rc = L.run_graph(false, m))) return rc;
+    if (m % 4 != 0 && m + 1 < mlanc) continue;
     if ((rc = fetch_coefs(m))) return rc;
+    while (++seen <= m)
+      if (nnl[seen] < tol) {
+        L.nmatvec -= m - seen;
+        tridiag(seen);
+        return finish(seen, true);
+      }
+    seen = m;
     tridiag(m);
-    if (nnl[m] < tol) return finish(m, true);
     if (m % 4 == 0) {
       std::vector<double> z0(z.begin(), z.begin() + m);
       if ((rc = L.combine(z0, m, psi))) return rc;

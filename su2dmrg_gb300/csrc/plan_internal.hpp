@@ -47,7 +47,9 @@ struct su2g_heff_plan {
   // graph-captured Lanczos steps: lanc_step[m] produces Krylov vector m
   // (matvec, orthogonalisation, normalisation), lanc_last[m] the final
   // matvec and alpha; captured on cap_stream for this plan's Krylov buffers
+  // the second time a step runs
   std::vector<cudaGraphExec_t> lanc_step, lanc_last;
+  std::vector<char> lanc_step_ran, lanc_last_ran;
   cudaStream_t cap_stream = nullptr;
   double* d_lcoef = nullptr;  // alpha[0..), beta[0..), reorthogonalisation and norm scratch
   int lcoef_m = 0;            // largest mlanc the coefficient layout serves
