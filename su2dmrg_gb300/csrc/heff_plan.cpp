@@ -107,11 +107,18 @@ void add_tiles(std::vector<GemmTile>& tiles, int64_t c_off, int64_t c_len, int c
 // GB300, phase 1 (one product a tile) + phase 2 (all terms), ms: D = 2000, 18
 // terms, K <= 555 and 31,000: whole 64.7 + 72.6, split 67.1 + 67.0; D = 1000:
 // 8.44 + 8.86 and 9.22 + 8.65; D = 400, 12 terms, K <= 105 and 4,000: 0.39 and
-// 0.51 + 0.41; D = 251, 9 terms: phase 2 2.13 whole, 0.096 split.
+// 0.51 + 0.41; D = 251, 9 terms: phase 2 2.13 whole, 0.096 split.  A few
+// products of few values in a row are a chain of load latencies for one warp:
+// phase 2 of D = 24, 2 terms, 16.0 us whole, 6.8 split; D = 8, 4 terms, 17.9
+// and 7.8.  Single products too short to split go in 16 x 16 tiles where 32 x
+// 32 ones are uneven: phase 1 of D = 123, 5 terms (255 tiles of up to 34
+// values), 17.7 -> 14.9 us, D = 200, 6 terms, 47.1 -> 42.5; taking the line
+// further up, D = 251, 9 terms, loses: 84 -> 94.
 namespace {
 constexpr int64_t kF64SplitK = 1024;    // split from this many contracted values on,
-constexpr int64_t kF64MinSplitK = 96;   // and from this many on where 32 x 32 tiles are uneven:
-constexpr double kF64Uneven = 3.0;      // one takes more than a third of an SM's share
+constexpr int64_t kF64MinSplitK = 96;   // and where 32 x 32 tiles are uneven from this many
+constexpr int kF64MinSplitSegs = 3;     // or this many products on;
+constexpr double kF64Uneven = 3.0;      // uneven: one takes more than a third of an SM's share
 }  // namespace
 
 std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles) {
@@ -121,14 +128,17 @@ std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles) {
   auto up = [](int n, int d) { return (n + d - 1) / d; };
   double total = 0, largest = 0;
   int64_t kmax = 0;
+  int segs = 0;
   for (const GemmTile& t : tiles) {
+    segs = std::max(segs, t.nseg);
     total += (double)up(t.mlen, 8) * up(t.nlen, 8) * t.kwork;
     largest = std::max(largest, (double)up(std::min(t.mlen, 32), 8) * up(std::min(t.nlen, 32), 8) * t.kwork);
     kmax = std::max(kmax, t.kwork);
   }
   const bool uneven = largest * kF64Uneven > total / kF64Sms;
-  const bool split = kmax >= kF64SplitK || (kmax >= kF64MinSplitK && uneven);
-  const int side = split ? 8 : 32;
+  const bool split =
+      kmax >= kF64SplitK || (uneven && (kmax >= kF64MinSplitK || (segs >= kF64MinSplitSegs && kmax >= 8)));
+  const int side = split ? 8 : uneven ? 16 : 32;
   std::vector<GemmTile> out;
   for (const GemmTile& t : tiles)
     for (int m = 0; m < t.mlen; m += side)

@@ -42,9 +42,9 @@ int tile_class_for(int M, int N);
 void add_tiles(std::vector<GemmTile>& tiles, int64_t c_off, int64_t c_len, int c_buf, int ldc, int M, int N,
                int seg0, int nseg, int64_t kwork);
 
-// The tiles one phase launches, cut from the planner's: 32 x 32, each element
-// summed by one warp in k order, or 8 x 8 with the contraction split over the
-// CTA's warps.  Which, follows from the phase's output blocks and products
+// The tiles one phase launches, cut from the planner's: 32 x 32 (16 x 16 where
+// those are uneven), each element summed by one warp in k order, or 8 x 8 with
+// the contraction split over the CTA's warps.  Which, follows from the phase's output blocks and products
 // alone (not from the tile classes).
 std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles);
 // how many of each kind a list holds; the list must be ordered by kind (f64_order_by_kind)
