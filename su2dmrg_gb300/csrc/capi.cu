@@ -926,10 +926,6 @@ struct LanczosCtx {
     ++nmatvec;
     return su2g::heff_apply_impl(p, x, y, st);
   }
-  int copy(const double* x, double* y) {
-    cudaError_t e = cudaMemcpyAsync(y, x, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos copy");
-  }
 
   // ---- device-side coefficients: alpha[j], beta[j], q[j] (reorthogonalisation) ----
   int M() const { return p->lcoef_m; }
@@ -991,20 +987,18 @@ struct LanczosCtx {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos fetch");
   }
-  // vout = sum_j z[j] ff[j]  (lanczos_su2::compute_eigenvector, lanczos_su2.cpp:262-279);
-  // leaves the partial sums of its norm in half 0 of the scratch
-  int combine(const std::vector<double>& z, int m, double* vout) {
-    cudaError_t e = su2g::launch_combine_vectors(z.data(), m, ff(0), n, vout, n, p->d_red, 0, st);
+  // vout = sum_j z[j] ff[j]  (lanczos_su2::compute_eigenvector, lanczos_su2.cpp:262-279),
+  // of norm 1 (unit: what a check starts with)
+  int combine(const std::vector<double>& z, int m, double* vout, bool unit) {
+    cudaError_t e = su2g::launch_combine_vectors(z.data(), m, ff(0), n, vout, n, p->d_red, unit, st);
     return e == cudaSuccess ? SU2G_OK : cuda_fail(e, "lanczos combine");
   }
   // lanczos_su2::check_eigenvector (lanczos_su2.cpp:320-332) of the vector
-  // combine() just left in v: normalises it, returns |Hv| and |<Hv,v>|/|Hv|
+  // combine() just left in v: returns |Hv| and |<Hv,v>|/|Hv|
   int check(double* v, double* eig, double* olap) {
-    cudaError_t e = su2g::launch_normalize_part(p->d_red, 0, v, n, nullptr, st);
-    if (e != cudaSuccess) return cuda_fail(e, "lanczos check");
     int rc = matvec(v, tmp());
     if (rc) return rc;
-    e = su2g::launch_dot2(tmp(), v, n, p->d_red, st);
+    const cudaError_t e = su2g::launch_dot2(tmp(), v, n, p->d_red, st);
     if (e != cudaSuccess) return cuda_fail(e, "lanczos check");
     double r[2];  // |Hv|^2, <Hv,v>
     rc = fetch(p->d_red + su2g::lanczos_scratch_doubles() - 2, r, 2);
@@ -1062,7 +1056,7 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
   };
   auto finish = [&](int m, bool do_check) -> int {
     std::vector<double> z0(z.begin(), z.begin() + m);  // ground-state column
-    int r = L.combine(z0, m, psi);
+    int r = L.combine(z0, m, psi, do_check);
     if (r) return r;
     if (do_check) {
       double ee, ov;
@@ -1080,9 +1074,7 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
   };
 
   // ff[0] = normalised start vector (lanczos_su2.cpp:45-46)
-  if ((rc = L.copy(psi, L.ff(0)))) return rc;
-  SU2G_CUDA(su2g::launch_dot_partial(L.ff(0), L.ff(0), n, p->d_red, 0, L.st));
-  SU2G_CUDA(su2g::launch_normalize_part(p->d_red, 0, L.ff(0), n, L.beta(0), L.st));
+  SU2G_CUDA(su2g::launch_unit(psi, L.ff(0), n, p->d_red, L.beta(0), L.st));
   // first step (lanczos_su2.cpp:136-142)
   if ((rc = L.run_graph(false, 1))) return rc;
   if (mlanc == 2) {  // lanczos_su2.cpp:143-154
@@ -1115,7 +1107,7 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
     tridiag(m);
     if (m % 4 == 0) {
       std::vector<double> z0(z.begin(), z.begin() + m);
-      if ((rc = L.combine(z0, m, psi))) return rc;
+      if ((rc = L.combine(z0, m, psi, true))) return rc;
       double ee, ov;
       if ((rc = L.check(psi, &ee, &ov))) return rc;
       if (std::fabs(ov - 1.) < 1.e-8) {  // lanczos_su2.cpp:178-188

@@ -423,9 +423,7 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
   // ff[0] = normalised start vector (lanczos_su2.cpp:45-46)
   for (Solve& s : sv) {
     double* f0 = slice(B->ff(0), s);
-    BATCH_CUDA(cudaMemcpyAsync(f0, s.psi, s.n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    BATCH_CUDA(su2g::launch_dot_partial(f0, f0, s.n, s.red, 0, st));
-    BATCH_CUDA(su2g::launch_normalize_part(s.red, 0, f0, s.n, s.beta(0), st));
+    BATCH_CUDA(su2g::launch_unit(s.psi, f0, s.n, s.red, s.beta(0), st));
   }
   // host copies of the device scalars of several solves, one synchronisation
   std::vector<double> hbuf;
@@ -435,19 +433,19 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
     su2g::tridiag_eigh(d, e, &s.eig, &s.z);
   };
   // psi = sum_j z[j] ff[j]  (lanczos_su2::compute_eigenvector, lanczos_su2.cpp:262-279)
-  auto combine = [&](Solve& s, int m) -> int {
-    BATCH_CUDA(su2g::launch_combine_vectors(s.z.data(), m, slice(B->ff(0), s), B->total, s.psi, s.n, s.red, 0, st));
+  // (unit: of norm 1, what a check starts with)
+  auto combine = [&](Solve& s, int m, bool unit) -> int {
+    BATCH_CUDA(su2g::launch_combine_vectors(s.z.data(), m, slice(B->ff(0), s), B->total, s.psi, s.n, s.red, unit, st));
     return SU2G_OK;
   };
   // lanczos_su2::check_eigenvector (lanczos_su2.cpp:320-332) for every solve
-  // in `who`, whose vector combine() just formed: normalise psi, one shared
-  // matvec, |Hv| and |<Hv,v>|/|Hv|
+  // in `who`, whose vector combine() just formed: one shared matvec, |Hv| and
+  // |<Hv,v>|/|Hv|
   auto checks = [&](const std::vector<int>& who) -> int {
     if (who.empty()) return SU2G_OK;
     hbuf.assign(2 * who.size(), 0.0);
     for (size_t k = 0; k < who.size(); ++k) {
       Solve& s = sv[who[k]];
-      BATCH_CUDA(su2g::launch_normalize_part(s.red, 0, s.psi, s.n, nullptr, st));
       BATCH_CUDA(cudaMemcpyAsync(slice(B->stage(), s), s.psi, s.n * sizeof(double), cudaMemcpyDeviceToDevice, st));
       ++s.nmv;
     }
@@ -498,14 +496,14 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
       if (s.mlanc == 2) {  // lanczos_su2.cpp:143-154
         if (m == 1 && s.nnl[1] >= tol) continue;
         tridiag(s, m);
-        if ((rc = combine(s, m))) return rc;
+        if ((rc = combine(s, m, false))) return rc;
         s.energy = s.eig[0];
         s.active = false;
         continue;
       }
       if (m == s.mlanc) {  // the final step
         tridiag(s, m);
-        if ((rc = combine(s, m))) return rc;
+        if ((rc = combine(s, m, true))) return rc;
         s.pending = Solve::kFinal;
         need_check.push_back(i);
         continue;
@@ -513,11 +511,11 @@ int su2g_heff_batch_lanczos(su2g_heff_batch* B, double* const* psi, int mlanc, d
       if (m < 2) continue;
       tridiag(s, m);
       if (s.nnl[m] < tol) {
-        if ((rc = combine(s, m))) return rc;
+        if ((rc = combine(s, m, true))) return rc;
         s.pending = Solve::kFinal;
         need_check.push_back(i);
       } else if (m % 4 == 0) {
-        if ((rc = combine(s, m))) return rc;
+        if ((rc = combine(s, m, true))) return rc;
         s.pending = Solve::kEarly;
         need_check.push_back(i);
       }

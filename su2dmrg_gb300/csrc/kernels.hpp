@@ -37,25 +37,16 @@ int reduction_scratch_doubles();
 cudaError_t launch_dot(const double* x, const double* y, int64_t n, double* scratch, cudaStream_t stream);
 cudaError_t launch_axpy(double alpha, const double* x, double* y, int64_t n, cudaStream_t stream);
 // The vector work of a Lanczos step with every scalar on the device.  scratch
-// holds lanczos_scratch_doubles(): two halves of partial sums (half 0 or 1,
-// the one a call reads or writes) and two results.
+// holds lanczos_scratch_doubles(): two halves of partial sums and two results.
 int lanczos_scratch_doubles();
 // *out = x . y
 cudaError_t launch_dot_to(const double* x, const double* y, int64_t n, double* scratch, double* out,
                           cudaStream_t stream);
-// the partial sums of x . y into a half
-cudaError_t launch_dot_partial(const double* x, const double* y, int64_t n, double* scratch, int half,
-                               cudaStream_t stream);
-// c = the dot product in `half`, *c_out = c, y -= c x0, y -= (*c1) x1 (c1 null:
-// not), then the partial sums of y . z (z null: y . y) into the other half
-cudaError_t launch_update_dot(double* scratch, int half, double* c_out, const double* x0, const double* c1,
-                              const double* x1, double* y, const double* z, int64_t n, cudaStream_t stream);
-// b = sqrt of the dot product in `half`, x *= 1 / b, *b_out = b (b_out null: not)
-cudaError_t launch_normalize_part(const double* scratch, int half, double* x, int64_t n, double* b_out,
-                                  cudaStream_t stream);
-// v = sum_j z[j] (f + j stride_f) for j < m in order (z on the host), and the partial sums of v . v into `half`
+// out = x / |x|, *b_out = |x| (b_out null: not); x and out may be one vector
+cudaError_t launch_unit(const double* x, double* out, int64_t n, double* scratch, double* b_out, cudaStream_t stream);
+// v = sum_j z[j] (f + j stride_f) for j < m in order (z on the host), then (unit) v /= |v|
 cudaError_t launch_combine_vectors(const double* z, int m, const double* f, int64_t stride_f, double* v, int64_t n,
-                                   double* scratch, int half, cudaStream_t stream);
+                                   double* scratch, bool unit, cudaStream_t stream);
 // x . x and x . y to the two results at the end of scratch
 cudaError_t launch_dot2(const double* x, const double* y, int64_t n, double* scratch, cudaStream_t stream);
 // every launch of a step after its matvec (lanczos_su2.cpp:136-142, 156-173):

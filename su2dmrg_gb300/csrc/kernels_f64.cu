@@ -8,6 +8,8 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "gemm_work.hpp"
@@ -347,8 +349,8 @@ __global__ void __launch_bounds__(kRedThreads) dot_final(const double* __restric
 // m + 3 launches where a dot product, its final sum and an update apiece were
 // 3 m + 7; with the eigenvector's combination below in one launch, a solve on
 // a kept plan (five vectors, seven matvecs) takes 547 us instead of 797 at
-// D = 123 in FP64 and 2459 instead of 2704 at D = 600 with 7 slices.  The
-// same operations on the same values in the same order.
+// D = 123 in FP64 and 2459 instead of 2704 at D = 600 with 7 slices.  (Vectors
+// of up to kClMax elements now go through one cluster, further down.)
 __global__ void __launch_bounds__(kRedThreads) update_dot_kernel(const double* __restrict__ part_in, double* c_out,
                                                                 const double* __restrict__ x0,
                                                                 const double* __restrict__ c1,
@@ -428,6 +430,248 @@ __global__ void __launch_bounds__(kRedThreads) combine_vectors_kernel(CombineCoe
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
+// ---- the same steps on one cluster ----
+// A vector of a few thousand elements is a microsecond's work, and a launch per
+// coefficient (4 to 5 us each, most of it launch, the partial sums' way through
+// L2 and the ramps) is all a Lanczos step's tail then costs.  One cluster of
+// sixteen CTAs holds the vector in registers and goes through the whole tail:
+// the CTAs' sums meet in shared memory (every CTA writes its own to all
+// sixteen), the next vector's elements are loaded while they do.  Each
+// coefficient takes 1.3 to 2 us instead of 5: a chain of FP64 additions, the
+// cluster's barrier (920 clocks) and the FP64 pipe of sixteen SMs, one
+// multiply-add a clock each.  A solve on a new plan (five vectors, FP64) takes
+// 407 us instead of 455 at D = 123 (6,111 elements), 266 instead of 330 at D =
+// 24; 490 instead of 525 at 15,700 elements, but 600 instead of 590 at 17,400.
+constexpr int kClCtas = 16, kClThreads = 128, kClMostElems = 8;
+constexpr int64_t kClMax = (int64_t)kClCtas * kClThreads * kClMostElems;
+
+struct ClusterSum {
+  double part[kClThreads];
+  double cta[2][kClCtas];  // by turns: one is read while the other is written
+  double all;
+};
+
+// The cluster's slice of one thread: E elements, kClThreads apart.  E follows
+// the vector's length (by_elems): an FP64 instruction whose lanes are all
+// switched off holds the pipe as long as any other.
+template <int E>
+struct ClusterSlice {
+  int64_t base;
+  int len;
+  __device__ explicit ClusterSlice(int64_t n) {
+    const int64_t share = (n + kClCtas - 1) / kClCtas, begin = blockIdx.x * share;
+    base = begin + threadIdx.x;
+    len = (int)(min(n, begin + share) - begin) - (int)threadIdx.x;
+  }
+  __device__ bool has(int u) const { return u * kClThreads < len; }
+  __device__ void load(const double* x, double (&r)[E]) const {
+#pragma unroll
+    for (int u = 0; u < E; ++u)
+      if (has(u)) r[u] = x[base + u * kClThreads];
+  }
+  __device__ void store(double* x, const double (&r)[E]) const {
+#pragma unroll
+    for (int u = 0; u < E; ++u)
+      if (has(u)) x[base + u * kClThreads] = r[u];
+  }
+  // this thread's part of a . b
+  __device__ double dot(const double (&a)[E], const double (&b)[E]) const {
+    double v = 0.0;
+#pragma unroll
+    for (int u = 0; u < E; ++u)
+      if (has(u)) v = fma(a[u], b[u], v);
+    return v;
+  }
+  __device__ void axpy(double c, const double (&x)[E], double (&y)[E]) const {
+#pragma unroll
+    for (int u = 0; u < E; ++u)
+      if (has(u)) y[u] = fma(c, x[u], y[u]);
+  }
+  __device__ void scale(double c, double (&y)[E]) const {
+#pragma unroll
+    for (int u = 0; u < E; ++u)
+      if (has(u)) y[u] *= c;
+  }
+};
+
+// The sum of every thread's v over the cluster, in every thread; turn: 0, 1, 0,
+// ...  An FP64 addition keeps the SM's pipe busy for 32 clocks whatever its
+// lanes hold, so one warp does them all, twelve in a row: with a butterfly in
+// every warp (sixteen of them then) a coefficient took 2.9 us.
+__device__ __forceinline__ double cluster_sum(double v, ClusterSum& sh, int turn) {
+  const int lane = threadIdx.x & 31;
+  sh.part[threadIdx.x] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int i = 1; i < kClThreads / 32; ++i) v += sh.part[threadIdx.x + 32 * i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane < kClCtas) {
+      uint32_t to;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;"
+          : "=r"(to)
+          : "r"((uint32_t)__cvta_generic_to_shared(&sh.cta[turn][blockIdx.x])), "r"(lane));
+      asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(v) : "memory");
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (threadIdx.x < 32) {
+    v = sh.cta[turn][lane & (kClCtas - 1)];
+#pragma unroll
+    for (int o = kClCtas / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) sh.all = v;
+  }
+  __syncthreads();
+  return sh.all;
+}
+
+// launch_lanczos_tail in one launch
+template <int E>
+__global__ void __launch_bounds__(kClThreads) lanczos_tail_cluster(int m, double* f, int64_t stride_f, int64_t n,
+                                                                  double* alpha, double* beta, double* q) {
+  __shared__ ClusterSum sh;
+  const ClusterSlice<E> at(n);
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  double y[E], x[E], next[E];
+  at.load(f + m * stride_f, y);
+  at.load(f + (m - 1) * stride_f, x);
+  if (m >= 2) at.load(f + (m - 2) * stride_f, next);
+  int turn = 0;
+  double c = cluster_sum(at.dot(x, y), sh, turn);
+  if (first) alpha[m - 1] = c;
+  at.axpy(-c, x, y);
+  if (m >= 2) {
+    at.axpy(-beta[m - 1], next, y);
+    at.load(f, x);
+    for (int j = 0; j < m; ++j) {
+      const double part = at.dot(x, y);
+      if (j + 1 < m) at.load(f + (j + 1) * stride_f, next);
+      c = cluster_sum(part, sh, turn ^= 1);
+      if (first) q[j] = c;
+      at.axpy(-c, x, y);
+#pragma unroll
+      for (int u = 0; u < E; ++u) x[u] = next[u];
+    }
+  }
+  const double b = sqrt(cluster_sum(at.dot(y, y), sh, turn ^= 1)), s = 1.0 / b;
+  if (first) beta[m] = b;
+  at.scale(s, y);
+  at.store(f + m * stride_f, y);
+}
+
+// out = x / |x|, *b_out = |x| (null: not stored)
+template <int E>
+__global__ void __launch_bounds__(kClThreads) unit_cluster(const double* x, double* out, int64_t n, double* b_out) {
+  __shared__ ClusterSum sh;
+  const ClusterSlice<E> at(n);
+  double y[E];
+  at.load(x, y);
+  const double b = sqrt(cluster_sum(at.dot(y, y), sh, 0)), s = 1.0 / b;
+  if (b_out && blockIdx.x == 0 && threadIdx.x == 0) *b_out = b;
+  at.scale(s, y);
+  at.store(out, y);
+}
+
+// out[0] = x . y, or (two) out[0] = x . x and out[1] = x . y
+template <int E>
+__global__ void __launch_bounds__(kClThreads) dot_cluster(const double* x, const double* y, int64_t n, bool two,
+                                                         double* out) {
+  __shared__ ClusterSum sh;
+  const ClusterSlice<E> at(n);
+  double a[E], b[E];
+  at.load(x, a);
+  at.load(y, b);
+  const double v = cluster_sum(at.dot(a, b), sh, 0);
+  const double w = two ? cluster_sum(at.dot(a, a), sh, 1) : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (two) out[0] = w, out[1] = v;
+    else out[0] = v;
+  }
+}
+
+// v = z_0 f_0 + z_1 f_1 + ... (as combine_vectors_kernel), then v /= |v|
+template <int E>
+__global__ void __launch_bounds__(kClThreads) combine_unit_cluster(CombineCoefs c, int m, const double* f,
+                                                                  int64_t stride_f, double* out, int64_t n) {
+  __shared__ ClusterSum sh;
+  const ClusterSlice<E> at(n);
+  double y[E], x[E];
+  at.load(f, y);
+  at.scale(c.z[0], y);
+  for (int j = 1; j < m; ++j) {
+    at.load(f + j * stride_f, x);
+    at.axpy(c.z[j], x, y);
+  }
+  const double s = 1.0 / sqrt(cluster_sum(at.dot(y, y), sh, 0));
+  at.scale(s, y);
+  at.store(out, y);
+}
+
+cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* attr, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = kClCtas;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg.gridDim = dim3(kClCtas);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// clusters of sixteen, beyond the portable eight, are allowed per kernel
+template <int E>
+bool allow_clusters() {
+  const void* kernels[] = {(const void*)lanczos_tail_cluster<E>, (const void*)unit_cluster<E>,
+                           (const void*)dot_cluster<E>, (const void*)combine_unit_cluster<E>};
+  for (const void* k : kernels) {
+    cudaLaunchAttribute attr = {};
+    const cudaLaunchConfig_t cfg = cluster_config(&attr, nullptr);
+    int most = 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&most, k, &cfg) != cudaSuccess || most < 1) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  return true;
+}
+
+// whether the current device runs them; asked once per device
+bool cluster_runs() {
+  static std::mutex mu;
+  static std::map<int, bool> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  return known[dev] = allow_clusters<1>() && allow_clusters<2>() && allow_clusters<4>() && allow_clusters<8>();
+}
+
+template <class... P, class... A>
+cudaError_t launch_cluster(cudaStream_t stream, void (*kernel)(P...), A... args) {
+  cudaLaunchAttribute attr = {};
+  const cudaLaunchConfig_t cfg = cluster_config(&attr, stream);
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
+// launch(E) with the elements a thread that a vector of n asks for
+template <class F>
+cudaError_t by_elems(int64_t n, F launch) {
+  const int64_t e = (n + kClCtas * kClThreads - 1) / (kClCtas * kClThreads);
+  if (e <= 1) return launch(std::integral_constant<int, 1>());
+  if (e <= 2) return launch(std::integral_constant<int, 2>());
+  if (e <= 4) return launch(std::integral_constant<int, 4>());
+  return launch(std::integral_constant<int, kClMostElems>());
+}
+
+// Vectors of up to kClMax elements go through one cluster, longer ones through
+// the whole chip.
+bool on_cluster(int64_t n) { return n > 0 && n <= kClMax && cluster_runs(); }
+
 __global__ void axpy_kernel(double alpha, const double* __restrict__ x, double* __restrict__ y, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] += alpha * x[i];
@@ -443,21 +687,18 @@ __global__ void scale_kernel(double alpha, double* __restrict__ x, int64_t n) {
 int reduction_scratch_doubles() { return kRedBlocks + 1; }
 int lanczos_scratch_doubles() { return 2 * kRedBlocks + 2; }
 
-cudaError_t launch_dot(const double* x, const double* y, int64_t n, double* scratch, cudaStream_t stream) {
-  return launch_dot_to(x, y, n, scratch, scratch + kRedBlocks, stream);
-}
-
-cudaError_t launch_dot_to(const double* x, const double* y, int64_t n, double* scratch, double* out,
-                          cudaStream_t stream) {
-  cudaError_t e = launch_dot_partial(x, y, n, scratch, 0, stream);
-  if (e != cudaSuccess) return e;
-  dot_final<<<1, kRedThreads, 0, stream>>>(scratch, out);
-  return cudaGetLastError();
-}
-
+namespace {
 cudaError_t launch_dot_partial(const double* x, const double* y, int64_t n, double* scratch, int half,
                                cudaStream_t stream) {
   dot_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch + half * kRedBlocks);
+  return cudaGetLastError();
+}
+
+cudaError_t dot_on_grid(const double* x, const double* y, int64_t n, double* scratch, double* out,
+                        cudaStream_t stream) {
+  cudaError_t e = launch_dot_partial(x, y, n, scratch, 0, stream);
+  if (e != cudaSuccess) return e;
+  dot_final<<<1, kRedThreads, 0, stream>>>(scratch, out);
   return cudaGetLastError();
 }
 
@@ -473,20 +714,54 @@ cudaError_t launch_normalize_part(const double* scratch, int half, double* x, in
   normalize_part_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(scratch + half * kRedBlocks, x, n, b_out);
   return cudaGetLastError();
 }
+}  // namespace
+
+cudaError_t launch_dot(const double* x, const double* y, int64_t n, double* scratch, cudaStream_t stream) {
+  return dot_on_grid(x, y, n, scratch, scratch + kRedBlocks, stream);
+}
+
+cudaError_t launch_dot_to(const double* x, const double* y, int64_t n, double* scratch, double* out,
+                          cudaStream_t stream) {
+  if (on_cluster(n))
+    return by_elems(n, [&](auto E) { return launch_cluster(stream, dot_cluster<E.value>, x, y, n, false, out); });
+  return dot_on_grid(x, y, n, scratch, out, stream);
+}
+
+cudaError_t launch_unit(const double* x, double* out, int64_t n, double* scratch, double* b_out, cudaStream_t stream) {
+  if (on_cluster(n))
+    return by_elems(n, [&](auto E) { return launch_cluster(stream, unit_cluster<E.value>, x, out, n, b_out); });
+  cudaError_t e = x == out ? cudaSuccess
+                           : cudaMemcpyAsync(out, x, n * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+  if (e == cudaSuccess) e = launch_dot_partial(out, out, n, scratch, 0, stream);
+  if (e == cudaSuccess) e = launch_normalize_part(scratch, 0, out, n, b_out, stream);
+  return e;
+}
 
 cudaError_t launch_combine_vectors(const double* z, int m, const double* f, int64_t stride_f, double* v, int64_t n,
-                                   double* scratch, int half, cudaStream_t stream) {
+                                   double* scratch, bool unit, cudaStream_t stream) {
+  if (unit && m <= kCombineMax && on_cluster(n)) {
+    CombineCoefs c{};
+    std::copy(z, z + m, c.z);
+    return by_elems(n, [&](auto E) {
+      return launch_cluster(stream, combine_unit_cluster<E.value>, c, m, f, stride_f, v, n);
+    });
+  }
   for (int j0 = 0; j0 < m; j0 += kCombineMax) {
     CombineCoefs c{};
     const int k = std::min(kCombineMax, m - j0);
     std::copy(z + j0, z + j0 + k, c.z);
     combine_vectors_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(c, k, j0 == 0, f + j0 * stride_f, stride_f, v, n,
-                                                                  scratch + half * kRedBlocks);
+                                                                  scratch);
   }
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess && unit ? launch_normalize_part(scratch, 0, v, n, nullptr, stream) : e;
 }
 
 cudaError_t launch_dot2(const double* x, const double* y, int64_t n, double* scratch, cudaStream_t stream) {
+  if (on_cluster(n))
+    return by_elems(n, [&](auto E) {
+      return launch_cluster(stream, dot_cluster<E.value>, x, y, n, true, scratch + 2 * kRedBlocks);
+    });
   dot2_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch);
   dot_final<<<2, kRedThreads, 0, stream>>>(scratch, scratch + 2 * kRedBlocks);
   return cudaGetLastError();
@@ -494,6 +769,10 @@ cudaError_t launch_dot2(const double* x, const double* y, int64_t n, double* scr
 
 cudaError_t launch_lanczos_tail(int m, double* f, int64_t stride_f, int64_t n, double* alpha, double* beta, double* q,
                                 double* scratch, cudaStream_t stream) {
+  if (on_cluster(n))
+    return by_elems(n, [&](auto E) {
+      return launch_cluster(stream, lanczos_tail_cluster<E.value>, m, f, stride_f, n, alpha, beta, q);
+    });
   auto ff = [&](int j) { return f + j * stride_f; };
   double* y = ff(m);
   cudaError_t e = launch_dot_partial(ff(m - 1), y, n, scratch, 0, stream);
