@@ -31,6 +31,19 @@ cudaError_t launch_gemm_f64(const GemmTile* tiles, const F64Counts& n, const Gem
 cudaError_t launch_gemm_f64_dense(bool transA, int M, int N, int K, const double* A, int lda, const double* B,
                                   int ldb, double* C, int ldc, cudaStream_t stream);
 
+// several of them in one launch (48 at a time): the same sums
+struct DenseGemm {
+  bool transA;
+  int M, N, K;
+  const double* A;
+  int lda;
+  const double* B;
+  int ldb;
+  double* C;
+  int ldc;
+};
+cudaError_t launch_gemm_f64_dense_many(const DenseGemm* jobs, int njobs, cudaStream_t stream);
+
 // deterministic dot product: partial sums in scratch[0..reduction_scratch_doubles()-1),
 // the result in scratch[reduction_scratch_doubles()-1]
 int reduction_scratch_doubles();

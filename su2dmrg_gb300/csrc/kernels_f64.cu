@@ -2,7 +2,7 @@
 //   * gemm_f64_tiles: the block-sparse contraction engine (one CTA per tile of
 //     the work list, gemm_work.hpp), FP64 tensor-core MMA
 //     (mma.sync.m8n8k4.f64) fed from global memory through L1;
-//   * gemm_f64_dense: one dense product with the same tile code;
+//   * gemm_f64_dense: dense products with the same tile code;
 //   * deterministic BLAS-1 (dot, axpy, scale) for the Lanczos iteration.
 #include <cuda_runtime.h>
 
@@ -195,39 +195,53 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_f64_tiles(const GemmTile* __
     for (int n1 = 0; n1 < t.nlen; n1 += 32) sub_tile<2, 4, 2>(t, m1, n1, segs, bases);
 }
 
-// One dense product C = op(A) B in tiles of WM x WN FN fragments, the tile
-// and its segment formed from the kernel's arguments (no work list to
+// One dense product C = op(A) B in tiles of WM x WN FN fragments, the tile at
+// (bx, by) and its segment formed from the kernel's arguments (no work list to
 // upload): the same tile code, so the same sums in the same order as a
 // work-list launch of unsplit tiles.
 template <int FN, int WM, int WN>
-__global__ void __launch_bounds__(WM * WN * 32) gemm_f64_dense(int transA, int M, int N, int K, const double* A,
-                                                              int lda, const double* B, int ldb, double* C, int ldc) {
+__device__ __forceinline__ void dense_tile(const DenseGemm& d, int bx, int by) {
   GemmSeg g;
-  g.a = (int64_t)((uintptr_t)A / 8);
-  g.b = (int64_t)((uintptr_t)B / 8);
+  g.a = (int64_t)((uintptr_t)d.A / 8);
+  g.b = (int64_t)((uintptr_t)d.B / 8);
   g.a_len = 0;
   g.b_len = 0;
   g.a_buf = g.b_buf = kBufAbs;
-  g.lda = lda;
-  g.ldb = ldb;
-  g.K = K;
-  g.transA = transA;
+  g.lda = d.lda;
+  g.ldb = d.ldb;
+  g.K = d.K;
+  g.transA = d.transA;
   g.alpha = 1.0;
   GemmTile t;
-  t.c = (int64_t)((uintptr_t)C / 8);
+  t.c = (int64_t)((uintptr_t)d.C / 8);
   t.c_len = 0;
   t.c_buf = kBufAbs;
-  t.ldc = ldc;
-  t.m0 = blockIdx.x * (WM * 8);
-  t.n0 = blockIdx.y * (WN * FN * 8);
-  t.mlen = min(WM * 8, M - t.m0);
-  t.nlen = min(WN * FN * 8, N - t.n0);
+  t.ldc = d.ldc;
+  t.m0 = bx * (WM * 8);
+  t.n0 = by * (WN * FN * 8);
+  t.mlen = min(WM * 8, d.M - t.m0);
+  t.nlen = min(WN * FN * 8, d.N - t.n0);
   t.seg0 = 0;
   t.nseg = 1;
-  t.kwork = K;
+  t.kwork = d.K;
   t.cls = 0;
   t.ksplit = 0;
   sub_tile<FN, WM, WN>(t, 0, 0, &g, Bases{});
+}
+
+// Several products in one launch: a truncation takes three for every sector and
+// refinement level, each a few microseconds' work for a few dozen CTAs.
+constexpr int kDenseMost = 48;  // 3.3 KB of parameters
+struct DenseList {
+  DenseGemm job[kDenseMost];
+  int first[kDenseMost];  // the job's first tile
+};
+template <int FN, int WM, int WN>
+__global__ void __launch_bounds__(WM * WN * 32) gemm_f64_dense(const __grid_constant__ DenseList list, int njobs) {
+  int j = 0;
+  while (j + 1 < njobs && list.first[j + 1] <= (int)blockIdx.x) ++j;
+  const int tile = blockIdx.x - list.first[j], across = (list.job[j].M + WM * 8 - 1) / (WM * 8);
+  dense_tile<FN, WM, WN>(list.job[j], tile % across, tile / across);
 }
 
 }  // namespace
@@ -235,15 +249,37 @@ __global__ void __launch_bounds__(WM * WN * 32) gemm_f64_dense(int transA, int M
 // Tiles of 32 x 32 once they fill the SMs three times over, else of 16 x 16
 // (the same sums): the operands' traffic is no bound at either size, idle SMs
 // are.
+cudaError_t launch_gemm_f64_dense_many(const DenseGemm* jobs, int njobs, cudaStream_t stream) {
+  auto tiles = [](const DenseGemm& d, int side) {
+    return (int64_t)((d.M + side - 1) / side) * ((d.N + side - 1) / side);
+  };
+  int64_t total = 0;
+  for (int j = 0; j < njobs; ++j) total += tiles(jobs[j], 32);
+  const int side = total >= 3 * kF64Sms ? 32 : 16;
+  for (int j = 0; j < njobs;) {
+    DenseList list{};
+    int n = 0;
+    int64_t first = 0;
+    for (; j < njobs && n < kDenseMost; ++j) {
+      if (jobs[j].M <= 0 || jobs[j].N <= 0) continue;
+      if (n > 0 && first + tiles(jobs[j], side) > INT32_MAX) break;
+      list.job[n] = jobs[j];
+      list.first[n++] = (int)first;
+      first += tiles(jobs[j], side);
+    }
+    if (n == 0) continue;
+    if (side == 32) gemm_f64_dense<2, 4, 2><<<(unsigned)first, 256, 0, stream>>>(list, n);
+    else gemm_f64_dense<1, 2, 2><<<(unsigned)first, 128, 0, stream>>>(list, n);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 cudaError_t launch_gemm_f64_dense(bool transA, int M, int N, int K, const double* A, int lda, const double* B,
                                   int ldb, double* C, int ldc, cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return cudaSuccess;
-  const dim3 big((M + 31) / 32, (N + 31) / 32), small((M + 15) / 16, (N + 15) / 16);
-  if ((int64_t)big.x * big.y >= 3 * kF64Sms)
-    gemm_f64_dense<2, 4, 2><<<big, 256, 0, stream>>>(transA ? 1 : 0, M, N, K, A, lda, B, ldb, C, ldc);
-  else
-    gemm_f64_dense<1, 2, 2><<<small, 128, 0, stream>>>(transA ? 1 : 0, M, N, K, A, lda, B, ldb, C, ldc);
-  return cudaGetLastError();
+  const DenseGemm d{transA, M, N, K, A, lda, B, ldb, C, ldc};
+  return launch_gemm_f64_dense_many(&d, 1, stream);
 }
 
 cudaError_t launch_gemm_f64(const GemmTile* tiles, const F64Counts& n, const GemmSeg* segs, const Bases& bases,

@@ -17,9 +17,9 @@
 //     depend on what else shares the GPU (a library GEMM picks its internal
 //     implementation by the concurrent load, and near a cut in the rounding
 //     noise that changes which multiplets are kept);
-//   * the sectors are independent: each runs on its own stream, cuSOLVER
-//     handle and host thread (the refinement reads eigenvalues back between
-//     steps), so their eigendecompositions overlap on the GPU;
+//   * the sectors go through these steps together, a launch a step for all of
+//     them; their first eigendecompositions run on a stream, cuSOLVER handle and
+//     host thread each;
 //   * on the host: all kept singular values sorted by the Shell sort of
 //     sort2.f (dsort2, whose handling of equal values decides ties), the
 //     largest max_dcut multiplets kept (no (2j+1) weighting), and the
@@ -29,10 +29,12 @@
 #include <cusolverDn.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
 #include <cmath>
+#include <cstring>
 #include <cstdio>
 #include <cstdlib>
 #include <functional>
@@ -52,12 +54,100 @@ namespace {
 
 int fail(int code, const std::string& msg) { return su2g::set_last_error(code, msg); }
 
-__global__ void scale_columns(double* a, int rows, int c0, int ncol, int ld, const double* f) {
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < (int64_t)rows * ncol;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(idx % rows), c = (int)(idx / rows);
-    a[(int64_t)(c0 + c) * ld + r] *= f[c];
+// Every sector's part of a step is one entry of a list in the kernel's
+// parameters (JobList): a step is one launch, whatever the sectors.
+constexpr int kJobMost = 60;
+template <class J>
+struct JobList {
+  J job[kJobMost];
+  int first[kJobMost];  // the job's first CTA
+};
+// kernel(list, njobs) with ctas(job) CTAs for each job
+template <class J, class C, class... A>
+cudaError_t launch_jobs(void (*kernel)(JobList<J>, int, A...), const std::vector<J>& jobs, C ctas, int threads,
+                        size_t smem, cudaStream_t st, A... args) {
+  static_assert(sizeof(JobList<J>) <= 4000, "kernel parameters");
+  for (size_t j = 0; j < jobs.size();) {
+    JobList<J> list;
+    int n = 0, first = 0;
+    for (; j < jobs.size() && n < kJobMost; ++j) {
+      const int c = ctas(jobs[j]);
+      if (c <= 0) continue;
+      list.job[n] = jobs[j];
+      list.first[n++] = first;
+      first += c;
+    }
+    if (n == 0) continue;
+    kernel<<<first, threads, smem, st>>>(list, n, args...);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
+  return cudaSuccess;
+}
+// this CTA's job, and in *cta its number within it
+template <class J>
+__device__ __forceinline__ const J& my_job(const JobList<J>& list, int n, int* cta) {
+  int j = 0;
+  while (j + 1 < n && list.first[j + 1] <= (int)blockIdx.x) ++j;
+  *cta = blockIdx.x - list.first[j];
+  return list.job[j];
+}
+
+struct ScaleJob {  // columns c0 .. c0 + ncol of a (ld rows) times f
+  double* a;
+  int rows, c0, ncol;
+  const double* f;
+};
+__global__ void scale_columns(const __grid_constant__ JobList<ScaleJob> list, int n) {
+  int c;
+  const ScaleJob& j = my_job(list, n, &c);
+  double* col = j.a + (int64_t)(j.c0 + c) * j.rows;
+  const double f = j.f[c];
+  for (int r = threadIdx.x; r < j.rows; r += blockDim.x) col[r] *= f;
+}
+
+struct CopyJob {
+  double* dst;
+  const double* src;
+  int64_t len;
+};
+constexpr int kCopyTile = 1024;
+__global__ void copy_arrays(const __grid_constant__ JobList<CopyJob> list, int n) {
+  int c;
+  const CopyJob& j = my_job(list, n, &c);
+  const int64_t end = min(j.len, (int64_t)(c + 1) * kCopyTile);
+  for (int64_t i = (int64_t)c * kCopyTile + threadIdx.x; i < end; i += blockDim.x) j.dst[i] = j.src[i];
+}
+
+// A matrix (n x n, ld n) as the leading block of one of size N for a batch of
+// equal sizes: beyond it a diagonal below every eigenvalue of a Gram matrix,
+// of the matrix's own scale, so that the padding comes first and its rows stay
+// zero in the others' eigenvectors.  And the vectors back.
+struct PadJob {
+  double* mat;
+  int n;
+  double* box;
+};
+__global__ void pad_matrix(const __grid_constant__ JobList<PadJob> list, int njobs, int N) {
+  __shared__ double smax[8];
+  int c;
+  const PadJob& j = my_job(list, njobs, &c);
+  double mx = 0;
+  for (int i = threadIdx.x; i < j.n; i += blockDim.x) mx = fmax(mx, j.mat[(int64_t)i * j.n + i]);
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  for (int w = 0; w < 8; ++w) mx = fmax(mx, smax[w]);
+  const double below = mx > 0 ? -mx : -1.0;
+  double* col = j.box + (int64_t)c * N;  // one column a CTA
+  for (int r = threadIdx.x; r < N; r += blockDim.x)
+    col[r] = r < j.n && c < j.n ? j.mat[(int64_t)c * j.n + r] : r == c ? below : 0.0;
+}
+__global__ void unpad_vectors(const __grid_constant__ JobList<PadJob> list, int njobs, int N) {
+  int c;
+  const PadJob& j = my_job(list, njobs, &c);
+  const double* col = j.box + (int64_t)(N - j.n + c) * N;
+  for (int r = threadIdx.x; r < j.n; r += blockDim.x) j.mat[(int64_t)c * j.n + r] = col[r];
 }
 
 // out (cols x rows) = in^T, 32 x 32 tiles through shared memory
@@ -76,13 +166,20 @@ __global__ void transpose_kernel(const double* __restrict__ in, int rows, int co
 }
 
 // The eigenvector sign rule of su2g::canonical_column_signs (tridiag.hpp)
-// on the device: one CTA per column of the rows x cols matrix z (ld rows).
+// on the device: one CTA per column of the n x n matrix z.
 // The largest magnitude and the first index above 1e-4 of it are exact
 // reductions (max, min), so the choice does not depend on the order.
-__global__ void __launch_bounds__(256) canonical_signs_kernel(double* z, int rows) {
+struct SignJob {
+  double* z;
+  int n;
+};
+__global__ void __launch_bounds__(256) canonical_signs_kernel(const __grid_constant__ JobList<SignJob> list, int n) {
   __shared__ double smax[8];
   __shared__ int sfirst[8];
-  double* col = z + (int64_t)blockIdx.x * rows;
+  int c;
+  const SignJob& job = my_job(list, n, &c);
+  const int rows = job.n;
+  double* col = job.z + (int64_t)c * rows;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double mx = 0;
   for (int i = threadIdx.x; i < rows; i += blockDim.x) mx = fmax(mx, fabs(col[i]));
@@ -135,13 +232,22 @@ constexpr double kLevelNoise = 8 * 2.220446049250313e-16;  // of the level's lar
 // x = I + E from S (the upper triangle counts; ld n) and P = X^T X (null: X =
 // I).  info[0]: the largest |E_ij| (as bits), lam[i] the eigenvalue estimates.
 // One CTA per column; every CTA finds the decade's first index itself.
-__global__ void __launch_bounds__(256) refine_step_kernel(const double* __restrict__ S, const double* __restrict__ P,
-                                                          int n, double* __restrict__ x, double* __restrict__ lam,
-                                                          unsigned long long* info) {
+struct StepJob {
+  const double *S, *P;
+  int n;
+  double *x, *lam;  // lam: n eigenvalue estimates, then info
+};
+__global__ void __launch_bounds__(256) refine_step_kernel(const __grid_constant__ JobList<StepJob> list, int njobs) {
   extern __shared__ double d[];  // n eigenvalue estimates
   __shared__ double red[8];
   __shared__ int redi[8];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, j = blockIdx.x;
+  int j;
+  const StepJob& job = my_job(list, njobs, &j);
+  const double* __restrict__ S = job.S;
+  const double* __restrict__ P = job.P;
+  const int n = job.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  double *x = job.x, *lam = job.lam;
+  unsigned long long* info = (unsigned long long*)(lam + n);
   double top = 0;
   for (int i = tid; i < n; i += 256) {
     const double v = S[(int64_t)i * n + i] / (P ? P[(int64_t)i * n + i] : 1.0);  // 1 - R_ii = P_ii
@@ -186,7 +292,7 @@ __global__ void __launch_bounds__(256) refine_step_kernel(const double* __restri
 struct Lane {
   cudaStream_t st = nullptr;
   cusolverDnHandle_t sol = nullptr;
-  cudaEvent_t done = nullptr;
+  cusolverDnParams_t params = nullptr;
 };
 struct DeviceRes {
   cudaMemPool_t pool = nullptr;
@@ -221,12 +327,12 @@ std::string take_lanes(int dev, int n, std::vector<Lane>* out, cudaMemPool_t* po
   while ((int)out->size() < n) {
     Lane l;
     if (cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking) != cudaSuccess) return "cannot create a stream";
-    if (cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming) != cudaSuccess) {
+    if (cusolverDnCreateParams(&l.params) != CUSOLVER_STATUS_SUCCESS) {
       cudaStreamDestroy(l.st);
-      return "cannot create an event";
+      return "cannot create cuSOLVER parameters";
     }
     if (cusolverDnCreate(&l.sol) != CUSOLVER_STATUS_SUCCESS) {
-      cudaEventDestroy(l.done);
+      cusolverDnDestroyParams(l.params);
       cudaStreamDestroy(l.st);
       return "cannot create a cuSOLVER handle";
     }
@@ -235,7 +341,7 @@ std::string take_lanes(int dev, int n, std::vector<Lane>* out, cudaMemPool_t* po
     // depend on what else runs on the GPU
     if (cusolverDnSetDeterministicMode(l.sol, CUSOLVER_DETERMINISTIC_RESULTS) != CUSOLVER_STATUS_SUCCESS) {
       cusolverDnDestroy(l.sol);
-      cudaEventDestroy(l.done);
+      cusolverDnDestroyParams(l.params);
       cudaStreamDestroy(l.st);
       return "cannot set the eigensolver's deterministic mode";
     }
@@ -250,10 +356,10 @@ void give_lanes(int dev, const std::vector<Lane>& lanes) {
   r.free_lanes.insert(r.free_lanes.end(), lanes.begin(), lanes.end());
 }
 
-// Host threads that run the sectors of a call (the refinement loop reads
-// eigenvalues back between its steps, so each sector needs its own thread).
-// Kept across calls and grown on demand, instead of one thread per sector per
-// call; never joined (the process ends with them).
+// Host threads for the eigendecompositions of a call (cuSOLVER launches a long
+// chain of kernels from the calling thread).  Kept across calls and grown on
+// demand, instead of one thread per sector per call; never joined (the process
+// ends with them).
 class SectorThreads {
  public:
   static SectorThreads& get() {
@@ -317,19 +423,21 @@ int small_count(const std::vector<double>& w, int n) {
   return 0;
 }
 
-// The work of one sector: its lane, its allocations (from the pool, on the
-// lane's stream; released on `free_st` once the caller's stream has used
-// them) and its error state.
+// One stream's part of a truncation: its allocations (from the pool, on the
+// stream; released on `free_st` once the caller's stream has used them) and its
+// error state.
 struct Ctx {
   cudaStream_t st = nullptr;
   cudaStream_t free_st = nullptr;
   cudaMemPool_t pool = nullptr;
   cusolverDnHandle_t sol = nullptr;
+  cusolverDnParams_t params = nullptr;
   std::vector<void*> allocs;
   std::string err;
   int code = SU2G_OK;
 
-  Ctx() = default;
+  Ctx(const Lane& lane, cudaStream_t free_stream, cudaMemPool_t p)
+      : st(lane.st), free_st(free_stream), pool(p), sol(lane.sol), params(lane.params) {}
   Ctx(const Ctx&) = delete;
   Ctx& operator=(const Ctx&) = delete;
   ~Ctx() {
@@ -342,105 +450,54 @@ struct Ctx {
       err = m;
     }
   }
-  double* dalloc(int64_t n) {
+  void cuda(cudaError_t e) {
+    if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
+  }
+  void* bytes(size_t n) {
     void* p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, std::max<int64_t>(n, 1) * sizeof(double), pool, st);
+    cudaError_t e = cudaMallocFromPoolAsync(&p, std::max<size_t>(n, 8), pool, st);
     if (e != cudaSuccess) {
       set(e == cudaErrorMemoryAllocation ? SU2G_ENOMEM : SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
       return nullptr;
     }
     allocs.push_back(p);
-    return (double*)p;
+    return p;
   }
-  // C (M x N, ld ldc) = op(A) B with op(A) = A (M x K, ld lda) or, for
-  // transA, A^T with A stored K x M; B stored K x N (ld ldb).  The library's
-  // FP64 tile engine (gemm_f64_tiles): every element sums its K products in a
-  // fixed order, whatever else runs on the GPU.
-  void gemm(bool transA, int M, int N, int K, const double* A, int lda, const double* B, int ldb, double* C,
-            int ldc) {
-    if (!ok() || M == 0 || N == 0) return;
-    const cudaError_t e =
-        su2g::launch_gemm_f64_dense(transA, M, N, K, A, lda, B, ldb, C, ldc, st);
-    if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
+  double* dalloc(int64_t n) { return (double*)bytes((size_t)std::max<int64_t>(n, 1) * sizeof(double)); }
+  // products on the library's FP64 tile engine: every element sums its
+  // products in a fixed order, whatever else runs on the GPU
+  void gemms(const std::vector<su2g::DenseGemm>& jobs) {
+    if (ok()) cuda(su2g::launch_gemm_f64_dense_many(jobs.data(), (int)jobs.size(), st));
+  }
+  template <class J, class C, class... A>
+  void launch(void (*kernel)(JobList<J>, int, A...), const std::vector<J>& jobs, C ctas, size_t smem, A... args) {
+    if (ok()) cuda(launch_jobs(kernel, jobs, ctas, 256, smem, st, args...));
+  }
+  void signs(const std::vector<SignJob>& jobs) {
+    launch(canonical_signs_kernel, jobs, [](const SignJob& j) { return j.n; }, 0);
+  }
+  void copies(const std::vector<CopyJob>& jobs) {
+    launch(copy_arrays, jobs, [](const CopyJob& j) { return (int)((j.len + kCopyTile - 1) / kCopyTile); }, 0);
+  }
+  // device -> host, and everything queued so far is done
+  void fetch(void* dst, const void* src, size_t n) {
+    if (!ok()) return;
+    cudaError_t e = cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cuda(e);
   }
   // out (cols x rows) = in^T (in: rows x cols, column-major)
   void transpose(const double* in, int rows, int cols, double* out) {
     if (!ok() || rows == 0 || cols == 0) return;
     const dim3 grid((cols + 31) / 32, (rows + 31) / 32);
     transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(in, rows, cols, out);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
+    cuda(cudaGetLastError());
   }
-  void copy(double* dst, const double* src, int64_t n) {
-    if (!ok()) return;
-    cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
-  }
-  // The eigenvectors of a level's top decade from its nearly diagonal matrix m
-  // (n x n), the rest of the basis orthonormal beside them: x (n x n), lam the
-  // eigenvalues (top decade) and diagonal entries (rest).  False, x undefined,
-  // where the level needs an eigendecomposition: the couplings are too large
-  // for the gaps, the order of the values is not settled, or the subspace left
-  // is the last to be looked at (its values are reported as they are).
-  // y, p, q: n x n scratch.
-  bool refine(const double* m, int n, double lam_cut, double* x, double* y, double* p, double* q,
-              std::vector<double>* lam) {
-    if (n > kRefineMax) return false;
-    double* dlam = dalloc(n + 1);
-    if (!ok()) return false;
-    unsigned long long* info = (unsigned long long*)(dlam + n);
-    std::vector<double> h(n + 1);
-    for (int it = 0; it < 4 && ok(); ++it) {
-      if (it > 0) {
-        gemm(false, n, n, n, m, n, x, n, y, n);
-        gemm(true, n, n, n, x, n, y, n, q, n);  // S
-        gemm(true, n, n, n, x, n, x, n, p, n);  // P
-      }
-      double* step = it > 0 ? y : x;
-      cudaError_t e = cudaMemsetAsync(info, 0, sizeof(*info), st);
-      if (e == cudaSuccess) {
-        refine_step_kernel<<<n, 256, n * sizeof(double), st>>>(it > 0 ? q : m, it > 0 ? p : nullptr, n, step, dlam, info);
-        e = cudaGetLastError();
-      }
-      if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), dlam, (n + 1) * sizeof(double), cudaMemcpyDeviceToHost, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-      if (e != cudaSuccess) {
-        set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
-        return false;
-      }
-      const double big = h[n];
-      const int t0 = small_count(h, n);
-      // the kernel's T: from t0 on, in ascending order, everything below it
-      // smaller than a tenth of the last entry
-      bool good = big <= (it > 0 ? 10 * kStepMax : kStepMax) && h[n - 1] > 0;
-      for (int i = 0; i < n && good; ++i) {
-        const bool in_top = h[i] >= kDecade * h[n - 1];
-        good = in_top == (i >= t0) && (i <= t0 || h[i] >= h[i - 1]);
-      }
-      if (good && it == 0 && t0 > 1) good = !(lam_cut > 0 && h[t0 - 1] < kDecade * lam_cut);
-      if (!good) return false;
-      if (it > 0) {
-        gemm(false, n, n, n, x, n, y, n, q, n);
-        copy(x, q, (int64_t)n * n);
-      }
-      if (big <= kStepDone) {
-        if (!ok()) return false;
-        canonical_signs_kernel<<<n, 256, 0, st>>>(x, n);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
-        h.resize(n);
-        lam->swap(h);
-        return ok();
-      }
-    }
-    return false;
-  }
-  // symmetric eigendecomposition in place (a: n x n, ld n), eigenvector signs
-  // by the canonical rule; w: host eigenvalues
+  // symmetric eigendecomposition in place (a: n x n, ld n); w: host eigenvalues
   void eigh(double* a, int n, std::vector<double>* w) {
     if (!ok()) return;
     int lwork = 0;
-    double* dw = dalloc(n);
+    double* dw = dalloc(n + 1);
     if (!ok()) return;
     if (cusolverDnDsyevd_bufferSize(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, n, a, n, dw, &lwork) !=
         CUSOLVER_STATUS_SUCCESS) {
@@ -448,171 +505,406 @@ struct Ctx {
       return;
     }
     double* work = dalloc(lwork);
-    double* dinfo = dalloc(1);
     if (!ok()) return;
     if (cusolverDnDsyevd(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, n, a, n, dw, work, lwork,
-                         (int*)dinfo) != CUSOLVER_STATUS_SUCCESS) {
+                         (int*)(dw + n)) != CUSOLVER_STATUS_SUCCESS) {
       set(SU2G_ECUDA, "svd: syevd failed");
       return;
     }
-    w->assign(n, 0.0);
+    std::vector<double> h(n + 1);
+    fetch(h.data(), dw, h.size() * sizeof(double));
     int info = 0;
-    cudaError_t e = cudaMemcpyAsync(w->data(), dw, n * sizeof(double), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && n > 0) {
-      canonical_signs_kernel<<<n, 256, 0, st>>>(a, n);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&info, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
-    else if (info != 0) set(SU2G_ECUDA, "svd: syevd did not converge (info " + std::to_string(info) + ")");
+    std::memcpy(&info, &h[n], sizeof(info));
+    if (ok() && info != 0) set(SU2G_ECUDA, "svd: syevd did not converge (info " + std::to_string(info) + ")");
+    w->assign(h.begin(), h.begin() + n);
   }
 };
 
+// A matrix to decompose in place and where its eigenvalues go.
+struct EighJob {
+  double* a;
+  int n;
+  std::vector<double>* w;
+};
+
+// cuSOLVER's solver is a chain of small launches (4.8 ms for 108 rows, 0.4 for
+// 16).  The decompositions that refinement levels still need go through it
+// together, padded to the largest: 14 of up to 54 rows take 1.4 ms.  From 160
+// rows on a batch is the slower way (14 of 160: 10.7 ms, of 555: 69, and 15 ms
+// for one alone).  The first pass keeps a stream and a host thread for each of
+// eight sectors at a time, largest first (a truncation at D = 400, 14 sectors of
+// up to 108 rows: 9.1 ms; 11.1 with all 14 at once, whose threads wait for one
+// another in the driver, 10.6 with six; D = 2000: 95, 97 and 101).  A batch
+// would be faster (6.8), but the Gram matrix is known to its rounding only, so the
+// directions of its smallest eigenvalues are whatever the solver makes of that,
+// and a padded matrix gives other ones: the new tensors move by 7e-10, without
+// it by 6e-11.
+constexpr size_t kEighLanes = 8;
+constexpr int kBatchEigh = 128;
+
+// one sector of the truncation
 struct Sector {
-  int i = -1;      // leg-0 sector index
+  int i = -1;  // leg-0 sector index
   int m = 0, n = 0;
-  int dc = 0;      // singular values kept by the sector's own rule
+  const double* blk = nullptr;
+  bool tall = true;  // the Gram matrix is blk^T blk
+  int k = 0;         // its size
+  double* A0 = nullptr;
+  double* G = nullptr;    // eigenvectors
+  std::vector<double> w;  // eigenvalues, ascending
+  // refinement: the level's size, the size before it, and the buffers
+  int np = 0, npp = 0;
+  double *M = nullptr, *V = nullptr;  // the matrix and the basis it was projected from
+  double* buf[7] = {};                // k x k each
+  double *nextM = nullptr, *x = nullptr, *y = nullptr, *p = nullptr, *q = nullptr;
+  double* lam = nullptr;  // device: npp + 1, as StepJob's
+  const double* h = nullptr;  // the same on the host
+  std::vector<double> ws;     // the level's eigenvalues
+  std::vector<int> levels;    // trace: the levels' sizes
+  // result
+  int dc = 0;           // singular values kept by the sector's own rule
   double* u = nullptr;  // m x dc (ld m), smallest first
   double* v = nullptr;  // n x dc (ld n)
   std::vector<double> s;  // dc values, ascending
-};
 
-// First pass of tensor::svd for one m x n block (n0 = 1): the Gram matrix of
-// the smaller side and its eigendecomposition (tensor.cpp:1484-1490).
-struct SectorEig {
-  bool tall = true;
-  int k = 0;
-  // trace: host wall time of the two passes, refinement subspace sizes
-  double ms_eig = 0, ms_finish = 0;
-  std::vector<int> levels;
-  double* G = nullptr;   // eigenvectors (k x k)
-  double* A0 = nullptr;  // the Gram matrix
-  std::vector<double> w;  // eigenvalues, ascending
-};
-
-void sector_eig(Ctx& c, const double* blk, int m, int n, SectorEig* e) {
-  e->tall = m >= n;
-  const int k = e->k = e->tall ? n : m;
-  e->G = c.dalloc((int64_t)k * k);
-  e->A0 = c.dalloc((int64_t)k * k);
-  if (!c.ok()) return;
-  if (e->tall) {
-    c.gemm(true, n, n, m, blk, m, blk, m, e->G, n);  // blk^T blk
-  } else {  // blk blk^T = (blk^T)^T (blk^T)
-    double* bt = c.dalloc((int64_t)m * n);
-    c.transpose(blk, m, n, bt);
-    c.gemm(true, m, m, n, bt, n, bt, n, e->G, m);
+  // buffers for the next level: those that M and V do not hold
+  void assign() {
+    int at = 0;
+    auto next = [&] {
+      while (buf[at] == M || buf[at] == V) ++at;
+      return buf[at++];
+    };
+    nextM = next();
+    x = next();
+    y = next();
+    p = next();
+    q = next();
   }
-  c.copy(e->A0, e->G, (int64_t)k * k);
-  c.eigh(e->G, k, &e->w);  // G now holds the eigenvectors
-}
+};
 
-// Second pass: the reference's refinement of the small-eigenvalue subspace
-// (tensor.cpp:1491-1529), then the factors.  Each refinement re-solves the
-// subspace of eigenvalues below 0.1 of its largest and rotates only those
-// columns, so a subspace whose largest eigenvalue is below 0.1 of lam_cut (the
-// max_dcut-th largest eigenvalue over all sectors, 0 when every multiplet is
-// kept or when the cut is too close to the first pass's rounding error to be
-// placed) holds no multiplet the truncation keeps: refining it further changes
-// neither the kept columns, their values nor the selection, and is skipped
-// (its values, all discarded, stay those of the last refinement).
-void sector_finish(Ctx& c, const double* blk, int m, int n, double p1, double p2, int max_dcut, double lam_cut,
-                   SectorEig& e, Sector* out) {
-  const bool tall = e.tall;
-  const int k = e.k;
-  double* G = e.G;
-  std::vector<double>& w = e.w;
-  if (!c.ok()) return;
-  int np = small_count(w, k);
-  if (np > 1 && !(lam_cut > 0 && w[np - 1] < 0.1 * lam_cut)) {
-    double* ap = c.dalloc((int64_t)k * k);
-    double* vp = c.dalloc((int64_t)k * k);
-    double* app = c.dalloc((int64_t)k * k);
-    double* vpp = c.dalloc((int64_t)k * k);
-    double* tmp = c.dalloc((int64_t)k * k);
-    double* scr = c.dalloc((int64_t)k * k);
-    c.copy(ap, e.A0, (int64_t)k * k);
-    c.copy(vp, G, (int64_t)k * k);
-    int npp = np;
-    np = k;
-    std::vector<double> ws;
-    do {
-      e.levels.push_back(npp);
-      c.gemm(true, npp, np, np, vp, np, ap, np, app, npp);
-      c.gemm(false, npp, npp, np, app, npp, vp, np, vpp, npp);
-      c.copy(ap, vpp, (int64_t)npp * npp);
-      // the level's eigenvectors: by refinement of the basis at hand, else (ap
-      // still holds the matrix) by an eigendecomposition
-      if (!c.refine(ap, npp, lam_cut, vpp, app, tmp, scr, &ws)) {
-        c.copy(vpp, ap, (int64_t)npp * npp);
-        c.eigh(vpp, npp, &ws);
+// The sectors of a truncation in lockstep: every step (a product, a
+// correction, a copy) is one launch for all of them, and the host reads all
+// their eigenvalues back at once.  With a stream and a host thread for each
+// sector, ten launches a level and sector fought for the driver: nine levels of
+// 14 sectors took 5 ms, in lockstep 2.6, half of it the last levels' solver.
+class Truncation {
+ public:
+  // decomposes the jobs on other streams and runs `beside` meanwhile
+  using OnLanes = std::function<void(const std::vector<EighJob>&, const std::function<void()>& beside)>;
+  Truncation(Ctx& ctx, std::vector<Sector>& sectors, OnLanes lanes)
+      : c(ctx), secs(sectors), on_lanes(std::move(lanes)) {}
+
+  // First pass of tensor::svd (n0 = 1): the Gram matrix of every sector's
+  // smaller side and its eigendecomposition (tensor.cpp:1484-1490).
+  void first_pass() {
+    std::vector<su2g::DenseGemm> gram;
+    std::vector<CopyJob> keep;
+    std::vector<EighJob> eig;
+    std::vector<SignJob> signs;
+    for (Sector& s : secs) {
+      s.tall = s.m >= s.n;
+      const int k = s.k = std::min(s.m, s.n), r = std::max(s.m, s.n);
+      const int64_t kk = (int64_t)k * k;
+      s.A0 = c.dalloc(kk);
+      s.G = c.dalloc(kk);
+      const double* b = s.blk;
+      if (!s.tall) {  // blk blk^T = (blk^T)^T (blk^T)
+        double* bt = c.dalloc((int64_t)s.m * s.n);
+        if (!c.ok()) return;
+        c.transpose(s.blk, s.m, s.n, bt);
+        b = bt;
       }
       if (!c.ok()) return;
-      for (int q = 0; q < npp; ++q) w[q] = ws[q];
-      c.gemm(false, k, npp, npp, G, k, vpp, npp, tmp, k);
-      c.copy(G, tmp, (int64_t)k * npp);
-      c.copy(vp, vpp, (int64_t)npp * npp);
-      const int j = small_count(ws, npp);
-      np = npp;
-      npp = j;
-      if (npp > 1 && lam_cut > 0 && ws[npp - 1] < 0.1 * lam_cut) break;
-    } while (npp > 1 && c.ok());
+      gram.push_back({true, k, k, r, b, r, b, r, s.A0, k});
+      keep.push_back({s.G, s.A0, kk});
+      eig.push_back({s.G, k, &s.w});
+      signs.push_back({s.G, k});
+    }
+    c.gemms(gram);
+    c.copies(keep);
+    eigh(eig, false);
+    c.signs(signs);  // G now holds the eigenvectors
   }
-  if (!c.ok()) return;
-  double *U, *V;
-  if (tall) {  // V = eigenvectors (n x n), U = blk V (m x n)
-    V = G;
-    U = c.dalloc((int64_t)m * n);
-    c.gemm(false, m, n, n, blk, m, V, n, U, m);
-  } else {  // U = eigenvectors (m x m), V = blk^T U (n x m)
-    U = G;
-    V = c.dalloc((int64_t)n * m);
-    c.gemm(true, n, m, m, blk, m, U, m, V, n);
+
+  // The reference's refinement of the small-eigenvalue subspaces
+  // (tensor.cpp:1491-1529).  Each refinement re-solves the
+  // subspace of eigenvalues below 0.1 of its largest and rotates only those
+  // columns, so a subspace whose largest eigenvalue is below 0.1 of lam_cut (the
+  // max_dcut-th largest eigenvalue over all sectors, 0 when every multiplet is
+  // kept or when the cut is too close to the first pass's rounding error to be
+  // placed) holds no multiplet the truncation keeps: refining it further changes
+  // neither the kept columns, their values nor the selection, and is skipped
+  // (its values, all discarded, stay those of the last refinement).
+  void refine(double lam_cut) {
+    cut = lam_cut;
+    std::vector<Sector*> run, wait;
+    int64_t nlam = 0;
+    for (Sector& s : secs) {
+      s.npp = small_count(s.w, s.k);
+      if (s.npp <= 1 || beyond_cut(s.w, s.npp)) continue;
+      s.np = s.k;
+      s.M = s.A0;
+      s.V = s.G;
+      for (double*& b : s.buf) b = c.dalloc((int64_t)s.k * s.k);
+      nlam += s.k + 1;
+      run.push_back(&s);
+    }
+    lam_dev = c.dalloc(nlam);
+    if (!c.ok()) return;
+    lam_host.resize(nlam);
+    int64_t at = 0;
+    for (Sector* s : run) {
+      s->lam = lam_dev + at;
+      s->h = lam_host.data() + at;
+      at += s->k + 1;
+    }
+    // Sectors whose level needs an eigendecomposition wait until no other can
+    // go on without one: they are decomposed together.
+    while (c.ok() && !(run.empty() && wait.empty())) {
+      if (run.empty()) {
+        std::vector<CopyJob> copies;
+        std::vector<EighJob> eig;
+        for (Sector* s : wait) {
+          copies.push_back({s->x, s->nextM, (int64_t)s->npp * s->npp});
+          eig.push_back({s->x, s->npp, &s->ws});
+        }
+        c.copies(copies);
+        eigh(eig, true);
+        run = finish_level(wait);
+        wait.clear();
+        continue;
+      }
+      const std::vector<Sector*> solved = level(run, &wait);
+      run = finish_level(solved);
+    }
   }
-  if (!c.ok()) return;
-  // singular values above 1e-100 of the largest, scaling (tensor.cpp:1532-1567)
-  const double num = w[k - 1];
-  int dcut = 0;
-  if (num > 1.e-100)
-    for (int i = k - 1; i >= 0; --i) {
-      if (w[i] / num > 1.e-100) {
-        w[i] = std::sqrt(w[i]);
-        ++dcut;
-      } else {
-        w[i] = 0;
+
+  // The other factors, singular values above 1e-100 of the largest, scaling
+  // (tensor.cpp:1530-1567).
+  void factors(double p1, double p2, int max_dcut) {
+    std::vector<su2g::DenseGemm> gemms;
+    std::vector<double> f;
+    for (Sector& s : secs) {
+      const int m = s.m, n = s.n, k = s.k;
+      double *U, *V;
+      if (s.tall) {  // V = eigenvectors (n x n), U = blk V (m x n)
+        V = s.G;
+        U = c.dalloc((int64_t)m * n);
+        gemms.push_back({false, m, n, n, s.blk, m, V, n, U, m});
+      } else {  // U = eigenvectors (m x m), V = blk^T U (n x m)
+        U = s.G;
+        V = c.dalloc((int64_t)n * m);
+        gemms.push_back({true, n, m, m, s.blk, m, U, m, V, n});
+      }
+      const double num = s.w[k - 1];
+      int dcut = 0;
+      if (num > 1.e-100)
+        for (int i = k - 1; i >= 0; --i) {
+          if (s.w[i] / num > 1.e-100) {
+            s.w[i] = std::sqrt(s.w[i]);
+            ++dcut;
+          } else {
+            s.w[i] = 0;
+          }
+        }
+      if (dcut > max_dcut) dcut = max_dcut;
+      s.dc = dcut;
+      s.u = U;
+      s.v = V;
+      s.s.assign(s.w.begin() + (k - dcut), s.w.begin() + k);
+      for (int side = 0; side < 2; ++side)
+        for (double x : s.s) {
+          const double down = s.tall ? std::pow(x, p1 - 1.) : std::pow(x, p1);
+          const double across = s.tall ? std::pow(x, p2) : std::pow(x, p2 - 1.);
+          f.push_back(x > 0 ? (side ? across : down) : 0.0);
+        }
+    }
+    c.gemms(gemms);
+    double* df = c.dalloc((int64_t)f.size());
+    if (!c.ok()) return;
+    if (!f.empty()) c.cuda(cudaMemcpyAsync(df, f.data(), f.size() * sizeof(double), cudaMemcpyHostToDevice, c.st));
+    std::vector<ScaleJob> scale;
+    int64_t at = 0;
+    for (Sector& s : secs) {
+      scale.push_back({s.u, s.m, s.k - s.dc, s.dc, df + at});
+      scale.push_back({s.v, s.n, s.k - s.dc, s.dc, df + at + s.dc});
+      at += 2 * s.dc;
+      s.u += (int64_t)s.m * (s.k - s.dc);
+      s.v += (int64_t)s.n * (s.k - s.dc);
+    }
+    c.launch(scale_columns, scale, [](const ScaleJob& j) { return j.ncol; }, 0);
+  }
+
+ private:
+  bool beyond_cut(const std::vector<double>& w, int n) const { return cut > 0 && w[n - 1] < kDecade * cut; }
+
+  // eigendecompositions in place, signs as they come: each on a stream and
+  // host thread of its own, or (together) the small ones as a batch beside them
+  void eigh(const std::vector<EighJob>& jobs, bool together) {
+    std::vector<EighJob> small, alone;
+    for (const EighJob& j : jobs) (together && j.n <= kBatchEigh ? small : alone).push_back(j);
+    if (alone.empty()) {
+      batch(small);
+    } else if (c.ok()) {
+      c.cuda(cudaStreamSynchronize(c.st));  // the matrices are there for the other streams
+      if (c.ok()) on_lanes(alone, [&] { batch(small); });
+    }
+  }
+  void batch(const std::vector<EighJob>& small) {
+    if (small.size() == 1) {
+      c.eigh(small[0].a, small[0].n, small[0].w);
+    } else if (!small.empty()) {
+      int N = 0;
+      for (const EighJob& j : small) N = std::max(N, j.n);
+      const int nb = (int)small.size();
+      double* box = c.dalloc((int64_t)nb * N * N);
+      double* dw = c.dalloc((int64_t)nb * (N + 1));  // eigenvalues, then info
+      if (!c.ok()) return;
+      int* info = (int*)(dw + (int64_t)nb * N);
+      std::vector<PadJob> pads;
+      for (int q = 0; q < nb; ++q) pads.push_back({small[q].a, small[q].n, box + (int64_t)q * N * N});
+      c.launch(pad_matrix, pads, [&](const PadJob&) { return N; }, 0, N);
+      size_t ldev = 0, lhost = 0;
+      if (c.ok() && cusolverDnXsyevBatched_bufferSize(c.sol, c.params, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER,
+                                                      N, CUDA_R_64F, box, N, CUDA_R_64F, dw, CUDA_R_64F, &ldev, &lhost,
+                                                      nb) != CUSOLVER_STATUS_SUCCESS)
+        c.set(SU2G_ECUDA, "svd: syev buffer query failed");
+      void* work = c.bytes(ldev);
+      std::vector<uint8_t> host(lhost);
+      if (c.ok() && cusolverDnXsyevBatched(c.sol, c.params, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, N,
+                                           CUDA_R_64F, box, N, CUDA_R_64F, dw, CUDA_R_64F, work, ldev, host.data(),
+                                           lhost, info, nb) != CUSOLVER_STATUS_SUCCESS)
+        c.set(SU2G_ECUDA, "svd: syev failed");
+      c.launch(unpad_vectors, pads, [](const PadJob& j) { return j.n; }, 0, N);
+      std::vector<double> h((size_t)nb * (N + 1));
+      c.fetch(h.data(), dw, h.size() * sizeof(double));
+      if (!c.ok()) return;
+      const int* hinfo = (const int*)(h.data() + (size_t)nb * N);
+      for (int q = 0; q < nb; ++q) {
+        if (hinfo[q] != 0)
+          c.set(SU2G_ECUDA, "svd: syev did not converge (info " + std::to_string(hinfo[q]) + ")");
+        small[q].w->assign(h.begin() + (size_t)q * N + (N - small[q].n), h.begin() + (size_t)(q + 1) * N);
       }
     }
-  if (dcut > max_dcut) dcut = max_dcut;
-  if (dcut > (tall ? m : n)) dcut = tall ? m : n;
-  std::vector<double> fu(dcut), fv(dcut);
-  for (int q = 0; q < dcut; ++q) {
-    const double s = w[k - dcut + q];
-    if (s > 0) {
-      fu[q] = tall ? std::pow(s, p1 - 1.) : std::pow(s, p1);
-      fv[q] = tall ? std::pow(s, p2) : std::pow(s, p2 - 1.);
-    } else {
-      fu[q] = fv[q] = 0.0;
+  }
+
+  // One level of every sector of `run`: the Gram matrix projected on the
+  // subspace (nextM) and its eigenvectors (x) by refinement of the basis at
+  // hand.  Returns the sectors solved; the others, for which couplings are too
+  // large for the gaps, the order of the values is not settled, or the
+  // subspace left is the last to be looked at (its values are reported as they
+  // are), go to `wait`.
+  std::vector<Sector*> level(const std::vector<Sector*>& run, std::vector<Sector*>* wait) {
+    std::vector<su2g::DenseGemm> g1, g2;
+    for (Sector* s : run) {
+      const int np = s->np, npp = s->npp;
+      s->assign();
+      s->levels.push_back(npp);
+      g1.push_back({true, npp, np, np, s->V, np, s->M, np, s->y, npp});
+      g2.push_back({false, npp, npp, np, s->y, npp, s->V, np, s->nextM, npp});
     }
+    c.gemms(g1);
+    c.gemms(g2);
+    std::vector<Sector*> open, solved;
+    for (Sector* s : run) (s->npp <= kRefineMax ? open : *wait).push_back(s);
+    for (int it = 0; it < 4 && !open.empty() && c.ok(); ++it) {
+      if (it > 0) {
+        g1.clear();
+        g2.clear();
+        for (Sector* s : open) {
+          const int n = s->npp;
+          g1.push_back({false, n, n, n, s->nextM, n, s->x, n, s->y, n});
+          g2.push_back({true, n, n, n, s->x, n, s->y, n, s->q, n});  // S
+          g2.push_back({true, n, n, n, s->x, n, s->x, n, s->p, n});  // P
+        }
+        c.gemms(g1);
+        c.gemms(g2);
+      }
+      std::vector<StepJob> step;
+      int most = 0;
+      for (Sector* s : open) {
+        step.push_back({it > 0 ? s->q : s->nextM, it > 0 ? s->p : nullptr, s->npp, it > 0 ? s->y : s->x, s->lam});
+        most = std::max(most, s->npp);
+      }
+      if (c.ok()) c.cuda(cudaMemsetAsync(lam_dev, 0, lam_host.size() * sizeof(double), c.st));
+      c.launch(refine_step_kernel, step, [](const StepJob& j) { return j.n; }, most * sizeof(double));
+      c.fetch(lam_host.data(), lam_dev, lam_host.size() * sizeof(double));
+      if (!c.ok()) return {};
+      std::vector<Sector*> more;
+      g1.clear();
+      for (Sector* s : open) {
+        const int n = s->npp;
+        if (!settled(*s, it)) {
+          wait->push_back(s);
+          continue;
+        }
+        if (it > 0) {
+          g1.push_back({false, n, n, n, s->x, n, s->y, n, s->q, n});
+          std::swap(s->x, s->q);
+        }
+        if (s->h[n] <= kStepDone) {
+          s->ws.assign(s->h, s->h + n);
+          solved.push_back(s);
+        } else {
+          more.push_back(s);
+        }
+      }
+      c.gemms(g1);
+      open = more;
+    }
+    wait->insert(wait->end(), open.begin(), open.end());
+    return solved;
   }
-  if (dcut > 0) {
-    double* dfu = c.dalloc(dcut);
-    double* dfv = c.dalloc(dcut);
-    if (!c.ok()) return;
-    cudaMemcpyAsync(dfu, fu.data(), dcut * sizeof(double), cudaMemcpyHostToDevice, c.st);
-    cudaMemcpyAsync(dfv, fv.data(), dcut * sizeof(double), cudaMemcpyHostToDevice, c.st);
-    scale_columns<<<256, 256, 0, c.st>>>(U, m, k - dcut, dcut, m, dfu);
-    scale_columns<<<256, 256, 0, c.st>>>(V, n, k - dcut, dcut, n, dfv);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) c.set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
+
+  // whether a step of the refinement may be taken (kernel's T: from t0 on, in
+  // ascending order, everything below it smaller than a tenth of the last entry)
+  bool settled(const Sector& s, int it) const {
+    const int n = s.npp;
+    const std::vector<double> h(s.h, s.h + n);
+    const int t0 = small_count(h, n);
+    bool good = s.h[n] <= (it > 0 ? 10 * kStepMax : kStepMax) && h[n - 1] > 0;
+    for (int i = 0; i < n && good; ++i) {
+      const bool in_top = h[i] >= kDecade * h[n - 1];
+      good = in_top == (i >= t0) && (i <= t0 || h[i] >= h[i - 1]);
+    }
+    if (good && it == 0 && t0 > 1) good = !beyond_cut(h, t0);
+    return good;
   }
-  out->m = m;
-  out->n = n;
-  out->dc = dcut;
-  out->u = U + (int64_t)m * (k - dcut);
-  out->v = V + (int64_t)n * (k - dcut);
-  out->s.assign(w.begin() + (k - dcut), w.begin() + k);
-}
+
+  // Rotates the solved sectors' columns and goes on to their next levels;
+  // returns the sectors that have one.
+  std::vector<Sector*> finish_level(const std::vector<Sector*>& solved) {
+    std::vector<SignJob> signs;
+    std::vector<su2g::DenseGemm> rotate;
+    std::vector<CopyJob> copies;
+    std::vector<Sector*> next;
+    if (!c.ok()) return next;
+    for (Sector* s : solved) {
+      const int k = s->k, n = s->npp;
+      signs.push_back({s->x, n});
+      // s->G may still be the basis of the first level: it is not read after this
+      rotate.push_back({false, k, n, n, s->G, k, s->x, n, s->y, k});
+      copies.push_back({s->G, s->y, (int64_t)k * n});
+      std::copy(s->ws.begin(), s->ws.end(), s->w.begin());
+      s->V = s->x;
+      s->M = s->nextM;
+      s->np = n;
+      s->npp = small_count(s->ws, n);
+      if (s->npp > 1 && !beyond_cut(s->ws, s->npp)) next.push_back(s);
+    }
+    c.signs(signs);
+    c.gemms(rotate);
+    c.copies(copies);
+    return next;
+  }
+
+  Ctx& c;
+  std::vector<Sector>& secs;
+  OnLanes on_lanes;
+  double cut = 0;
+  double* lam_dev = nullptr;
+  std::vector<double> lam_host;
+};
 
 }  // namespace
 
@@ -637,8 +929,8 @@ extern "C" int su2g_svd(const int* psi_desc, const int* psi_flag, const double* 
   if (P.total > 0 && !psi) return fail(SU2G_EINVAL, "svd: null psi");
   cudaStream_t cst = (cudaStream_t)stream;
   // SU2G_SVD_TRACE=<file>: one JSON line per call appended there (per sector:
-  // m, n, Gram size, host milliseconds of the two passes, the sizes of the
-  // refinement subspaces), for time breakdowns of whole sweeps
+  // m, n, Gram size, host milliseconds of the call's two passes, the sizes of
+  // the refinement subspaces), for time breakdowns of whole sweeps
   const char* trace = std::getenv("SU2G_SVD_TRACE");
   if (trace && !*trace) trace = nullptr;
   const auto t_call = std::chrono::steady_clock::now();
@@ -657,9 +949,10 @@ extern "C" int su2g_svd(const int* psi_desc, const int* psi_flag, const double* 
   int dev = 0;
   cudaError_t ce = cudaGetDevice(&dev);
   if (ce != cudaSuccess) return fail(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(ce));
+  // lane 0 for everything the sectors share, the others for decompositions
   std::vector<Lane> lanes;
   cudaMemPool_t pool = nullptr;
-  const std::string rerr = take_lanes(dev, (int)jobs.size(), &lanes, &pool);
+  const std::string rerr = take_lanes(dev, 1 + (int)std::min<size_t>(jobs.size(), kEighLanes), &lanes, &pool);
   if (!rerr.empty()) {
     give_lanes(dev, lanes);
     return fail(SU2G_ECUDA, "svd: " + rerr);
@@ -670,50 +963,54 @@ extern "C" int su2g_svd(const int* psi_desc, const int* psi_flag, const double* 
     const std::vector<Lane>& lanes;
     ~LaneReturn() { give_lanes(dev, lanes); }
   } lane_return{dev, lanes};
-  // every sector on its own lane (stream + handles) and host thread: the
-  // eigendecompositions and the refinement loops of all sectors overlap
-  cudaEvent_t ready = nullptr;
-  ce = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
-  if (ce == cudaSuccess) ce = cudaEventRecord(ready, cst);
-  if (ce != cudaSuccess) {
-    if (ready) cudaEventDestroy(ready);
-    return fail(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(ce));
-  }
-  std::vector<std::unique_ptr<Ctx>> ctx(jobs.size());
+  std::vector<std::unique_ptr<Ctx>> ctx;
+  for (const Lane& l : lanes) ctx.emplace_back(new Ctx(l, cst, pool));
+  Ctx& c = *ctx[0];
   std::vector<Sector> secs(jobs.size());
   for (size_t q = 0; q < jobs.size(); ++q) {
-    ctx[q].reset(new Ctx());
-    Ctx& c = *ctx[q];
-    c.st = lanes[q].st;
-    c.free_st = cst;
-    c.pool = pool;
-    c.sol = lanes[q].sol;
-    const cudaError_t we = cudaStreamWaitEvent(c.st, ready, 0);  // psi is written on the caller's stream
-    if (we != cudaSuccess) c.set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(we));
+    secs[q].i = jobs[q].i;
+    secs[q].m = jobs[q].m;
+    secs[q].n = jobs[q].n;
+    secs[q].blk = psi + P.offset[jobs[q].b];
   }
-  // two passes over the sectors, each sector on its own host thread: the
-  // eigendecompositions, then (with the global cut known) the refinements
-  // and the factors
-  std::vector<SectorEig> eig(jobs.size());
-  double lam_cut = 0.0, lam_cut_raw = 0.0, noise_floor = 0.0;
-  auto on_threads = [&](const std::function<void(size_t)>& body) { SectorThreads::get().run(jobs.size(), body); };
-  on_threads([&](size_t q) {
-    Ctx& c = *ctx[q];
-    if (cudaSetDevice(dev) != cudaSuccess) c.set(SU2G_ECUDA, "svd: cannot select the device");
-    const auto t0 = std::chrono::steady_clock::now();
-    if (c.ok()) sector_eig(c, psi + P.offset[jobs[q].b], jobs[q].m, jobs[q].n, &eig[q]);
-    eig[q].ms_eig = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  // psi is written on the caller's stream
+  cudaEvent_t order = nullptr;
+  ce = cudaEventCreateWithFlags(&order, cudaEventDisableTiming);
+  if (ce == cudaSuccess) ce = cudaEventRecord(order, cst);
+  if (ce == cudaSuccess) ce = cudaStreamWaitEvent(c.st, order, 0);
+  c.cuda(ce);
+  Truncation tr(c, secs, [&](const std::vector<EighJob>& alone, const std::function<void()>& beside) {
+    // largest first, each lane taking the next when it is through with one
+    std::vector<EighJob> order(alone);
+    std::stable_sort(order.begin(), order.end(), [](const EighJob& x, const EighJob& y) { return x.n > y.n; });
+    std::atomic<size_t> next{0};
+    SectorThreads::get().run(std::min(ctx.size() - 1, alone.size()) + 1, [&](size_t q) {
+      if (q == 0) {
+        beside();
+        return;
+      }
+      Ctx& mine = *ctx[q];
+      mine.cuda(cudaSetDevice(dev));
+      for (size_t j = next++; j < order.size(); j = next++) mine.eigh(order[j].a, order[j].n, order[j].w);
+    });
+    for (size_t q = 1; q < ctx.size(); ++q)
+      if (!ctx[q]->ok()) c.set(ctx[q]->code, ctx[q]->err);
   });
-  {  // the max_dcut-th largest eigenvalue over all sectors; 0 (refine every
-     // subspace, as the reference) when nothing is cut or when the cut lies
-     // within 1e3 of the first pass's error k eps lambda_max of some sector,
-     // where values near it are not yet known well enough to place them
+  const auto t_eig = std::chrono::steady_clock::now();
+  if (c.ok()) tr.first_pass();
+  const auto t_refine = std::chrono::steady_clock::now();
+  double lam_cut = 0.0, lam_cut_raw = 0.0, noise_floor = 0.0;
+  if (c.ok()) {
+    // the max_dcut-th largest eigenvalue over all sectors; 0 (refine every
+    // subspace, as the reference) when nothing is cut or when the cut lies
+    // within 1e3 of the first pass's error k eps lambda_max of some sector,
+    // where values near it are not yet known well enough to place them
     std::vector<double> all;
     double floor = 0.0;
-    for (const SectorEig& e : eig) {
-      const double top = e.w.empty() ? 0.0 : e.w.back();
-      floor = std::max(floor, (double)e.k * 2.3e-16 * top);
-      for (double v : e.w)
+    for (const Sector& s : secs) {
+      const double top = s.w.empty() ? 0.0 : s.w.back();
+      floor = std::max(floor, (double)s.k * 2.3e-16 * top);
+      for (double v : s.w)
         if (v > 0 && v / top > 1.e-100) all.push_back(v);
     }
     if (max_dcut > 0 && (int64_t)all.size() > max_dcut) {
@@ -722,26 +1019,19 @@ extern "C" int su2g_svd(const int* psi_desc, const int* psi_flag, const double* 
       if (lam_cut < 1e3 * floor) lam_cut = 0.0;
     }
     noise_floor = floor;
+    tr.refine(lam_cut);
   }
-  on_threads([&](size_t q) {
-    Ctx& c = *ctx[q];
-    if (cudaSetDevice(dev) != cudaSuccess) c.set(SU2G_ECUDA, "svd: cannot select the device");
-    const auto t0 = std::chrono::steady_clock::now();
-    if (c.ok()) {
-      secs[q].i = jobs[q].i;
-      sector_finish(c, psi + P.offset[jobs[q].b], jobs[q].m, jobs[q].n, p1, p2, max_dcut, lam_cut, eig[q],
-                    &secs[q]);
-    }
-    if (trace) cudaStreamSynchronize(c.st);
-    eig[q].ms_finish = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    const cudaError_t e = cudaEventRecord(lanes[q].done, c.st);
-    if (e != cudaSuccess) c.set(SU2G_ECUDA, std::string("svd: ") + cudaGetErrorString(e));
-  });
-  // the caller's stream continues after every sector (placement copies, frees)
-  for (size_t q = 0; q < jobs.size(); ++q) cudaStreamWaitEvent(cst, lanes[q].done, 0);
-  cudaEventDestroy(ready);
-  for (const auto& c : ctx)
-    if (!c->ok()) return fail(c->code, c->err);
+  if (c.ok()) tr.factors(p1, p2, max_dcut);
+  if (trace) cudaStreamSynchronize(c.st);
+  const auto t_done = std::chrono::steady_clock::now();
+  // the caller's stream continues after the sectors' (placement copies, frees)
+  if (order) {
+    ce = cudaEventRecord(order, c.st);
+    if (ce == cudaSuccess) ce = cudaStreamWaitEvent(cst, order, 0);
+    cudaEventDestroy(order);
+    c.cuda(ce);
+  }
+  if (!c.ok()) return fail(c.code, c.err);
   // global selection of the max_dcut largest multiplets (tensor_su2.cpp:1686-1695)
   std::vector<double> ws;
   std::vector<int> is;
@@ -830,8 +1120,10 @@ extern "C" int su2g_svd(const int* psi_desc, const int* psi_flag, const double* 
                    ms, max_dcut, lam_cut, lam_cut_raw, noise_floor, total_kept);
       for (size_t q = 0; q < jobs.size(); ++q) {
         std::fprintf(f, "%s{\"m\": %d, \"n\": %d, \"k\": %d, \"ms_eig\": %.3f, \"ms_finish\": %.3f, \"levels\": [",
-                     q ? ", " : "", jobs[q].m, jobs[q].n, eig[q].k, eig[q].ms_eig, eig[q].ms_finish);
-        for (size_t l = 0; l < eig[q].levels.size(); ++l) std::fprintf(f, "%s%d", l ? ", " : "", eig[q].levels[l]);
+                     q ? ", " : "", jobs[q].m, jobs[q].n, secs[q].k,
+                     std::chrono::duration<double, std::milli>(t_refine - t_eig).count(),
+                     std::chrono::duration<double, std::milli>(t_done - t_refine).count());
+        for (size_t l = 0; l < secs[q].levels.size(); ++l) std::fprintf(f, "%s%d", l ? ", " : "", secs[q].levels[l]);
         std::fprintf(f, "]}");
       }
       std::fprintf(f, "]}\n");
