@@ -890,7 +890,7 @@ int su2g_vec_dot(const double* x, const double* y, int64_t n, double* result, vo
   cudaStream_t st = (cudaStream_t)stream;
   double* scratch = nullptr;
   const int ns = su2g::reduction_scratch_doubles();
-  SU2G_CUDA(cudaMallocAsync((void**)&scratch, ns * sizeof(double), st));
+  SU2G_CUDA(su2g::stream_alloc((void**)&scratch, ns * sizeof(double), st));
   cudaError_t e = su2g::launch_dot(x, y, n, scratch, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(result, scratch + ns - 1, sizeof(double), cudaMemcpyDeviceToHost, st);
   cudaFreeAsync(scratch, st);

@@ -8,7 +8,10 @@
 // memory is usable on any stream when dev_alloc returns), and a free is queued
 // on the stream the buffer was last used on, so it is returned to the pool only
 // once that stream has passed it; nothing ever waits for other streams.  Freed
-// blocks stay cached in the pool up to kKeepBytes.
+// blocks stay cached in the pool up to kKeepBytes.  A one-shot call's scratch is
+// taken on the call's own stream (stream_alloc): the device's default pool gives
+// its memory back to the system at every synchronisation, and mapping it again
+// took an input vector at D = 1500 (12 MB of scratch) 220 us of its 473.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -80,6 +83,16 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
   if (e == cudaSuccess) e = setup_stream(&st);
   if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  return e;
+}
+
+cudaError_t stream_alloc(void** p, size_t bytes, cudaStream_t st) {
+  *p = nullptr;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  cudaMemPool_t pool = nullptr;
+  if (e == cudaSuccess) e = device_pool(dev, &pool);
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, st);
   return e;
 }
 

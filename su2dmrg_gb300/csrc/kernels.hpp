@@ -18,6 +18,8 @@ int set_last_error(int code, const std::string& msg);
 // synchronises the device.
 cudaError_t dev_alloc(void** p, size_t bytes);
 void dev_free(void* p, cudaStream_t after);
+// the same pool, for use on `st` alone
+cudaError_t stream_alloc(void** p, size_t bytes, cudaStream_t st);
 // dev_alloc + a copy of `bytes` host bytes, complete on return
 cudaError_t upload_bytes(const void* host, size_t bytes, void** dptr);
 // the calling thread's private non-blocking stream on the current device

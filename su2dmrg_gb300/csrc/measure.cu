@@ -96,8 +96,8 @@ cudaError_t run_sums(const std::vector<SumItem>& items, std::vector<double>* sum
   if (items.empty()) return cudaSuccess;
   SumItem* d_items = nullptr;
   double* d_out = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&d_items, items.size() * sizeof(SumItem), st);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_out, items.size() * sizeof(double), st);
+  cudaError_t e = su2g::stream_alloc((void**)&d_items, items.size() * sizeof(SumItem), st);
+  if (e == cudaSuccess) e = su2g::stream_alloc((void**)&d_out, items.size() * sizeof(double), st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(SumItem), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
@@ -237,7 +237,7 @@ extern "C" int su2g_multiply_singular_value(const int* desc, const int* flag, do
   ScaleItem* d_items = nullptr;
   std::vector<ScaleItem> items;
   int64_t maxlen = 0;
-  cudaError_t e = cudaMallocAsync((void**)&d_w, off.back() * sizeof(double), st);
+  cudaError_t e = su2g::stream_alloc((void**)&d_w, off.back() * sizeof(double), st);
   for (int b = 0; b < s.nten && e == cudaSuccess; ++b) {
     if (!s.flag[b]) continue;
     ScaleItem it{};
@@ -253,7 +253,7 @@ extern "C" int su2g_multiply_singular_value(const int* desc, const int* flag, do
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_w, w, off.back() * sizeof(double), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && !items.empty()) {
     if (items.size() > 65535) e = cudaErrorInvalidValue;
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_items, items.size() * sizeof(ScaleItem), st);
+    if (e == cudaSuccess) e = su2g::stream_alloc((void**)&d_items, items.size() * sizeof(ScaleItem), st);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(ScaleItem), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
@@ -283,7 +283,7 @@ extern "C" int su2g_mea_enr(su2g_tensor hl, su2g_tensor hr, const double* ww, in
     return fail(SU2G_EINVAL, "mea_enr: fewer weights than multiplets of hr");
   cudaStream_t st = (cudaStream_t)stream;
   double* d_w = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&d_w, nww * sizeof(double), st);
+  cudaError_t e = su2g::stream_alloc((void**)&d_w, nww * sizeof(double), st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_w, ww, nww * sizeof(double), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) {
     if (d_w) cudaFreeAsync(d_w, st);

@@ -127,7 +127,7 @@ cudaError_t launch_transposes(std::vector<TrItem>& items, cudaStream_t st) {
   }
   TrItem* d_items = nullptr;
   const size_t bytes = live.size() * sizeof(TrItem);
-  cudaError_t e = cudaMallocAsync((void**)&d_items, bytes, st);
+  cudaError_t e = su2g::stream_alloc((void**)&d_items, bytes, st);
   if (e != cudaSuccess) return e;
   e = cudaMemcpyAsync(d_items, live.data(), bytes, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
@@ -281,7 +281,7 @@ extern "C" int su2g_vectran(su2g_tensor u, int flag, double* out, void* stream) 
   cudaError_t e = cudaSuccess;
   const bool overlap = out < u.data + in.total && u.data < out + in.total;
   if (overlap) {
-    e = cudaMallocAsync((void**)&copy, in.total * sizeof(double), st);
+    e = su2g::stream_alloc((void**)&copy, in.total * sizeof(double), st);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(copy, u.data, in.total * sizeof(double), cudaMemcpyDeviceToDevice, st);
     src = copy;
@@ -320,7 +320,7 @@ extern "C" int su2g_prepare_input_vector(su2g_tensor ul, su2g_tensor ur, double*
   cudaStream_t st = (cudaStream_t)stream;
   double* urt = nullptr;  // ur's blocks transposed, at ur's own offsets
   cudaError_t e = cudaMemsetAsync(out, 0, v.total * sizeof(double), st);
-  if (e == cudaSuccess && R.total > 0) e = cudaMallocAsync((void**)&urt, R.total * sizeof(double), st);
+  if (e == cudaSuccess && R.total > 0) e = su2g::stream_alloc((void**)&urt, R.total * sizeof(double), st);
   if (e == cudaSuccess && R.total > 0) {
     std::vector<TrItem> items;
     for (int b = 0; b < R.nten; ++b) {
@@ -374,7 +374,7 @@ extern "C" int su2g_fuse_tensor(const int* bonds_desc, double* out, void* stream
   OneItem* d_items = nullptr;
   cudaError_t e = cudaMemsetAsync(out, 0, f.total * sizeof(double), st);
   if (e == cudaSuccess && items.size() > 65535) e = cudaErrorInvalidValue;
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_items, items.size() * sizeof(OneItem), st);
+  if (e == cudaSuccess) e = su2g::stream_alloc((void**)&d_items, items.size() * sizeof(OneItem), st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(OneItem), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
@@ -481,7 +481,7 @@ extern "C" int su2g_random_vector(int64_t* state, double* out, int64_t n, void* 
   cudaError_t e = cudaGetLastError();
   const int ns = su2g::reduction_scratch_doubles();
   double* scratch = nullptr;
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&scratch, ns * sizeof(double), st);
+  if (e == cudaSuccess) e = su2g::stream_alloc((void**)&scratch, ns * sizeof(double), st);
   for (int pass = 0; pass < 2 && e == cudaSuccess; ++pass) {  // random_initialize_tensor, then the caller
     e = su2g::launch_dot(out, out, n, scratch, st);
     if (e == cudaSuccess) {
