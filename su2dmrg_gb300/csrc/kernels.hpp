@@ -90,9 +90,11 @@ cudaError_t bounded_wait_selftest(long long limit, int* timed_out_host, cudaStre
 // CTAs of the persistent GEMM grid on the current device (its SM count); 152
 // when no device answers (host-only planning and validation).
 int ozaki_persistent_grid();
-// row-exponent pass (when rows_pass) + digit pass: 1 or 2 kernels, none for nunits == 0
+// row-exponent pass (when rows_pass) + digit pass: 1 or 2 kernels, none for nunits == 0;
+// before them clear[0, nclear) = 0 (part of the row pass where there is one)
 cudaError_t launch_pack(int S, const PackJob* jobs, const int2* units, int nunits, int max_nkt, bool rows_pass,
-                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream);
+                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream, int* clear = nullptr,
+                        int nclear = 0);
 cudaError_t launch_ozaki_gemm(int S, const OzTile* tiles, int ntiles, const OzSeg* segs, const uint8_t* packed,
                               int* exps, const Bases& bases, int* err, cudaStream_t stream);
 int gemm_smem_bytes(int S);

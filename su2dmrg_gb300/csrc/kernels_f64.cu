@@ -14,6 +14,7 @@
 
 #include "gemm_work.hpp"
 #include "kernels.hpp"
+#include "overlap.cuh"
 
 namespace su2g {
 namespace {
@@ -45,16 +46,16 @@ __device__ __forceinline__ void dmma_m8n8k4(double (&d)[2], double a, double b) 
 // that are never stored; values past K are zero in both operands.
 template <int FN>
 __device__ __forceinline__ void seg_mma(const GemmSeg& g, const Bases& bases, int row, const int (&col)[FN], int nj,
-                                        int step0, int step1, int fc, double (&sacc)[FN][2]) {
+                                        int step0, int step1, int fc, int64_t zero, double (&sacc)[FN][2]) {
   constexpr int U = 4;
 #pragma unroll
   for (int j = 0; j < FN; ++j) sacc[j][0] = sacc[j][1] = 0.0;
   const int64_t ks = g.transA ? 1 : g.lda;  // distance of neighbouring k in A
   const int k = step0 * 4 + fc;
-  const double* ap = resolve(bases, g.a_buf, g.a) + (g.transA ? (int64_t)row * g.lda : row) + k * ks;
+  const double* ap = after_wait(resolve(bases, g.a_buf, g.a), zero) + (g.transA ? (int64_t)row * g.lda : row) + k * ks;
   const double* bp[FN];
 #pragma unroll
-  for (int j = 0; j < FN; ++j) bp[j] = resolve(bases, g.b_buf, g.b) + (int64_t)col[j] * g.ldb + k;
+  for (int j = 0; j < FN; ++j) bp[j] = after_wait(resolve(bases, g.b_buf, g.b), zero) + (int64_t)col[j] * g.ldb + k;
   int step = step0;
   const int full = min(step1, g.K / 4);
   for (; step + U <= full; step += U) {
@@ -105,7 +106,7 @@ __device__ __forceinline__ void add_scaled(double alpha, const double (&sacc)[FN
 // order whatever the tile shape.
 template <int FN, int WM, int WN>
 __device__ __forceinline__ void sub_tile(const GemmTile& t, int m1, int n1, const GemmSeg* __restrict__ segs,
-                                         const Bases& bases) {
+                                         const Bases& bases, int64_t zero) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wr = warp % WM, wc = warp / WM;
   const int fr = lane >> 2, fc = lane & 3;
@@ -120,7 +121,7 @@ __device__ __forceinline__ void sub_tile(const GemmTile& t, int m1, int n1, cons
   for (int s = t.seg0; s < t.seg0 + t.nseg; ++s) {
     const GemmSeg g = segs[s];
     double sacc[FN][2];
-    seg_mma<FN>(g, bases, row, col, nj, 0, (g.K + 3) / 4, fc, sacc);
+    seg_mma<FN>(g, bases, row, col, nj, 0, (g.K + 3) / 4, fc, zero, sacc);
     add_scaled<FN>(g.alpha, sacc, acc);
   }
   double* C = resolve(bases, t.c_buf, t.c);
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_f64_ksplit(const GemmTile* _
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
   const int lo = (int)((int64_t)total * warp / kWarps), hi = (int)((int64_t)total * (warp + 1) / kWarps);
+  const int64_t zero = wait_for_predecessor();
   for (int s0 = 0, base = 0; s0 < t.nseg && base < hi; s0 += 32) {
     const int n = s0 + lane < t.nseg ? (segs[t.seg0 + s0 + lane].K + 3) / 4 : 0;
     int end = n;  // inclusive prefix sum
@@ -167,11 +169,15 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_f64_ksplit(const GemmTile* _
       const int e1 = __shfl_sync(0xffffffffu, end, b), e0 = e1 - __shfl_sync(0xffffffffu, n, b);
       const GemmSeg g = segs[t.seg0 + s0 + b];
       double sacc[1][2];
-      seg_mma<1>(g, bases, row, col, 1, max(lo - e0, 0), min(hi, e1) - e0, fc, sacc);
+      seg_mma<1>(g, bases, row, col, 1, max(lo - e0, 0), min(hi, e1) - e0, fc, zero, sacc);
       add_scaled<1>(g.alpha, sacc, acc);
     }
     base = __shfl_sync(0xffffffffu, end, 31);
   }
+  // Not earlier: the next launch's CTAs would take whatever slots are free, four
+  // heavy ones on one SM while others idle, instead of spreading (an
+  // application at D = 123: 38 us, with nothing overlapped 28, like this 23).
+  dependents_may_start();
   part[warp * 64 + lane] = acc[0][0];
   part[warp * 64 + 32 + lane] = acc[0][1];
   __syncthreads();
@@ -187,12 +193,14 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_f64_ksplit(const GemmTile* _
   }
 }
 
-// One CTA per whole tile of the work list, 32 x 32 at a time.
+// One CTA per whole tile of the work list, 32 x 32 at a time.  (The dependents
+// start as the CTAs end, for the reason given above.)
 __global__ void __launch_bounds__(kThreads, 4) gemm_f64_tiles(const GemmTile* __restrict__ tiles,
                                                               const GemmSeg* __restrict__ segs, Bases bases) {
   const GemmTile t = tiles[blockIdx.x];
+  const int64_t zero = wait_for_predecessor();
   for (int m1 = 0; m1 < t.mlen; m1 += 32)
-    for (int n1 = 0; n1 < t.nlen; n1 += 32) sub_tile<2, 4, 2>(t, m1, n1, segs, bases);
+    for (int n1 = 0; n1 < t.nlen; n1 += 32) sub_tile<2, 4, 2>(t, m1, n1, segs, bases, zero);
 }
 
 // One dense product C = op(A) B in tiles of WM x WN FN fragments, the tile at
@@ -226,7 +234,7 @@ __device__ __forceinline__ void dense_tile(const DenseGemm& d, int bx, int by) {
   t.kwork = d.K;
   t.cls = 0;
   t.ksplit = 0;
-  sub_tile<FN, WM, WN>(t, 0, 0, &g, Bases{});
+  sub_tile<FN, WM, WN>(t, 0, 0, &g, Bases{}, 0);
 }
 
 // Several products in one launch: a truncation takes three for every sector and
@@ -284,10 +292,11 @@ cudaError_t launch_gemm_f64_dense(bool transA, int M, int N, int K, const double
 
 cudaError_t launch_gemm_f64(const GemmTile* tiles, const F64Counts& n, const GemmSeg* segs, const Bases& bases,
                             cudaStream_t stream) {
-  if (n.whole > 0) gemm_f64_tiles<<<n.whole, kThreads, 0, stream>>>(tiles, segs, bases);
-  tiles += n.whole;
-  if (n.split > 0) gemm_f64_ksplit<<<n.split, kThreads, 0, stream>>>(tiles, segs, bases);
-  return cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  if (n.whole > 0) e = launch_overlapped(gemm_f64_tiles, dim3(n.whole), kThreads, 0, 0, stream, tiles, segs, bases);
+  if (e == cudaSuccess && n.split > 0)
+    e = launch_overlapped(gemm_f64_ksplit, dim3(n.split), kThreads, 0, 0, stream, tiles + n.whole, segs, bases);
+  return e;
 }
 
 namespace {
@@ -316,7 +325,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 }
 
 // a dot product's value from its kRedBlocks partial sums, in every thread
-__device__ __forceinline__ double sum_partials(const double* __restrict__ part, double* sh) {
+__device__ __forceinline__ double sum_partials(const double* part, double* sh) {
   double v = 0;
 #pragma unroll
   for (int i = 0; i < kRedBlocks; i += kRedThreads) v += part[i + threadIdx.x];
@@ -337,9 +346,11 @@ __device__ __forceinline__ void grid_stride4(int64_t n, F f) {
   for (; i < n; i += stride) f(i, stride, std::integral_constant<int, 1>());
 }
 
-__global__ void __launch_bounds__(kRedThreads) dot_partial(const double* __restrict__ x, const double* __restrict__ y,
-                                                          int64_t n, double* __restrict__ part) {
+__global__ void __launch_bounds__(kRedThreads) dot_partial(const double* x_in, const double* y_in, int64_t n, double* part) {
   __shared__ double sh[kRedThreads];
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  const double *x = after_wait(x_in, zero), *y = after_wait(y_in, zero);
   double v = 0;
   grid_stride4(n, [&](int64_t i, int64_t stride, auto U) {
     double a[U.value], b[U.value];
@@ -353,9 +364,11 @@ __global__ void __launch_bounds__(kRedThreads) dot_partial(const double* __restr
 }
 
 // x . x and x . y in one pass
-__global__ void __launch_bounds__(kRedThreads) dot2_partial(const double* __restrict__ x, const double* __restrict__ y,
-                                                           int64_t n, double* __restrict__ part) {
+__global__ void __launch_bounds__(kRedThreads) dot2_partial(const double* x_in, const double* y_in, int64_t n, double* part) {
   __shared__ double sh[kRedThreads];
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  const double *x = after_wait(x_in, zero), *y = after_wait(y_in, zero);
   double v = 0, w = 0;
   grid_stride4(n, [&](int64_t i, int64_t stride, auto U) {
     double a[U.value], b[U.value];
@@ -369,9 +382,11 @@ __global__ void __launch_bounds__(kRedThreads) dot2_partial(const double* __rest
 }
 
 // out[b] = the value of the dot product whose partial sums are part[b kRedBlocks ..]
-__global__ void __launch_bounds__(kRedThreads) dot_final(const double* __restrict__ part, double* __restrict__ out) {
+__global__ void __launch_bounds__(kRedThreads) dot_final(const double* part, double* out) {
   __shared__ double sh[kRedThreads];
-  const double s = sum_partials(part + blockIdx.x * kRedBlocks, sh);
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  const double s = sum_partials(after_wait(part, zero) + blockIdx.x * kRedBlocks, sh);
   if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
@@ -387,13 +402,14 @@ __global__ void __launch_bounds__(kRedThreads) dot_final(const double* __restric
 // a kept plan (five vectors, seven matvecs) takes 547 us instead of 797 at
 // D = 123 in FP64 and 2459 instead of 2704 at D = 600 with 7 slices.  (Vectors
 // of up to kClMax elements now go through one cluster, further down.)
-__global__ void __launch_bounds__(kRedThreads) update_dot_kernel(const double* __restrict__ part_in, double* c_out,
-                                                                const double* __restrict__ x0,
-                                                                const double* __restrict__ c1,
-                                                                const double* __restrict__ x1, double* y,
-                                                                const double* z, int64_t n,
-                                                                double* __restrict__ part_out) {
+__global__ void __launch_bounds__(kRedThreads) update_dot_kernel(const double* part_in, double* c_out, const double* x0_in,
+                                                                const double* c1_in, const double* x1_in, double* y,
+                                                                const double* z_in, int64_t n, double* part_out) {
   __shared__ double sh[kRedThreads];
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  const double *x0 = after_wait(x0_in, zero), *c1 = after_wait(c1_in, zero), *x1 = after_wait(x1_in, zero), *z = after_wait(z_in, zero);
+  part_in = after_wait(part_in, zero);
   if ((int64_t)blockIdx.x * kRedThreads >= n) {  // no element here
     if (threadIdx.x == 0) part_out[blockIdx.x] = 0.0;
     return;
@@ -426,10 +442,13 @@ __global__ void __launch_bounds__(kRedThreads) update_dot_kernel(const double* _
 
 // b = sqrt of the dot product whose partial sums are part_in, x *= 1 / b
 // (b_out null: not stored)
-__global__ void __launch_bounds__(kRedThreads) normalize_part_kernel(const double* __restrict__ part_in,
-                                                                    double* __restrict__ x, int64_t n,
+__global__ void __launch_bounds__(kRedThreads) normalize_part_kernel(const double* part_in, double* x_in, int64_t n,
                                                                     double* b_out) {
   __shared__ double sh[kRedThreads];
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  part_in = after_wait(part_in, zero);
+  double* x = after_wait(x_in, zero);
   if ((int64_t)blockIdx.x * kRedThreads >= n) return;
   const double b = sqrt(sum_partials(part_in, sh));
   const double f = 1.0 / b;
@@ -450,10 +469,13 @@ struct CombineCoefs {
   double z[kCombineMax];
 };
 __global__ void __launch_bounds__(kRedThreads) combine_vectors_kernel(CombineCoefs c, int m, bool first,
-                                                                     const double* __restrict__ f, int64_t stride_f,
-                                                                     double* __restrict__ v, int64_t n,
-                                                                     double* __restrict__ part) {
+                                                                     const double* f_in, int64_t stride_f, double* v_in,
+                                                                     int64_t n, double* part) {
   __shared__ double sh[kRedThreads];
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  const double* f = after_wait(f_in, zero);
+  double* v = after_wait(v_in, zero);
   double s = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double t = first ? __dmul_rn(c.z[0], f[i]) : fma(c.z[0], f[i], v[i]);
@@ -567,6 +589,10 @@ template <int E>
 __global__ void __launch_bounds__(kClThreads) lanczos_tail_cluster(int m, double* f, int64_t stride_f, int64_t n,
                                                                   double* alpha, double* beta, double* q) {
   __shared__ ClusterSum sh;
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  f = after_wait(f, zero);
+  beta = after_wait(beta, zero);
   const ClusterSlice<E> at(n);
   const bool first = blockIdx.x == 0 && threadIdx.x == 0;
   double y[E], x[E], next[E];
@@ -600,6 +626,9 @@ __global__ void __launch_bounds__(kClThreads) lanczos_tail_cluster(int m, double
 template <int E>
 __global__ void __launch_bounds__(kClThreads) unit_cluster(const double* x, double* out, int64_t n, double* b_out) {
   __shared__ ClusterSum sh;
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  x = after_wait(x, zero);
   const ClusterSlice<E> at(n);
   double y[E];
   at.load(x, y);
@@ -614,6 +643,10 @@ template <int E>
 __global__ void __launch_bounds__(kClThreads) dot_cluster(const double* x, const double* y, int64_t n, bool two,
                                                          double* out) {
   __shared__ ClusterSum sh;
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  x = after_wait(x, zero);
+  y = after_wait(y, zero);
   const ClusterSlice<E> at(n);
   double a[E], b[E];
   at.load(x, a);
@@ -631,6 +664,9 @@ template <int E>
 __global__ void __launch_bounds__(kClThreads) combine_unit_cluster(CombineCoefs c, int m, const double* f,
                                                                   int64_t stride_f, double* out, int64_t n) {
   __shared__ ClusterSum sh;
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  f = after_wait(f, zero);
   const ClusterSlice<E> at(n);
   double y[E], x[E];
   at.load(f, y);
@@ -689,9 +725,7 @@ bool cluster_runs() {
 
 template <class... P, class... A>
 cudaError_t launch_cluster(cudaStream_t stream, void (*kernel)(P...), A... args) {
-  cudaLaunchAttribute attr = {};
-  const cudaLaunchConfig_t cfg = cluster_config(&attr, stream);
-  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+  return launch_overlapped(kernel, dim3(kClCtas), kClThreads, 0, kClCtas, stream, args...);
 }
 
 // launch(E) with the elements a thread that a vector of n asks for
@@ -726,29 +760,26 @@ int lanczos_scratch_doubles() { return 2 * kRedBlocks + 2; }
 namespace {
 cudaError_t launch_dot_partial(const double* x, const double* y, int64_t n, double* scratch, int half,
                                cudaStream_t stream) {
-  dot_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch + half * kRedBlocks);
-  return cudaGetLastError();
+  return launch_overlapped(dot_partial, dim3(kRedBlocks), kRedThreads, 0, 0, stream, x, y, n, scratch + half * kRedBlocks);
 }
 
 cudaError_t dot_on_grid(const double* x, const double* y, int64_t n, double* scratch, double* out,
                         cudaStream_t stream) {
   cudaError_t e = launch_dot_partial(x, y, n, scratch, 0, stream);
   if (e != cudaSuccess) return e;
-  dot_final<<<1, kRedThreads, 0, stream>>>(scratch, out);
-  return cudaGetLastError();
+  return launch_overlapped(dot_final, dim3(1), kRedThreads, 0, 0, stream, scratch, out);
 }
 
 cudaError_t launch_update_dot(double* scratch, int half, double* c_out, const double* x0, const double* c1,
                               const double* x1, double* y, const double* z, int64_t n, cudaStream_t stream) {
-  update_dot_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(scratch + half * kRedBlocks, c_out, x0, c1, x1, y, z, n,
-                                                            scratch + (1 - half) * kRedBlocks);
-  return cudaGetLastError();
+  return launch_overlapped(update_dot_kernel, dim3(kRedBlocks), kRedThreads, 0, 0, stream, scratch + half * kRedBlocks,
+                           c_out, x0, c1, x1, y, z, n, scratch + (1 - half) * kRedBlocks);
 }
 
 cudaError_t launch_normalize_part(const double* scratch, int half, double* x, int64_t n, double* b_out,
                                   cudaStream_t stream) {
-  normalize_part_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(scratch + half * kRedBlocks, x, n, b_out);
-  return cudaGetLastError();
+  return launch_overlapped(normalize_part_kernel, dim3(kRedBlocks), kRedThreads, 0, 0, stream,
+                           scratch + half * kRedBlocks, x, n, b_out);
 }
 }  // namespace
 
@@ -782,14 +813,14 @@ cudaError_t launch_combine_vectors(const double* z, int m, const double* f, int6
       return launch_cluster(stream, combine_unit_cluster<E.value>, c, m, f, stride_f, v, n);
     });
   }
-  for (int j0 = 0; j0 < m; j0 += kCombineMax) {
+  cudaError_t e = cudaSuccess;
+  for (int j0 = 0; j0 < m && e == cudaSuccess; j0 += kCombineMax) {
     CombineCoefs c{};
     const int k = std::min(kCombineMax, m - j0);
     std::copy(z + j0, z + j0 + k, c.z);
-    combine_vectors_kernel<<<kRedBlocks, kRedThreads, 0, stream>>>(c, k, j0 == 0, f + j0 * stride_f, stride_f, v, n,
-                                                                  scratch);
+    e = launch_overlapped(combine_vectors_kernel, dim3(kRedBlocks), kRedThreads, 0, 0, stream, c, k, j0 == 0,
+                          f + j0 * stride_f, stride_f, v, n, scratch);
   }
-  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess && unit ? launch_normalize_part(scratch, 0, v, n, nullptr, stream) : e;
 }
 
@@ -798,9 +829,9 @@ cudaError_t launch_dot2(const double* x, const double* y, int64_t n, double* scr
     return by_elems(n, [&](auto E) {
       return launch_cluster(stream, dot_cluster<E.value>, x, y, n, true, scratch + 2 * kRedBlocks);
     });
-  dot2_partial<<<kRedBlocks, kRedThreads, 0, stream>>>(x, y, n, scratch);
-  dot_final<<<2, kRedThreads, 0, stream>>>(scratch, scratch + 2 * kRedBlocks);
-  return cudaGetLastError();
+  const cudaError_t e = launch_overlapped(dot2_partial, dim3(kRedBlocks), kRedThreads, 0, 0, stream, x, y, n, scratch);
+  if (e != cudaSuccess) return e;
+  return launch_overlapped(dot_final, dim3(2), kRedThreads, 0, 0, stream, scratch, scratch + 2 * kRedBlocks);
 }
 
 cudaError_t launch_lanczos_tail(int m, double* f, int64_t stride_f, int64_t n, double* alpha, double* beta, double* q,

@@ -43,6 +43,7 @@
 #include <mutex>
 
 #include "kernels.hpp"
+#include "overlap.cuh"
 #include "ozaki.hpp"
 
 namespace su2g {
@@ -256,9 +257,8 @@ struct Smem {
 template <int S>
 __global__ void __launch_bounds__(kThreads, 1) ozaki_gemm(const OzTile* __restrict__ tiles, int ntiles,
                                                           const OzSeg* __restrict__ segs,
-                                                          const uint8_t* __restrict__ packed,
-                                                          const int* __restrict__ exps, int* rowmax_out,
-                                                          Bases bases, int* err) {
+                                                          const uint8_t* packed_in, const int* exps_in,
+                                                          int* rowmax_out, Bases bases, int* err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   // accumulators full / empty, per half: [0] the low groups, [1] the high ones
@@ -299,6 +299,9 @@ __global__ void __launch_bounds__(kThreads, 1) ozaki_gemm(const OzTile* __restri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_sh;
+  const int64_t zero = wait_for_predecessor();
+  const uint8_t* const packed = after_wait(packed_in, zero);
+  const int* const exps = after_wait(exps_in, zero);
   volatile int* abort_v = &abort_sh;
   auto stage_a = [&](int st) { return smem_u32(smem) + (uint32_t)(st * Smem<S>::kStage); };
 
@@ -573,6 +576,7 @@ __global__ void __launch_bounds__(kThreads, 1) ozaki_gemm(const OzTile* __restri
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_bookf[n & 1]));
     }
+    dependents_may_start();  // this CTA is at its last tiles
   } else {
     // ============================ epilogue ============================
     // The drain warps share nothing but the accumulators and the tiles' books:
@@ -845,11 +849,8 @@ cudaError_t launch_ozaki_gemm(int S, const OzTile* tiles, int ntiles, const OzSe
   if (e != cudaSuccess) return e;
   const int grid = ntiles < g_sms ? ntiles : g_sms;
   const int smem = gemm_smem_bytes(S);
-  if (S == 6)
-    ozaki_gemm<6><<<grid, kThreads, smem, stream>>>(tiles, ntiles, segs, packed, exps, exps, bases, err);
-  else
-    ozaki_gemm<7><<<grid, kThreads, smem, stream>>>(tiles, ntiles, segs, packed, exps, exps, bases, err);
-  return cudaGetLastError();
+  return launch_overlapped(S == 6 ? ozaki_gemm<6> : ozaki_gemm<7>, dim3(grid), kThreads, smem, 0, stream, tiles, ntiles,
+                           segs, packed, exps, exps, bases, err);
 }
 
 }  // namespace oz

@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "kernels.hpp"
+#include "overlap.cuh"
 #include "ozaki.hpp"
 
 namespace su2g {
@@ -61,7 +62,10 @@ constexpr int kDigitKt = 2;        // k tiles (16 k each) per CTA of the digit k
 // |alpha X| 2^-e < 1/2 with e = ilogb(max |alpha X|) + 2, kExpZero for a zero row.
 __global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob* __restrict__ jobs,
                                                                  const int2* __restrict__ units, int nunits,
-                                                                 Bases bases, int* __restrict__ exps) {
+                                                                 Bases bases, int* exps, int* clear, int nclear) {
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
+  for (int i = blockIdx.x * kPackThreads + threadIdx.x; i < nclear; i += gridDim.x * kPackThreads) clear[i] = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t gw = (int64_t)blockIdx.x * (kPackThreads / 32) + warp;
   const int ui = (int)(gw / kRowsPerUnit), row = (int)(gw % kRowsPerUnit);
@@ -79,7 +83,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob* 
     return ((unsigned long long)hi << 32) | (unsigned)__double2loint(x);
   };
   if (r < job.R) {
-    const double* p = resolve(bases, job.src_buf, job.src) + (int64_t)r * job.ld_r;
+    const double* p = after_wait(resolve(bases, job.src_buf, job.src), zero) + (int64_t)r * job.ld_r;
     int k = lane;
     for (; k + 96 < job.K; k += 128) {  // four loads in flight
       const double a = p[(int64_t)k * job.ld_k], b = p[(int64_t)(k + 32) * job.ld_k];
@@ -164,17 +168,19 @@ __device__ __forceinline__ void store_digits(const uint32_t (&lo)[8], const uint
 template <int S>
 __global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const PackJob* __restrict__ jobs,
                                                                    const int2* __restrict__ units, Bases bases,
-                                                                   uint8_t* __restrict__ packed,
-                                                                   int* __restrict__ exps, int span) {
+                                                                   uint8_t* packed, int* exps_in, int span) {
   __shared__ int rexp[kTM];
   __shared__ int tmax;
   __shared__ __align__(16) double stage[kPackThreads / 32][8 * kPitch];  // a tile a warp
   const int2 u = units[blockIdx.x];
   const PackJob job = jobs[u.x];
   const int kt0 = blockIdx.y * kDigitKt * span;
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
   if (kt0 >= job.nkt) return;
+  int* const exps = after_wait(exps_in, zero);
   const int rt = u.y, RT = job.rt, r0 = rt * RT;
-  const double* src = resolve(bases, job.src_buf, job.src);
+  const double* src = after_wait(resolve(bases, job.src_buf, job.src), zero);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // a warp's tiles: the 8-row groups warp (and, for 128 rows, warp + 8) of every 32 k
   const int two = RT == kTM ? 1 : 0;
@@ -295,11 +301,13 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const Pack
 // (18 terms); spread out 8.2, 14.3 and 22.5 us.
 constexpr int kRedThreads = 256;
 __global__ void __launch_bounds__(kRedThreads) reduce_partials(const RedTile* __restrict__ reds, Bases bases) {
-  const RedTile& r = reds[blockIdx.x];
+  const RedTile r = reds[blockIdx.x];
+  dependents_may_start();
+  const int64_t zero = wait_for_predecessor();
   const int idx = blockIdx.y * kRedThreads + threadIdx.x;
   const int i = idx % kTM, j = idx / kTM;
   if (i >= r.mlen || j >= r.nlen) return;
-  const double* P = resolve(bases, kBufScratch, r.part) + idx;
+  const double* P = after_wait(resolve(bases, kBufScratch, r.part), zero) + idx;
   const int nparts = r.nparts;
   double s = 0.0;
   int p = 0;
@@ -318,17 +326,22 @@ __global__ void __launch_bounds__(kRedThreads) reduce_partials(const RedTile* __
 
 cudaError_t launch_reduce(const RedTile* reds, int n, const Bases& bases, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  reduce_partials<<<dim3(n, kTM * kTN / kRedThreads), kRedThreads, 0, stream>>>(reds, bases);
-  return cudaGetLastError();
+  return launch_overlapped(reduce_partials, dim3(n, kTM * kTN / kRedThreads), kRedThreads, 0, 0, stream, reds, bases);
 }
 
 cudaError_t launch_pack(int S, const PackJob* jobs, const int2* units, int nunits, int max_nkt, bool rows_pass,
-                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream) {
+                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream, int* clear, int nclear) {
+  if (nclear > 0 && !(nunits > 0 && rows_pass)) {  // no row pass to do it
+    const cudaError_t e = cudaMemsetAsync(clear, 0, nclear * sizeof(int), stream);
+    if (e != cudaSuccess) return e;
+  }
   if (nunits <= 0) return cudaSuccess;
   if (rows_pass) {
     const int64_t warps = (int64_t)nunits * kRowsPerUnit;
     const int rows_blocks = (int)((warps + kPackThreads / 32 - 1) / (kPackThreads / 32));
-    pack_rows_kernel<<<rows_blocks, kPackThreads, 0, stream>>>(jobs, units, nunits, bases, exps);
+    const cudaError_t e = launch_overlapped(pack_rows_kernel, dim3(rows_blocks), kPackThreads, 0, 0, stream, jobs,
+                                            units, nunits, bases, exps, clear, nclear);
+    if (e != cudaSuccess) return e;
   }
   // CTAs of several chunks (exponents read once, tiles fetched ahead) once
   // there are enough to fill the SMs' slots twice over: 321 us at D = 2000
@@ -337,11 +350,14 @@ cudaError_t launch_pack(int S, const PackJob* jobs, const int2* units, int nunit
   const int span = (int)std::min<int64_t>(std::max<int64_t>((int64_t)nunits * chunks / (8 * kF64Sms), 1), 8);
   const dim3 grid(nunits, (chunks + span - 1) / span);
   switch (S) {
-    case 6: pack_digits_kernel<6><<<grid, kPackThreads, 0, stream>>>(jobs, units, bases, packed, exps, span); break;
-    case 7: pack_digits_kernel<7><<<grid, kPackThreads, 0, stream>>>(jobs, units, bases, packed, exps, span); break;
-    default: return cudaErrorInvalidValue;
+    case 6:
+      return launch_overlapped(pack_digits_kernel<6>, grid, kPackThreads, 0, 0, stream, jobs, units, bases, packed,
+                               exps, span);
+    case 7:
+      return launch_overlapped(pack_digits_kernel<7>, grid, kPackThreads, 0, 0, stream, jobs, units, bases, packed,
+                               exps, span);
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace oz
