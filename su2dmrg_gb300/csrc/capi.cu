@@ -63,19 +63,13 @@ struct Staging {
   void add(const std::vector<T>& v, T** slot) {
     add_bytes(v.data(), v.size() * sizeof(T), (void**)slot);
   }
-  // with `caller`, the copy is queued on that stream (pageable source: it is
-  // staged before the call returns); else on the thread's own stream, waited for
-  cudaError_t send(void** base, const cudaStream_t* caller) {
+  // allocation and copy in st's order (pageable source: it is staged before
+  // the call returns)
+  cudaError_t send(void** base, cudaStream_t st) {
     *base = nullptr;
     if (host.empty()) return cudaSuccess;
-    cudaError_t e = su2g::dev_alloc(base, host.size());
-    cudaStream_t st = nullptr;
-    if (e == cudaSuccess) {
-      if (caller) st = *caller;
-      else e = su2g::setup_stream(&st);
-    }
+    cudaError_t e = su2g::stream_alloc(base, host.size(), st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(*base, host.data(), host.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && !caller) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
     for (auto& sl : slots) *sl.first = static_cast<uint8_t*>(*base) + sl.second;
     return cudaSuccess;
@@ -104,25 +98,15 @@ su2g::Bases make_bases(const su2g_heff_plan* p, const double* psi, double* y) {
 }
 
 // device buffers of the split-precision work, and the one-time packing of
-// the operators (they stay fixed for the lifetime of the plan).  The pack
-// reads the caller's operator data: with `caller` given (the one-shot work
-// lists, whose operands may still be in flight on the caller's stream, such
-// as transposes queued just before) it runs on that stream, ordered after
-// them; without (su2g_heff_plan_create, whose operands must be complete) on
-// the thread's own stream, waited for.
-cudaError_t setup_split(su2g_heff_plan* p, const cudaStream_t* caller) {
+// the operators (they stay fixed for the lifetime of the plan), in st's order.
+cudaError_t setup_split(su2g_heff_plan* p, cudaStream_t st) {
   su2g::oz::OzWork& w = p->oz;
-  cudaError_t e = dalloc(&p->d_packed, std::max<int64_t>(w.packed_bytes, 16));
-  if (e == cudaSuccess) e = dalloc(&p->d_exps, std::max<int64_t>(w.exp_len, 1) * sizeof(int));
+  cudaError_t e = su2g::stream_alloc((void**)&p->d_packed, std::max<int64_t>(w.packed_bytes, 16), st);
+  if (e == cudaSuccess) e = su2g::stream_alloc((void**)&p->d_exps, std::max<int64_t>(w.exp_len, 1) * sizeof(int), st);
   if (e != cudaSuccess) return e;
   const su2g::Bases b = make_bases(p, nullptr, nullptr);
-  cudaStream_t st = nullptr;
-  if (caller) st = *caller;
-  else e = su2g::setup_stream(&st);
-  if (e == cudaSuccess)
-    e = su2g::oz::launch_pack(p->S, p->d_jobs[0], p->d_units[0], (int)w.units[0].size(), w.max_nkt[0],
-                              w.rows_pass[0], b, p->d_packed, p->d_exps, st);
-  if (e == cudaSuccess && !caller) e = cudaStreamSynchronize(st);
+  e = su2g::oz::launch_pack(p->S, p->d_jobs[0], p->d_units[0], (int)w.units[0].size(), w.max_nkt[0],
+                            w.rows_pass[0], b, p->d_packed, p->d_exps, st);
   // the GEMM's one-time setup happens here, never inside a graph capture
   if (e == cudaSuccess) e = su2g::oz::prepare_ozaki_gemm(p->S);
   return e;
@@ -207,7 +191,12 @@ int su2g_fac_operator_transformation(int side, int j, int m, int l, int i, int k
 
 namespace {
 // device side of a plan whose host work lists are built: work lists, scratch
-// (intermediates + split partial tiles) and, in split mode, the packed operands
+// (intermediates + split partial tiles) and, in split mode, the packed
+// operands.  The pack reads the caller's operator data: with `caller` given (the
+// one-shot work lists, whose operands may still be in flight on the caller's
+// stream, such as transposes queued just before) everything is queued on that
+// stream; without (su2g_heff_plan_create, whose operands must be complete) on
+// the thread's own stream, waited for once, at the end.
 int plan_from_work(su2g::HeffWork&& work, int mode, su2g_heff_plan** plan, const cudaStream_t* caller = nullptr) {
   *plan = nullptr;
   const int S = slices_of_mode(mode);
@@ -254,11 +243,19 @@ int plan_from_work(su2g::HeffWork&& work, int mode, su2g_heff_plan** plan, const
     stage.add(w.tile2, &p->d_otile2);
     stage.add(w.red2, &p->d_red2);
   }
-  cudaError_t e = stage.send(&p->d_lists, caller);
+  cudaStream_t st = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (caller) p->last_st = st = *caller;
+  else e = su2g::setup_stream(&st);
+  if (e == cudaSuccess) e = stage.send(&p->d_lists, st);
   const int64_t scratch_doubles = p->work.scratch_len + p->oz.partial_len;
-  if (e == cudaSuccess && scratch_doubles > 0) e = dalloc(&p->d_scratch, scratch_doubles * sizeof(double));
-  if (e == cudaSuccess && S > 0) e = setup_split(p, caller);
-  if (caller) p->last_st = *caller;
+  if (e == cudaSuccess && scratch_doubles > 0)
+    e = su2g::stream_alloc((void**)&p->d_scratch, scratch_doubles * sizeof(double), st);
+  if (e == cudaSuccess && S > 0) e = setup_split(p, st);
+  if (!caller) {
+    const cudaError_t done = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = done;
+  }
   if (e != cudaSuccess) {
     p->release();
     delete p;
@@ -282,11 +279,10 @@ int su2g::run_work_once(HeffWork&& w, int mode, void* stream) {
   int rc = plan_from_work(std::move(w), mode, &p, &st);
   if (rc) return rc;
   rc = su2g_heff_apply(p, nullptr, nullptr, stream);
-  cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
   int code = 0;
-  if (!rc && e == cudaSuccess) rc = su2g_heff_plan_status(p, &code);
+  if (!rc) rc = su2g_heff_plan_status(p, &code);  // waits
+  else cudaStreamSynchronize(st);
   su2g_heff_plan_destroy(p);
-  if (e != cudaSuccess) return cuda_fail(e, "work list");
   return rc;
 }
 
@@ -625,10 +621,13 @@ int su2g_heff_plan_status(su2g_heff_plan* p, int* code) {
   if (!p || !code) return fail(SU2G_EINVAL, "plan_status: bad arguments");
   *code = 0;
   if (!p->d_err) return SU2G_OK;
-  // read after the plan's latest work, on its stream
-  SU2G_CUDA(cudaMemcpyAsync(code, p->d_err, sizeof(int), cudaMemcpyDeviceToHost, p->last_st));
-  SU2G_CUDA(cudaMemsetAsync(p->d_err, 0, sizeof(int), p->last_st));
+  // read after the plan's latest work, on its stream; no FP64 kernel sets it
+  if (p->S > 0 || p->marked) SU2G_CUDA(cudaMemcpyAsync(code, p->d_err, sizeof(int), cudaMemcpyDeviceToHost, p->last_st));
   SU2G_CUDA(cudaStreamSynchronize(p->last_st));
+  if (*code) {
+    SU2G_CUDA(cudaMemsetAsync(p->d_err, 0, sizeof(int), p->last_st));
+    SU2G_CUDA(cudaStreamSynchronize(p->last_st));
+  }
   if (*code) return fail(SU2G_ETIMEOUT, "a bounded device wait gave up (code " + std::to_string(*code) + ")");
   return SU2G_OK;
 }
@@ -711,6 +710,7 @@ int su2g_f64_tile_bench(int M, int N, int K, int nblocks, int cls, int reps, dou
 
 int su2g_heff_plan_mark_failed(su2g_heff_plan* p, int code) {
   if (!p || !p->d_err || code == 0) return fail(SU2G_EINVAL, "plan_mark_failed: bad arguments");
+  p->marked = true;
   SU2G_CUDA(cudaMemcpyAsync(p->d_err, &code, sizeof(int), cudaMemcpyHostToDevice, p->last_st));
   SU2G_CUDA(cudaStreamSynchronize(p->last_st));
   return SU2G_OK;
@@ -1061,8 +1061,6 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
     }
     *energy = eig[0];
     if (nmatvec) *nmatvec = L.nmatvec;
-    cudaError_t e = cudaStreamSynchronize(L.st);
-    if (e != cudaSuccess) return cuda_fail(e, "lanczos");
     // a bounded wait of the split GEMM that gave up leaves partial products:
     // the result is refused, not returned
     int code = 0;
@@ -1109,9 +1107,8 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
       if (std::fabs(ov - 1.) < 1.e-8) {  // lanczos_su2.cpp:178-188
         *energy = eig[0];
         if (nmatvec) *nmatvec = L.nmatvec;
-        SU2G_CUDA(cudaStreamSynchronize(L.st));
         int code = 0;
-        return su2g_heff_plan_status(p, &code);
+        return su2g_heff_plan_status(p, &code);  // waits
       }
     }
   }

@@ -35,6 +35,7 @@ struct su2g_heff_plan {
   su2g::oz::OzTile* d_otile2 = nullptr;
   su2g::oz::RedTile* d_red2 = nullptr;
   int* d_err = nullptr;
+  bool marked = false;  // the error word was set from the host (su2g_heff_plan_mark_failed)
   void* d_lists = nullptr;  // one device block holding every work list above and d_err
   // Lanczos workspace (allocated on first use)
   double* d_krylov = nullptr;
