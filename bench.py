@@ -399,17 +399,17 @@ def run_su2g(args):
         t_kernel = (prof[1] + prof[3]) / 1e3
         achieved = pairs * flops / t_kernel / 1e12
         # DRAM bytes of the two GEMM launches, measured with ncu (dram__bytes_read.sum +
-        # dram__bytes_write.sum) on this D=2000 width-20 workload: 1.828e9 (phase 1) +
-        # 2.970e9 (phase 2) = 3.74 bytes per algorithmic byte of an application (FP64
+        # dram__bytes_write.sum) on this D=2000 width-20 workload: 1.825e9 (phase 1) +
+        # 3.035e9 (phase 2) = 3.79 bytes per algorithmic byte of an application (FP64
         # operators + psi in/out); other sizes are scaled by their algorithmic bytes.
         alg_bytes = 8.0 * (sum(x.numel() for (_s1, x1, _s2, x2, _c) in terms for x in (x1, x2))
                            + sum(h[1].numel() for h in (hl, hr) if h is not None) + 2 * w.psi.size())
         captured = args.D == 2000 and args.nspin1 == 18 and S == 7
-        traffic = 3.737 * alg_bytes / 2 if captured else None
+        traffic = 3.786 * alg_bytes / 2 if captured else None
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": traffic,
-                "traffic_definition": "DRAM bytes per GEMM launch: ncu-measured 3.737 x algorithmic bytes per "
-                                      "application (D=2000 width-20 capture: 1.828e9 + 2.970e9 B over the two "
+                "traffic_definition": "DRAM bytes per GEMM launch: ncu-measured 3.786 x algorithmic bytes per "
+                                      "application (D=2000 width-20 capture: 1.825e9 + 3.035e9 B over the two "
                                       f"launches), this workload's algorithmic bytes {alg_bytes:.4g} B, halved "
                                       "over the two launches; the digit-pack launches are not included; "
                                       "null when the workload is not the captured one",
