@@ -599,7 +599,7 @@ int su2g_heff_plan_launches(const su2g_heff_plan* p, int* n) {
   } else {
     const su2g::oz::OzWork& w = p->oz;
     for (int k = 1; k <= 2; ++k)
-      if (!w.units[k].empty()) c += w.rows_pass[k] ? 2 : 1;
+      if (!w.units[k].empty()) c += su2g::oz::pack_launches(w.rows_pass[k], k == 1, w.max_nkt[k]);
     c += w.tile1.empty() ? 0 : 1;
     c += w.tile2.empty() ? 0 : 1;
     c += w.red2.empty() ? 0 : 1;
@@ -782,7 +782,7 @@ int su2g::heff_apply_impl(su2g_heff_plan* p, const double* psi, double* y, cudaS
   const su2g::oz::OzWork& w = p->oz;
   // the row maxima that phase 1 leaves for the intermediates' pack start at zero
   SU2G_CUDA(su2g::oz::launch_pack(p->S, p->d_jobs[1], p->d_units[1], (int)w.units[1].size(), w.max_nkt[1], w.rows_pass[1], b, p->d_packed,
-                                  p->d_exps, st, p->d_exps + w.rowmax_base, (int)w.rowmax_len));
+                                  p->d_exps, st, true, p->d_exps + w.rowmax_base, (int)w.rowmax_len));
   SU2G_CUDA(su2g::oz::launch_ozaki_gemm(p->S, p->d_otile1, (int)w.tile1.size(), p->d_oseg1, p->d_packed, p->d_exps, b,
                                         p->d_err, st));
   SU2G_CUDA(su2g::oz::launch_pack(p->S, p->d_jobs[2], p->d_units[2], (int)w.units[2].size(), w.max_nkt[2], w.rows_pass[2], b, p->d_packed,
@@ -825,7 +825,7 @@ int su2g_heff_apply_profile(su2g_heff_plan* p, const double* psi, double* y, voi
     const su2g::oz::OzWork& w = p->oz;
     if (e == cudaSuccess)
       e = su2g::oz::launch_pack(p->S, p->d_jobs[1], p->d_units[1], (int)w.units[1].size(), w.max_nkt[1], w.rows_pass[1], b, p->d_packed, p->d_exps,
-                                st, p->d_exps + w.rowmax_base, (int)w.rowmax_len);
+                                st, true, p->d_exps + w.rowmax_base, (int)w.rowmax_len);
     if (e == cudaSuccess) e = cudaEventRecord(ev[1], st);
     if (e == cudaSuccess)
       e = su2g::oz::launch_ozaki_gemm(p->S, p->d_otile1, (int)w.tile1.size(), p->d_oseg1, p->d_packed, p->d_exps, b,

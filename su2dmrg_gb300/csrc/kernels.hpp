@@ -90,11 +90,14 @@ cudaError_t bounded_wait_selftest(long long limit, int* timed_out_host, cudaStre
 // CTAs of the persistent GEMM grid on the current device (its SM count); 152
 // when no device answers (host-only planning and validation).
 int ozaki_persistent_grid();
+// kernels of a launch_pack of some units
+int pack_launches(bool rows_pass, bool unit_alpha, int max_nkt);
 // row-exponent pass (when rows_pass) + digit pass: 1 or 2 kernels, none for nunits == 0;
-// before them clear[0, nclear) = 0 (part of the row pass where there is one)
+// unit_alpha: every job's scale is 1 or -1 and none has row maxima; clear[0,
+// nclear) = 0 in the first of them
 cudaError_t launch_pack(int S, const PackJob* jobs, const int2* units, int nunits, int max_nkt, bool rows_pass,
-                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream, int* clear = nullptr,
-                        int nclear = 0);
+                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream, bool unit_alpha = false,
+                        int* clear = nullptr, int nclear = 0);
 cudaError_t launch_ozaki_gemm(int S, const OzTile* tiles, int ntiles, const OzSeg* segs, const uint8_t* packed,
                               int* exps, const Bases& bases, int* err, cudaStream_t stream);
 int gemm_smem_bytes(int S);

@@ -55,8 +55,17 @@ constexpr long long kDigitBias = S == 0 ? 0 : 64ll + 128ll * kDigitBias<(S > 0 ?
 template <>
 constexpr long long kDigitBias<0> = 0;
 
+// |x| as a bit pattern.  The sign comes off the high word alone: masking the 64
+// bits compiles to an FP64 |x|, sixteen clocks a warp.
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  unsigned hi;
+  asm("and.b32 %0, %1, 0x7FFFFFFF;" : "=r"(hi) : "r"(__double2hiint(x)));
+  return ((unsigned long long)hi << 32) | (unsigned)__double2loint(x);
+}
+
 constexpr int kRowsPerUnit = kTM;  // row slots per unit in the row kernel (RT <= 128)
 constexpr int kDigitKt = 2;        // k tiles (16 k each) per CTA of the digit kernel
+constexpr int kOwnRowsKt = 4;      // up to this many, it finds the row exponents itself (launch_pack)
 
 // Row exponents: one warp per row of every unit, lanes along k (coalesced):
 // |alpha X| 2^-e < 1/2 with e = ilogb(max |alpha X|) + 2, kExpZero for a zero row.
@@ -75,13 +84,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_rows_kernel(const PackJob* 
   if (row >= job.rt || job.rowmax >= 0) return;  // row maxima left by the producing GEMM
   const int r = u.y * job.rt + row;
   unsigned long long m = 0;  // max |x| as a bit pattern (order-preserving for |x|)
-  // the sign comes off the high word alone: masking the 64 bits compiles to an
-  // FP64 |x|, sixteen clocks a warp
-  auto bits = [](double x) {
-    unsigned hi;
-    asm("and.b32 %0, %1, 0x7FFFFFFF;" : "=r"(hi) : "r"(__double2hiint(x)));
-    return ((unsigned long long)hi << 32) | (unsigned)__double2loint(x);
-  };
+  auto bits = [](double x) { return abs_bits(x); };
   if (r < job.R) {
     const double* p = after_wait(resolve(bases, job.src_buf, job.src), zero) + (int64_t)r * job.ld_r;
     int k = lane;
@@ -165,18 +168,26 @@ __device__ __forceinline__ void store_digits(const uint32_t (&lo)[8], const uint
   }
 }
 
-template <int S>
+// OwnRows: the row exponents are found here, by every CTA for all k of its rows,
+// instead of by pack_rows_kernel before (no row maxima left by a GEMM then).
+template <int S, bool OwnRows>
 __global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const PackJob* __restrict__ jobs,
                                                                    const int2* __restrict__ units, Bases bases,
-                                                                   uint8_t* packed, int* exps_in, int span) {
+                                                                   uint8_t* packed, int* exps_in, int span, int* clear,
+                                                                   int nclear) {
   __shared__ int rexp[kTM];
   __shared__ int tmax;
+  __shared__ unsigned long long rmax[OwnRows ? kTM : 1];
   __shared__ __align__(16) double stage[kPackThreads / 32][8 * kPitch];  // a tile a warp
   const int2 u = units[blockIdx.x];
   const PackJob job = jobs[u.x];
   const int kt0 = blockIdx.y * kDigitKt * span;
   dependents_may_start();
   const int64_t zero = wait_for_predecessor();
+  if constexpr (OwnRows)
+    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * kPackThreads + threadIdx.x; i < nclear;
+         i += gridDim.x * gridDim.y * kPackThreads)
+      clear[i] = 0;
   if (kt0 >= job.nkt) return;
   int* const exps = after_wait(exps_in, zero);
   const int rt = u.y, RT = job.rt, r0 = rt * RT;
@@ -206,10 +217,45 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const Pack
   };
   if (ntiles > 0) fetch(0);
   if (tid == 0) tmax = kExpZero;
+  if constexpr (OwnRows) {  // the unit's row maxima, over all k
+    if (tid < kTM) rmax[tid] = 0;
+    __syncthreads();
+    if (rows) {  // a warp a row, four rows at a time
+      for (int q = warp; q < RT; q += 4 * (kPackThreads / 32)) {
+        unsigned long long m[4] = {0, 0, 0, 0};
+        for (int k = lane; k < job.K; k += 32) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int r = r0 + q + j * (kPackThreads / 32);
+            if (r < job.R) m[j] = max(m[j], abs_bits(__ldg(src + (int64_t)r * job.ld_r + k)));
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) m[j] = max(m[j], __shfl_xor_sync(0xffffffffu, m[j], o));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (lane == 0 && q + j * (kPackThreads / 32) < RT) rmax[q + j * (kPackThreads / 32)] = m[j];
+      }
+    } else {  // a lane a row, the warps share the k
+      const int groups = RT / 32, r = (warp % groups) * 32 + lane, step_k = (kPackThreads / 32) / groups;
+      unsigned long long m = 0;
+      if (r0 + r < job.R) {
+#pragma unroll 4
+        for (int k = warp / groups; k < job.K; k += step_k)
+          m = max(m, abs_bits(__ldg(src + (int64_t)(r0 + r) * job.ld_r + (int64_t)k * job.ld_k)));
+        atomicMax(&rmax[r], m);
+      }
+    }
+  }
   __syncthreads();
   if (tid < RT) {
     int e;
-    if (job.rowmax >= 0) {  // |X| 2^-e < 1/2 from the producer's ilogb maxima
+    if constexpr (OwnRows) {
+      e = rmax[tid] ? ilogb_bits(rmax[tid]) + 2 : kExpZero;
+      if (blockIdx.y == 0) exps[job.exp + r0 + tid] = e;
+    } else if (job.rowmax >= 0) {  // |X| 2^-e < 1/2 from the producer's ilogb maxima
       const int v = (r0 + tid < job.R) ? exps[job.rowmax + r0 + tid] : 0;
       e = v > 0 ? v - kRowmaxBias + 2 : kExpZero;
       if (blockIdx.y == 0) exps[job.exp + r0 + tid] = e;
@@ -329,19 +375,32 @@ cudaError_t launch_reduce(const RedTile* reds, int n, const Bases& bases, cudaSt
   return launch_overlapped(reduce_partials, dim3(n, kTM * kTN / kRedThreads), kRedThreads, 0, 0, stream, reds, bases);
 }
 
+int pack_launches(bool rows_pass, bool unit_alpha, int max_nkt) {
+  return rows_pass && !(unit_alpha && max_nkt <= kOwnRowsKt) ? 2 : 1;
+}
+
 cudaError_t launch_pack(int S, const PackJob* jobs, const int2* units, int nunits, int max_nkt, bool rows_pass,
-                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream, int* clear, int nclear) {
-  if (nclear > 0 && !(nunits > 0 && rows_pass)) {  // no row pass to do it
+                        const Bases& bases, uint8_t* packed, int* exps, cudaStream_t stream, bool unit_alpha, int* clear,
+                        int nclear) {
+  if (nclear > 0 && !(nunits > 0 && rows_pass)) {  // no kernel that does it
     const cudaError_t e = cudaMemsetAsync(clear, 0, nclear * sizeof(int), stream);
     if (e != cudaSuccess) return e;
+    nclear = 0;
   }
   if (nunits <= 0) return cudaSuccess;
-  if (rows_pass) {
+  // Operands of a scale +-1 without row maxima (psi) and of up to 64 k: the digit
+  // kernel finds the exponents itself, one launch less (an application at D =
+  // 100: 34.7 -> 31.3 us, at D = 200: 47.4 -> 45.5).  From 65 k on its CTAs, one for each
+  // 32 k of a row tile, read the rows too often: D = 400, K <= 108, 100 -> 105 us;
+  // D = 777, K <= 210, 239 -> 254.
+  const bool own_rows = rows_pass && pack_launches(rows_pass, unit_alpha, max_nkt) == 1;
+  if (rows_pass && !own_rows) {
     const int64_t warps = (int64_t)nunits * kRowsPerUnit;
     const int rows_blocks = (int)((warps + kPackThreads / 32 - 1) / (kPackThreads / 32));
     const cudaError_t e = launch_overlapped(pack_rows_kernel, dim3(rows_blocks), kPackThreads, 0, 0, stream, jobs,
                                             units, nunits, bases, exps, clear, nclear);
     if (e != cudaSuccess) return e;
+    nclear = 0;
   }
   // CTAs of several chunks (exponents read once, tiles fetched ahead) once
   // there are enough to fill the SMs' slots twice over: 321 us at D = 2000
@@ -349,14 +408,12 @@ cudaError_t launch_pack(int S, const PackJob* jobs, const int2* units, int nunit
   const int chunks = (max_nkt + kDigitKt - 1) / kDigitKt;
   const int span = (int)std::min<int64_t>(std::max<int64_t>((int64_t)nunits * chunks / (8 * kF64Sms), 1), 8);
   const dim3 grid(nunits, (chunks + span - 1) / span);
-  switch (S) {
-    case 6:
-      return launch_overlapped(pack_digits_kernel<6>, grid, kPackThreads, 0, 0, stream, jobs, units, bases, packed,
-                               exps, span);
-    case 7:
-      return launch_overlapped(pack_digits_kernel<7>, grid, kPackThreads, 0, 0, stream, jobs, units, bases, packed,
-                               exps, span);
-  }
+  auto digits = [&](auto kernel) {
+    return launch_overlapped(kernel, grid, kPackThreads, 0, 0, stream, jobs, units, bases, packed, exps, span, clear,
+                             nclear);
+  };
+  if (S == 6) return own_rows ? digits(pack_digits_kernel<6, true>) : digits(pack_digits_kernel<6, false>);
+  if (S == 7) return own_rows ? digits(pack_digits_kernel<7, true>) : digits(pack_digits_kernel<7, false>);
   return cudaErrorInvalidValue;
 }
 
