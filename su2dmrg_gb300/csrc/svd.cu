@@ -534,7 +534,7 @@ struct EighJob {
 // for one alone).  The first pass keeps a stream and a host thread for each of
 // eight sectors at a time, largest first (a truncation at D = 400, 14 sectors of
 // up to 108 rows: 9.1 ms; 11.1 with all 14 at once, whose threads wait for one
-// another in the driver, 10.6 with six; D = 2000: 95, 97 and 101).  A batch
+// another in CUDA's launch path, 10.6 with six; D = 2000: 95, 97 and 101).  A batch
 // would be faster (6.8), but the Gram matrix is known to its rounding only, so the
 // directions of its smallest eigenvalues are whatever the solver makes of that,
 // and a padded matrix gives other ones: the new tensors move by 7e-10, without
@@ -585,7 +585,7 @@ struct Sector {
 // The sectors of a truncation in lockstep: every step (a product, a
 // correction, a copy) is one launch for all of them, and the host reads all
 // their eigenvalues back at once.  With a stream and a host thread for each
-// sector, ten launches a level and sector fought for the driver: nine levels of
+// sector, ten launches a level and sector fought for CUDA's launch path: nine levels of
 // 14 sectors took 5 ms, in lockstep 2.6, half of it the last levels' solver.
 class Truncation {
  public:
