@@ -552,6 +552,14 @@ struct ClusterSlice {
   }
 };
 
+// A CTA's shared memory may be written from another one only once it runs:
+// every kernel of a cluster arrives here first of all and waits before its first
+// cluster_sum, behind the wait for the predecessor and the first loads.
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
 // The sum of every thread's v over the cluster, in every thread; turn: 0, 1, 0,
 // ...  An FP64 addition keeps the SM's pipe busy for 32 clocks whatever its
 // lanes hold, so one warp does them all, twelve in a row: with a butterfly in
@@ -572,6 +580,7 @@ __device__ __forceinline__ double cluster_sum(double v, ClusterSum& sh, int turn
           : "r"((uint32_t)__cvta_generic_to_shared(&sh.cta[turn][blockIdx.x])), "r"(lane));
       asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(v) : "memory");
     }
+    __syncwarp();  // the barrier is a whole warp's
   }
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (threadIdx.x < 32) {
@@ -589,6 +598,7 @@ template <int E>
 __global__ void __launch_bounds__(kClThreads) lanczos_tail_cluster(int m, double* f, int64_t stride_f, int64_t n,
                                                                   double* alpha, double* beta, double* q) {
   __shared__ ClusterSum sh;
+  cluster_arrive();
   dependents_may_start();
   const int64_t zero = wait_for_predecessor();
   f = after_wait(f, zero);
@@ -599,6 +609,7 @@ __global__ void __launch_bounds__(kClThreads) lanczos_tail_cluster(int m, double
   at.load(f + m * stride_f, y);
   at.load(f + (m - 1) * stride_f, x);
   if (m >= 2) at.load(f + (m - 2) * stride_f, next);
+  cluster_wait();
   int turn = 0;
   double c = cluster_sum(at.dot(x, y), sh, turn);
   if (first) alpha[m - 1] = c;
@@ -626,12 +637,14 @@ __global__ void __launch_bounds__(kClThreads) lanczos_tail_cluster(int m, double
 template <int E>
 __global__ void __launch_bounds__(kClThreads) unit_cluster(const double* x, double* out, int64_t n, double* b_out) {
   __shared__ ClusterSum sh;
+  cluster_arrive();
   dependents_may_start();
   const int64_t zero = wait_for_predecessor();
   x = after_wait(x, zero);
   const ClusterSlice<E> at(n);
   double y[E];
   at.load(x, y);
+  cluster_wait();
   const double b = sqrt(cluster_sum(at.dot(y, y), sh, 0)), s = 1.0 / b;
   if (b_out && blockIdx.x == 0 && threadIdx.x == 0) *b_out = b;
   at.scale(s, y);
@@ -643,6 +656,7 @@ template <int E>
 __global__ void __launch_bounds__(kClThreads) dot_cluster(const double* x, const double* y, int64_t n, bool two,
                                                          double* out) {
   __shared__ ClusterSum sh;
+  cluster_arrive();
   dependents_may_start();
   const int64_t zero = wait_for_predecessor();
   x = after_wait(x, zero);
@@ -651,6 +665,7 @@ __global__ void __launch_bounds__(kClThreads) dot_cluster(const double* x, const
   double a[E], b[E];
   at.load(x, a);
   at.load(y, b);
+  cluster_wait();
   const double v = cluster_sum(at.dot(a, b), sh, 0);
   const double w = two ? cluster_sum(at.dot(a, a), sh, 1) : 0.0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -664,6 +679,7 @@ template <int E>
 __global__ void __launch_bounds__(kClThreads) combine_unit_cluster(CombineCoefs c, int m, const double* f,
                                                                   int64_t stride_f, double* out, int64_t n) {
   __shared__ ClusterSum sh;
+  cluster_arrive();
   dependents_may_start();
   const int64_t zero = wait_for_predecessor();
   f = after_wait(f, zero);
@@ -675,6 +691,7 @@ __global__ void __launch_bounds__(kClThreads) combine_unit_cluster(CombineCoefs 
     at.load(f + j * stride_f, x);
     at.axpy(c.z[j], x, y);
   }
+  cluster_wait();
   const double s = 1.0 / sqrt(cluster_sum(at.dot(y, y), sh, 0));
   at.scale(s, y);
   at.store(out, y);
