@@ -62,9 +62,9 @@ __device__ __forceinline__ void seg_mma(const GemmSeg& g, const Bases& bases, in
     double a[U], b[U][FN];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      a[u] = __ldg(ap + 4 * u * ks);
+      a[u] = ap[4 * u * ks];
 #pragma unroll
-      for (int j = 0; j < FN; ++j) b[u][j] = j < nj ? __ldg(bp[j] + 4 * u) : 0.0;
+      for (int j = 0; j < FN; ++j) b[u][j] = j < nj ? bp[j][4 * u] : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -77,10 +77,10 @@ __device__ __forceinline__ void seg_mma(const GemmSeg& g, const Bases& bases, in
   }
   for (; step < step1; ++step) {  // the last steps one by one, the very last perhaps past K
     const bool ok = step * 4 + fc < g.K;
-    const double a = ok ? __ldg(ap) : 0.0;
+    const double a = ok ? *ap : 0.0;
 #pragma unroll
     for (int j = 0; j < FN; ++j) {
-      const double b = (ok && j < nj) ? __ldg(bp[j]) : 0.0;
+      const double b = (ok && j < nj) ? *bp[j] : 0.0;
       if (j < nj) dmma_m8n8k4(sacc[j], a, b);
       bp[j] += 4;
     }

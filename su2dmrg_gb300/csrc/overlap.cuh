@@ -8,8 +8,10 @@
 // Every CTA calls wait_for_predecessor() before it ends, so that a kernel's
 // completion implies that of all before it.  The wait returns a zero the
 // compiler does not know, and pointers to data that kernels write get it added
-// (after_wait): their loads, also ones taken for invariant, cannot then be
-// moved above the wait.
+// (after_wait): their loads cannot then be moved above the wait.  Such data is
+// read with plain loads only: a read-only one (__ldg) asks that nothing writes
+// the data while the reading grid exists, and this grid exists while its
+// predecessor still writes.
 //
 // What it saves is the gap between kernels, launch latency and prologue: an
 // application at D = 40 (two FP64 launches) takes 9 us instead of 14, at D =

@@ -208,11 +208,11 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const Pack
     const double* p = src + (int64_t)(r + tr) * job.ld_r + (int64_t)(k + tk) * job.ld_k;
     if (r + 8 <= job.R && k + kDigitKt * kKS <= job.K) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j, p += step) next[j] = __ldg(p);
+      for (int j = 0; j < 8; ++j, p += step) next[j] = *p;
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j, p += step)
-        next[j] = (r + tr + j * dr < job.R && k + tk + j * dk < job.K) ? __ldg(p) : 0.0;
+        next[j] = (r + tr + j * dr < job.R && k + tk + j * dk < job.K) ? *p : 0.0;
     }
   };
   if (ntiles > 0) fetch(0);
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const Pack
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int r = r0 + q + j * (kPackThreads / 32);
-            if (r < job.R) m[j] = max(m[j], abs_bits(__ldg(src + (int64_t)r * job.ld_r + k)));
+            if (r < job.R) m[j] = max(m[j], abs_bits(src[(int64_t)r * job.ld_r + k]));
           }
         }
 #pragma unroll
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_digits_kernel(const Pack
       if (r0 + r < job.R) {
 #pragma unroll 4
         for (int k = warp / groups; k < job.K; k += step_k)
-          m = max(m, abs_bits(__ldg(src + (int64_t)(r0 + r) * job.ld_r + (int64_t)k * job.ld_k)));
+          m = max(m, abs_bits(src[(int64_t)(r0 + r) * job.ld_r + (int64_t)k * job.ld_k]));
         atomicMax(&rmax[r], m);
       }
     }
