@@ -129,9 +129,9 @@ int su2g_heff_plan_status(su2g_heff_plan* plan, int* code);
  * DGEMM per block).  Buckets: M <= m_edges[i] (i < nm), N <= n_edges[j], the
  * last bucket of each open-ended; cls[i * nn + j] in 0..3 = tiles of 64 x 64,
  * 64 x 32, 32 x 64, 32 x 32.  The planner of plans built afterwards cuts by
- * it; without a table every block uses 64 x 64.  The launches are cut further
- * (32 x 32, 16 x 16, or 8 x 8 with a split contraction) whatever the table, so results
- * do not depend on it. */
+ * it; without a table every block uses 64 x 64.  It is launched so where a phase
+ * has tiles in plenty; else the launches are cut further (32 x 32, 16 x 16, or
+ * 8 x 8 with a split contraction).  Results do not depend on the table. */
 int su2g_f64_tile_table(const int* m_edges, int nm, const int* n_edges, int nn, const int* cls);
 /* The autotuner's measurement: nblocks independent M x N x K block products
  * in tiles of class cls, one launch, repeated reps times; *ms = device

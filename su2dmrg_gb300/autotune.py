@@ -12,11 +12,12 @@ afterwards cut every block by its size class.  The table persists as JSON;
 `load` installs a saved one (the package ships one, tile_table_gb300.json, and
 installs it when the library loads).
 
-A plan's launches no longer depend on the class: every phase is cut further
-for the device, into 32x32 tiles or into 8x8 tiles with a split contraction
-(f64_launch_tiles in heff_plan.cpp), because neither wastes FP64 work on
-padding and a finer cut keeps every SM busy.  Results are the same whatever
-table is installed.
+A phase with tiles in plenty (256 and more of 32x32 for each SM: site updates
+and phase 1 of H_eff from about D = 2000 on) launches them as the table cuts
+them.  The others are cut further for the device, into 32x32 or 16x16 tiles or
+into 8x8 tiles with a split contraction (f64_launch_tiles in heff_plan.cpp),
+because a finer cut keeps every SM busy.  Results are the same whatever table is
+installed.
 """
 from __future__ import annotations
 

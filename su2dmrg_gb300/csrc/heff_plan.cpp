@@ -102,23 +102,37 @@ void add_tiles(std::vector<GemmTile>& tiles, int64_t c_off, int64_t c_len, int c
     }
 }
 
-// Splitting pays where a tile contracts enough values for eight warps to share
-// (always), or where whole 32 x 32 tiles would leave SMs idle.  Measured on
-// GB300, phase 1 (one product a tile) + phase 2 (all terms), ms: D = 2000, 18
-// terms, K <= 555 and 31,000: whole 64.7 + 72.6, split 67.1 + 67.0; D = 1000:
-// 8.44 + 8.86 and 9.22 + 8.65; D = 400, 12 terms, K <= 105 and 4,000: 0.39 and
-// 0.51 + 0.41; D = 251, 9 terms: phase 2 2.13 whole, 0.096 split.  A few
-// products of few values in a row are a chain of load latencies for one warp:
-// phase 2 of D = 24, 2 terms, 16.0 us whole, 6.8 split; D = 8, 4 terms, 17.9
-// and 7.8.  Single products too short to split go in 16 x 16 tiles where 32 x
-// 32 ones are uneven: phase 1 of D = 123, 5 terms (255 tiles of up to 34
-// values), 17.7 -> 14.9 us, D = 200, 6 terms, 47.1 -> 42.5; taking the line
-// further up, D = 251, 9 terms, loses: 84 -> 94.
+// Whole tiles leave SMs idle at a phase's end, the more the fewer of them an SM
+// gets and the longer each one's contraction is; 8 x 8 tiles whose contraction
+// eight warps share leave none, but there are up to sixteen times as many to
+// list, upload and start.  So a phase is split where its contraction is long
+// against the whole tiles of an SM, or where whole tiles are uneven.  Measured
+// on GB300, ms (tiles an SM; whole, split): phase 2 of H_eff, D = 1000, 18
+// terms, K = 13,400 (2.2): 8.86, 8.65; D = 2000, K = 26,700 (8.8): 71.3, 67.1;
+// D = 3000, 10 terms, K = 22,300 (20): 131.3, 128.0; D = 400, 12 terms, K <=
+// 4,000 (0.4): 0.51, 0.41; D = 251, 9 terms (0.14): 2.13, 0.096.  Where tiles
+// are plenty the split only costs: phase 1 of D = 2000, K <= 540 (419): 64.7,
+// 67.1; a whole site update with its planning, K <= 1,080 in phase 2, D = 2000,
+// 18 operators (97): 52.5, 76.3 (338,546 tiles, 75 ms of host time), 4 operators
+// (22): 12.4, 17.0.  A few products of few values in a row are a chain of load
+// latencies for one warp: phase 2 of D = 24, 2 terms, 16.0 us whole, 6.8 split;
+// D = 8, 4 terms, 17.9 and 7.8.  Single products too short to split go in 16 x
+// 16 tiles where 32 x 32 ones are uneven: phase 1 of D = 123, 5 terms (255 tiles
+// of up to 34 values), 17.7 -> 14.9 us, D = 200, 6 terms, 47.1 -> 42.5; taking
+// the line further up, D = 251, 9 terms, loses: 84 -> 94.
+//
+// Long lists cost the host: from kF64Plenty tiles an SM on they are not sorted
+// (the planner's order, by contraction, is as good: the D = 2000 update 55.0 ->
+// 52.5 ms), and from kF64Uncut on the planner's tiles are launched as they are
+// (at D = 2000 phase 1 takes 64.5 ms so, 64.4 cut; at D = 1000, 106 tiles an SM,
+// 8.44 and 8.31).
 namespace {
 constexpr int64_t kF64SplitK = 1024;    // split from this many contracted values on,
+constexpr double kF64SplitPerTile = 128;  // if as many for each whole tile an SM gets,
 constexpr int64_t kF64MinSplitK = 96;   // and where 32 x 32 tiles are uneven from this many
 constexpr int kF64MinSplitSegs = 3;     // or this many products on;
 constexpr double kF64Uneven = 3.0;      // uneven: one takes more than a third of an SM's share
+constexpr double kF64Plenty = 16, kF64Uncut = 256;  // 32 x 32 tiles an SM
 }  // namespace
 
 std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles) {
@@ -136,10 +150,15 @@ std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles) {
     kmax = std::max(kmax, t.kwork);
   }
   const bool uneven = largest * kF64Uneven > total / kF64Sms;
-  const bool split =
-      kmax >= kF64SplitK || (uneven && (kmax >= kF64MinSplitK || (segs >= kF64MinSplitSegs && kmax >= 8)));
+  const double per_sm = largest > 0 ? total / kF64Sms / largest : 0.0;  // the largest tiles an SM's share is worth
+  const bool split = (kmax >= kF64SplitK && kmax >= kF64SplitPerTile * per_sm) ||
+                     (uneven && (kmax >= kF64MinSplitK || (segs >= kF64MinSplitSegs && kmax >= 8)));
+  if (!split && per_sm >= kF64Uncut) return tiles;
   const int side = split ? 8 : uneven ? 16 : 32;
+  size_t count = 0;
+  for (const GemmTile& t : tiles) count += (size_t)up(t.mlen, side) * up(t.nlen, side);
   std::vector<GemmTile> out;
+  out.reserve(count);
   for (const GemmTile& t : tiles)
     for (int m = 0; m < t.mlen; m += side)
       for (int n = 0; n < t.nlen; n += side) {
@@ -152,6 +171,7 @@ std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles) {
         u.ksplit = split ? 1 : 0;
         out.push_back(u);
       }
+  if (per_sm >= kF64Plenty) return out;
   // heaviest first, as the planner's
   auto work = [&](const GemmTile& t) { return (int64_t)up(t.mlen, 8) * up(t.nlen, 8) * t.kwork; };
   std::stable_sort(out.begin(), out.end(), [&](const GemmTile& x, const GemmTile& y) { return work(x) > work(y); });

@@ -43,9 +43,10 @@ void add_tiles(std::vector<GemmTile>& tiles, int64_t c_off, int64_t c_len, int c
                int seg0, int nseg, int64_t kwork);
 
 // The tiles one phase launches, cut from the planner's: 32 x 32 (16 x 16 where
-// those are uneven), each element summed by one warp in k order, or 8 x 8 with
-// the contraction split over the CTA's warps.  Which, follows from the phase's output blocks and products
-// alone (not from the tile classes).
+// those are uneven, the planner's own where a phase has tiles in plenty), each
+// element summed by one warp in k order, or 8 x 8 with the contraction split over
+// the CTA's warps.  Which of the two sums, follows from the phase's output
+// blocks and products alone (not from the tile classes).
 std::vector<GemmTile> f64_launch_tiles(const std::vector<GemmTile>& tiles);
 // how many of each kind a list holds; the list must be ordered by kind (f64_order_by_kind)
 F64Counts f64_counts(const std::vector<GemmTile>& tiles);
