@@ -18,10 +18,13 @@
 // values of k stays below 7 * 560 * 65^2 = 16,562,000 < 2^24 in magnitude
 // (every partial sum too), so the FP32 tensor-core accumulation of one group
 // over one K chunk of 560 is exact, and the chunk sums are combined in 64-bit
-// integers, C = 2^(e_i + f_j - 48) sum_g 2^(48 - 7g) G_g.  The only
-// rounding is in forming N (2^-48 relative to the row maximum for S = 7), in
-// the dropped pairs, and in aligning products of different exponents to the
-// tile's common fixed point (2^-46 of the tile's largest product).
+// integers, C = 2^(e_i + f_j - 48) sum_g 2^(48 - 7g) G_g.  Rounding happens in
+// forming N (2^-48 relative to the row maximum for S = 7), in the dropped
+// pairs, and once a chunk, when its sum is aligned to the tile's common fixed
+// point (half a unit, 2^-47 of the bound 2^(e+f-2) of the tile's largest
+// product) and, for S = 7, when G_7 and G_8, of weights 1/2 and 2^-8, are first
+// brought to the unit of their own product (at most one unit together; the
+// chunk's dropped pairs are worth up to 2^-15 6 560 64^2 = 420 units).
 //
 // Packed operand layout (bytes), built by the pack kernel:
 //   [row tile rt][k tile kt][slice p][rows RT x 16 k, tcgen05 canonical

@@ -152,13 +152,14 @@ __device__ __forceinline__ int f32_to_int_shift(uint32_t bits) {  // round(G 2^-
 
 // Twice the weighted sum of one column's S group sums, v = sum_g G_g 2^(34 - 7g)
 // (group g weighs 2^(kFixedTop - 7(g+2))), from their FP32 bit patterns in two
-// parts: the three low groups lo[i] = G_{kHi + i} first (undoubled), then the
-// high ones hi[i] = G_i.
+// parts: the three low groups lo[i] = G_{kHi + i} first (undoubled for 7 slices,
+// whose low part then fits 32 bits), then the high ones hi[i] = G_i.
 // |G_g| <= (g + 1) 560 65^2 <= 16,562,000 (the exactness bound of a chunk), so
 // G_i * 128 + G_{i+1} is exact in int32, as is G_4 2^6 and what lies below, and
 // few 64-bit shift-adds remain; |G_0| < 2^22.  The groups from 5 on weigh 1/2
-// and 1/256 of the fixed point's unit; their sums are rounded to it (the last
-// one of 6 slices, whose own digits end at 2^-42, to two units).
+// and 1/256 of the fixed point's unit.  Doubled, group 5 is a whole number:
+// 6 slices keep all of it.  7 slices cut it to the unit (error below 1/2) and
+// round group 6 to it (1/2), where cutting both left errors below 1/2 and 1.
 template <int S>
 struct Groups;
 template <>
@@ -180,11 +181,11 @@ struct Groups<6> {
   using Low = long long;
   __device__ static Low low(const uint32_t (&r)[3][4], int x) {
     const int X = f32_to_int_exact(r[0][x]) * 128 + f32_to_int_exact(r[1][x]);
-    return ((long long)X << 6) + (long long)(f32_to_int_shift<2>(r[2][x]) * 2);
+    return ((long long)X << 7) + f32_to_int_exact(r[2][x]);
   }
   __device__ static long long high(const uint32_t (&r)[kHi][4], int x, Low low) {
     const int Z = f32_to_int_shift<0>(r[0][x]) * 128 + f32_to_int_exact(r[1][x]);
-    return ((long long)Z << 28) + ((long long)f32_to_int_exact(r[2][x]) << 21) + low * 2;
+    return ((long long)Z << 28) + ((long long)f32_to_int_exact(r[2][x]) << 21) + low;
   }
 };
 
