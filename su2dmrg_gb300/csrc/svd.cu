@@ -48,6 +48,7 @@
 #include "heff_plan.hpp"
 #include "kernels.hpp"
 #include "su2_meta.hpp"
+#include "svd_levels.hpp"
 #include "su2g.h"
 
 namespace {
@@ -223,9 +224,9 @@ __global__ void __launch_bounds__(256) canonical_signs_kernel(const __grid_const
 // dependent launches); a truncation at D = 400 (14 sectors of up to 108 rows, 10
 // levels) 48.3 -> 13.7 ms, those of a sweep of the 8x4 cylinder at D = 400 2.49
 // -> 0.52 s, with the same or smaller residuals and orthonormality errors.
-constexpr double kDecade = 0.1;         // T: diagonal entries from a tenth of the largest on
+using su2g::kDecade;                    // T: diagonal entries from a tenth of the largest on
+using su2g::kStepMax;
 constexpr double kStepDone = 1e-8;      // steps up to this leave an error below rounding
-constexpr double kStepMax = 1e-3;       // larger ones: an eigendecomposition
 constexpr int kRefineMax = 6000;        // the kernel's shared memory (48 KB of eigenvalues)
 constexpr double kLevelNoise = 8 * 2.220446049250313e-16;  // of the level's largest entry
 
@@ -416,12 +417,7 @@ class SectorThreads {
   size_t idle_ = 0;
 };
 
-// index after the last eigenvalue below tol1 of the largest (tensor.cpp:1492-1497)
-int small_count(const std::vector<double>& w, int n) {
-  for (int i = n - 1; i >= 0; --i)
-    if (w[i] / w[n - 1] < 1.e-1) return i + 1;
-  return 0;
-}
+using su2g::small_count;
 
 // One stream's part of a truncation: its allocations (from the pool, on the
 // stream; released on `free_st` once the caller's stream has used them) and its
@@ -736,7 +732,7 @@ class Truncation {
   }
 
  private:
-  bool beyond_cut(const std::vector<double>& w, int n) const { return cut > 0 && w[n - 1] < kDecade * cut; }
+  bool beyond_cut(const std::vector<double>& w, int n) const { return su2g::beyond_cut(w, n, cut); }
 
   // eigendecompositions in place, signs as they come: each on a stream and
   // host thread of its own, or (together) the small ones as a batch beside them
@@ -834,7 +830,7 @@ class Truncation {
       g1.clear();
       for (Sector* s : open) {
         const int n = s->npp;
-        if (!settled(*s, it)) {
+        if (!su2g::level_settled(std::vector<double>(s->h, s->h + n), s->h[n], it, cut)) {
           wait->push_back(s);
           continue;
         }
@@ -854,21 +850,6 @@ class Truncation {
     }
     wait->insert(wait->end(), open.begin(), open.end());
     return solved;
-  }
-
-  // whether a step of the refinement may be taken (kernel's T: from t0 on, in
-  // ascending order, everything below it smaller than a tenth of the last entry)
-  bool settled(const Sector& s, int it) const {
-    const int n = s.npp;
-    const std::vector<double> h(s.h, s.h + n);
-    const int t0 = small_count(h, n);
-    bool good = s.h[n] <= (it > 0 ? 10 * kStepMax : kStepMax) && h[n - 1] > 0;
-    for (int i = 0; i < n && good; ++i) {
-      const bool in_top = h[i] >= kDecade * h[n - 1];
-      good = in_top == (i >= t0) && (i <= t0 || h[i] >= h[i - 1]);
-    }
-    if (good && it == 0 && t0 > 1) good = !beyond_cut(h, t0);
-    return good;
   }
 
   // Rotates the solved sectors' columns and goes on to their next levels;
