@@ -37,8 +37,8 @@ struct CombSrc {
 };
 // The lists travel in the kernel's parameters (3.6 KB, below the 4 KB every
 // launch has): nothing is allocated, copied or waited for before the launch.
-// More runs take more launches; a run of more sources than a list holds reads
-// them from device memory.
+// More runs take more launches; where a run may have more sources than a list
+// holds, all the sources go to device memory in one copy instead.
 constexpr int kCombRuns = 32, kCombSrcs = 160;
 struct CombList {
   CombRun run[kCombRuns];
@@ -52,8 +52,8 @@ constexpr int kCombTile = kCombThreads * kCombElems;
 // times four sources in flight, and three CTAs an SM already at 230,000
 // elements).  HBM-bound in principle; six operands of 1.9 MB (D = 900) are in
 // L2 or launch-bound.  With the lists allocated and copied for each call such
-// a sum took its caller 110 us (408 with the default pool cold), now 93 (152),
-// most of it the caller's own marshalling.
+// a sum took its caller 110 us (408 with the default pool cold), now 70, most of
+// it the caller's own marshalling.
 __global__ void __launch_bounds__(kCombThreads) combine_kernel(const __grid_constant__ CombList list, int nrun,
                                                                const CombSrc* many, double* out) {
   int r = 0;
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kCombThreads) combine_kernel(const __grid_cons
   double a0 = 0.0, a1 = 0.0;
 #pragma unroll 4
   for (int s = 0; s < it.nsrc; ++s) {
-    const CombSrc q = many ? many[s] : list.src[it.src0 + s];
+    const CombSrc q = many ? many[it.src0 + s] : list.src[it.src0 + s];
     const double x0 = in0 ? q.p[e0] : 0.0, x1 = in1 ? q.p[e0 + kCombThreads] : 0.0;
     a0 += q.c * x0;
     a1 += q.c * x1;
@@ -74,52 +74,57 @@ __global__ void __launch_bounds__(kCombThreads) combine_kernel(const __grid_cons
   if (in1) o[kCombThreads] = a1;
 }
 
-// The launches of one linear combination: runs and their sources are added one
-// by one and sent whenever a list is full.
+// The launches of one linear combination of n operands: runs and their sources
+// are added one by one and sent whenever a list is full; with more operands than
+// a list holds, once all are known (200 operands that hold different blocks: 356
+// us, 1,294 with a copy and a wait for each run).
 class CombLauncher {
  public:
-  CombLauncher(double* out, cudaStream_t st) : out_(out), st_(st) {}
-  ~CombLauncher() {
-    for (void* d : lists_) su2g::dev_free(d, st_);
-  }
+  CombLauncher(int n, double* out, cudaStream_t st) : many_(n > kCombSrcs), out_(out), st_(st) {}
   void add(int64_t dst, int64_t len, const std::vector<CombSrc>& src) {
-    const bool many = (int)src.size() > kCombSrcs;
-    if (many || nrun_ == kCombRuns || nsrc_ + (int)src.size() > kCombSrcs) flush(nullptr);
-    CombRun& r = list_.run[nrun_++];
-    r.dst = dst;
-    r.len = len;
-    r.tile0 = tiles_;
-    r.src0 = nsrc_;
-    r.nsrc = (int)src.size();
-    tiles_ += (len + kCombTile - 1) / kCombTile;
-    if (!many) {
-      std::copy(src.begin(), src.end(), list_.src + nsrc_);
-      nsrc_ += (int)src.size();
+    if (!many_ && (nrun_ == kCombRuns || nsrc_ + (int)src.size() > kCombSrcs)) send(list_.run, nrun_, nullptr);
+    const CombRun r{dst, len, 0, many_ ? (int)srcs_.size() : nsrc_, (int)src.size()};
+    if (many_) {
+      runs_.push_back(r);
+      srcs_.insert(srcs_.end(), src.begin(), src.end());
       return;
     }
-    void* d = nullptr;
-    if (e_ == cudaSuccess) e_ = su2g::upload_bytes(src.data(), src.size() * sizeof(CombSrc), &d);
-    if (d) lists_.push_back(d);
-    flush((const CombSrc*)d);
+    std::copy(src.begin(), src.end(), list_.src + nsrc_);
+    nsrc_ += (int)src.size();
+    list_.run[nrun_++] = r;
   }
   cudaError_t finish() {
-    flush(nullptr);
+    if (!many_) {
+      send(list_.run, nrun_, nullptr);
+      return e_;
+    }
+    void* d = nullptr;
+    if (!srcs_.empty()) e_ = su2g::upload_bytes(srcs_.data(), srcs_.size() * sizeof(CombSrc), &d);
+    for (size_t r = 0; r < runs_.size() && e_ == cudaSuccess; r += kCombRuns)
+      send(runs_.data() + r, (int)std::min<size_t>(kCombRuns, runs_.size() - r), (const CombSrc*)d);
+    su2g::dev_free(d, st_);
     return e_;
   }
 
  private:
-  void flush(const CombSrc* many) {
-    if (nrun_ > 0 && tiles_ > 0 && e_ == cudaSuccess) {
-      combine_kernel<<<(unsigned)tiles_, kCombThreads, 0, st_>>>(list_, nrun_, many, out_);
+  void send(const CombRun* runs, int n, const CombSrc* many) {
+    int64_t tiles = 0;
+    for (int r = 0; r < n; ++r) {
+      list_.run[r] = runs[r];
+      list_.run[r].tile0 = tiles;
+      tiles += (runs[r].len + kCombTile - 1) / kCombTile;
+    }
+    if (tiles > 0 && e_ == cudaSuccess) {
+      combine_kernel<<<(unsigned)tiles, kCombThreads, 0, st_>>>(list_, n, many, out_);
       e_ = cudaGetLastError();
     }
     nrun_ = nsrc_ = 0;
-    tiles_ = 0;
   }
+  const bool many_;
   CombList list_{};
-  std::vector<void*> lists_;  // device copies of the long source lists
+  std::vector<CombRun> runs_;
+  std::vector<CombSrc> srcs_;
   int nrun_ = 0, nsrc_ = 0;
-  int64_t tiles_ = 0;
   double* out_;
   cudaStream_t st_;
   cudaError_t e_ = cudaSuccess;
@@ -201,7 +206,7 @@ extern "C" int su2g_operator_combine(int n, const su2g_tensor* ops, const double
   if (nblocks == 0) return SU2G_OK;
   if (nblocks > 65535) return fail(SU2G_EUNSUPPORTED, "operator_combine: more than 65535 blocks");
   cudaStream_t st = (cudaStream_t)stream;
-  CombLauncher launcher(out, st);
+  CombLauncher launcher(n, out, st);
   std::vector<CombSrc> srcs;
   for (int b = 0; b < o.nten;) {
     if (!o.flag[b]) {
