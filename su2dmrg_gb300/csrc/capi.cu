@@ -910,6 +910,10 @@ int su2g_vec_scale(double alpha, double* x, int64_t n, void* stream) {
 // ----------------------------------------------------------------- Lanczos
 namespace {
 
+// about what an application of a plan does, FLOP/s, and the step from which on
+// the host looks at every coefficient (su2g_lanczos)
+constexpr double kF64StepRate = 1e12, kSplitStepRate = 4e13, kStepLookSeconds = 1e-3;
+
 struct LanczosCtx {
   su2g_heff_plan* p;
   cudaStream_t st;
@@ -1085,11 +1089,15 @@ int su2g_lanczos(su2g_heff_plan* p, double* psi, int mlanc, double* energy, int*
   // The coefficients are read where a check needs them (every fourth step and
   // the last), so that the device does not wait for the host in between.  A
   // norm below tol found then ends the solve at its own step, as if it had
-  // been looked at there: what came after is dropped.
+  // been looked at there: what came after is dropped.  Steps of a millisecond
+  // and more are looked at one by one: the wait is lost in them (some 12 us),
+  // steps run for nothing are not (a D = 1200 solve in FP64 that ends at its
+  // second step: 9.9 ms, 16.5 with the coefficients read at the fourth).
+  const bool each = p->work.flops >= kStepLookSeconds * (p->S == 0 ? kF64StepRate : kSplitStepRate);
   int seen = 1;
   for (int m = 2; m < mlanc; ++m) {  // lanczos_su2.cpp:155-188
     if ((rc = L.run_graph(false, m))) return rc;
-    if (m % 4 != 0 && m + 1 < mlanc) continue;
+    if (!each && m % 4 != 0 && m + 1 < mlanc) continue;
     if ((rc = fetch_coefs(m))) return rc;
     while (++seen <= m)
       if (nnl[seen] < tol) {
