@@ -121,9 +121,11 @@ __global__ void copy_arrays(const __grid_constant__ JobList<CopyJob> list, int n
 }
 
 // A matrix (n x n, ld n) as the leading block of one of size N for a batch of
-// equal sizes: beyond it a diagonal below every eigenvalue of a Gram matrix,
-// of the matrix's own scale, so that the padding comes first and its rows stay
-// zero in the others' eigenvectors.  And the vectors back.
+// equal sizes: beyond it a diagonal below every eigenvalue, of the matrix's own
+// scale, so that the padding comes first and its rows stay zero in the others'
+// eigenvectors.  And the vectors back.  A level in the rounding noise has
+// negative eigenvalues, often larger than every entry of its diagonal: the bound
+// lies an eighth beyond the largest column sum of magnitudes.
 struct PadJob {
   double* mat;
   int n;
@@ -133,13 +135,17 @@ __global__ void pad_matrix(const __grid_constant__ JobList<PadJob> list, int njo
   __shared__ double smax[8];
   int c;
   const PadJob& j = my_job(list, njobs, &c);
-  double mx = 0;
-  for (int i = threadIdx.x; i < j.n; i += blockDim.x) mx = fmax(mx, j.mat[(int64_t)i * j.n + i]);
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  double mx = 0;  // every CTA finds it: 128 columns at most
+  for (int q = threadIdx.x >> 5; q < j.n; q += 8) {
+    double sum = 0;
+    for (int i = threadIdx.x & 31; i < j.n; i += 32) sum += fabs(j.mat[(int64_t)q * j.n + i]);
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    mx = fmax(mx, sum);
+  }
   if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = mx;
   __syncthreads();
   for (int w = 0; w < 8; ++w) mx = fmax(mx, smax[w]);
-  const double below = mx > 0 ? -mx : -1.0;
+  const double below = mx > 0 ? -1.125 * mx : -1.0;
   double* col = j.box + (int64_t)c * N;  // one column a CTA
   for (int r = threadIdx.x; r < N; r += blockDim.x)
     col[r] = r < j.n && c < j.n ? j.mat[(int64_t)c * j.n + r] : r == c ? below : 0.0;
@@ -221,9 +227,10 @@ __global__ void __launch_bounds__(256) canonical_signs_kernel(const __grid_const
 // gap (a degenerate pair: any basis of it is as good).  Mostly one step from X =
 // I does, which is one launch and no product.  A level of 101 rows takes 0.3 ms
 // where cuSOLVER's eigendecomposition takes 4.6 (it is a chain of some hundred
-// dependent launches); a truncation at D = 400 (14 sectors of up to 108 rows, 10
-// levels) 48.3 -> 13.7 ms, those of a sweep of the 8x4 cylinder at D = 400 2.49
-// -> 0.52 s, with the same or smaller residuals and orthonormality errors.
+// dependent launches).  With it and the lockstep further down a truncation at D =
+// 400 (14 sectors of up to 108 rows, 10 levels) takes 9.0 ms, 47.3 before, and
+// those of a sweep of the 8x4 cylinder at D = 400 0.50 s, 2.49 before, with the
+// same or smaller residuals and orthonormality errors.
 using su2g::kDecade;                    // T: diagonal entries from a tenth of the largest on
 using su2g::kStepMax;
 constexpr double kStepDone = 1e-8;      // steps up to this leave an error below rounding
