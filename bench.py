@@ -387,7 +387,7 @@ def run_su2g(args):
         t_kernel = (prof[0] + prof[1]) / 1e3
         achieved = flops / t_kernel / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                "traffic": None, "kernel": "gemm_f64_tiles (FP64 DMMA m8n8k4), 2 launches per step",
+                "traffic": None, "kernel": "gemm_f64_tiles and gemm_f64_ksplit (FP64 DMMA m8n8k4), 2 launches per step",
                 "launch_ms": prof,
                 "peak_source": "measured cuBLAS DGEMM 8192^3 on this GPU (FP64 is not in MEASURED_PEAKS.json)"}
         accuracy = {"mode": "FP64", "rel_err_vs_fp64_path": 0.0}
@@ -439,7 +439,7 @@ def run_su2g(args):
         torch.cuda.synchronize()
         f64_ms = f0.elapsed_time(f1) / nf
         fp64 = {"value": flops / (f64_ms / 1e3) / 1e12, "unit": UNIT, "ms_per_step": f64_ms, "steps": nf,
-                "path": "gemm_f64_tiles (FP64 DMMA), same plan inputs, device-resident",
+                "path": "gemm_f64_tiles and gemm_f64_ksplit (FP64 DMMA), same plan inputs, device-resident",
                 "split_speedup": f64_ms / ms_per_step}
         ref_plan.close()
         accuracy = {"mode": f"BF16 x {S} slices", "rel_err_vs_fp64_path": rel,
